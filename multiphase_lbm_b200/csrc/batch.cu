@@ -468,6 +468,10 @@ mlbm_status mlbm_batch_iterate(mlbm_batch* b, int32_t nsteps, int32_t reverse,
   if (nsteps == 0) return MLBM_OK;
   mlbm::DeviceGuard restore_device;
   BCUDA(cudaSetDevice(b->device), "cudaSetDevice");
+  // a domain advanced on its own since may hold its state in another form
+  if (b->compact)
+    for (const mlbm_lattice* l : b->dom)
+      if (l && !l->compact.active) b->dirty = true;
   if (b->dirty)
     if (mlbm_status st = rebuild(b)) return st;
   if (b->nactive == 0) return MLBM_OK;

@@ -230,7 +230,21 @@ mlbm_status launch_steps(mlbm_lattice* lat, int64_t step0, int32_t nsteps,
                              lat->stream),
              "velocity clear");
   }
-  if (compact) {
+  // tau = 1 and no kernel asked for that holds populations: the moment step.
+  // Where its buffers do not fit the device, the population kernels run.
+  bool moments = false;
+  if ((compact && !band) ||
+      (lat->step_kernel == MLBM_KERNEL_AUTO && kind == MLBM_KERNEL_TWO_PASS)) {
+    if (moments_apply(lat)) {
+      const mlbm_status st = moments_prepare(lat);
+      if (st && st != MLBM_ERR_NOMEM) return st;
+      moments = st == MLBM_OK;
+    }
+  }
+  if (moments) {
+    if (lat->compact.active)
+      if (mlbm_status st = compact_leave(lat)) return st;
+  } else if (compact) {
     if (mlbm_status st = compact_enter(lat)) return st;
     // bands that do not fit shared memory: compact two-pass steps
     if (band && !compact_band_fits(lat)) band = false;
@@ -242,6 +256,12 @@ mlbm_status launch_steps(mlbm_lattice* lat, int64_t step0, int32_t nsteps,
     const bool last = s == nsteps - 1;
     const bool wu = (flags & MLBM_ITER_WRITE_VELOCITY) && last;
     mlbm_status st;
+    if (moments) {
+      if (mlbm_status ms = launch_moment_step<T>(lat, a, wu, last)) return ms;
+      lat->phase ^= 1;
+      if (wu) lat->vel_valid = true;
+      continue;
+    }
     // the one-pass step starts and ends in AA phase 1; from phase 0 one
     // two-pass step gets there
     const bool one_pass = band && lat->phase == 1;
@@ -574,6 +594,7 @@ mlbm_status mlbm_initialize(mlbm_lattice* lat) {
   }
   if (st) return st;
   lat->compact.active = false;  // the initial state is written densely
+  moments_reset(lat);
   lat->phase = 0;
   lat->initialized = true;
   lat->vel_valid = false;
@@ -664,10 +685,14 @@ mlbm_status stats_enqueue(mlbm_lattice* lat, double* h, bool full) {
                 "gather the slabs' own planes first");
   DeviceGuard restore_device;
   if (mlbm_status st = activate(lat)) return st;
-  // a lattice held in the fluid-only layout is walked through its node
-  // table (no lanes idle on solid nodes); otherwise the dense grid
+  // a lattice held in the fluid-only layout or as moments is walked through
+  // its node table (no lanes idle on solid nodes); otherwise the dense grid
   const CompactState& c = lat->compact;
-  const bool fluid_list = c.active && c.cinfo && lat->storage != MLBM_STORE_F64;
+  const uint2* nodes = lat->mom.active ? lat->mom.list
+                       : c.active      ? c.cinfo
+                                       : nullptr;
+  const long long nslots = lat->mom.active ? lat->mom.count : c.nfluid;
+  const bool fluid_list = nodes != nullptr;
   const dim3 grid(lat->g.px / 32, (lat->g.ly + 7) / 8,
                   (lat->g.lz + kStatZ - 1) / kStatZ);
   // The fluid-list form runs one wave of resident blocks over even spans of
@@ -689,10 +714,10 @@ mlbm_status stats_enqueue(mlbm_lattice* lat, double* h, bool full) {
       lat->stats_wave = std::max(1, per_sm * nsm);
     }
     const long long rounds =
-        std::max(1LL, (c.nfluid + kStatThreads - 1) / kStatThreads);
+        std::max(1LL, (nslots + kStatThreads - 1) / kStatThreads);
     nblocks = std::min<long long>(lat->stats_wave, rounds);
     span = (rounds + nblocks - 1) / nblocks * kStatThreads;
-    nblocks = std::max(1LL, (c.nfluid + span - 1) / span);
+    nblocks = std::max(1LL, (nslots + span - 1) / span);
   }
   // slot 0: the arrival counter; the block records; the results
   const size_t need = (1 + (size_t)nblocks * ST_COUNT + ST_COUNT + 1) * sizeof(double);
@@ -712,10 +737,15 @@ mlbm_status stats_enqueue(mlbm_lattice* lat, double* h, bool full) {
   sc.records = lat->stats_scratch + 1;
   sc.out = sc.records + (size_t)nblocks * ST_COUNT;
   double* fin = sc.out;
-  if (fluid_list) {
+  if (fluid_list && lat->storage == MLBM_STORE_F64) {
+    auto kernel = full ? k_stats_fluid<double, true> : k_stats_fluid<double, false>;
+    kernel<<<(unsigned)nblocks, kStatThreads, 0, lat->stream>>>(
+        static_cast<const double*>(lat->rho), nodes, nslots, span, lat->g,
+        lat->phys, sc, lat->err);
+  } else if (fluid_list) {
     auto kernel = full ? k_stats_fluid<float, true> : k_stats_fluid<float, false>;
     kernel<<<(unsigned)nblocks, kStatThreads, 0, lat->stream>>>(
-        static_cast<const float*>(lat->rho), c.cinfo, c.nfluid, span, lat->g,
+        static_cast<const float*>(lat->rho), nodes, nslots, span, lat->g,
         lat->phys, sc, lat->err);
   } else if (lat->storage == MLBM_STORE_F64) {
     auto kernel = full ? k_stats_partial<double, true> : k_stats_partial<double, false>;

@@ -34,6 +34,21 @@ struct CompactState {
   int band_slot = 0, band_slot_rows = -1, band_slot_nb = -1, band_slot_storage = -1;
 };
 
+// The moment step (moments.cuh): node list and buffers, built on first use.
+struct MomentState {
+  bool list_built = false;  // list matches the current mask
+  bool words_current = false;  // and its neighbour words are lat->nbw's
+  bool no_room = false;     // a buffer was refused: population kernels run
+  bool active = false;      // m holds the current state
+  void* buffer = nullptr;   // one allocation for m, n and list
+  uint2* list = nullptr;    // [count] fluid nodes (neighbour word, packed x, y, z)
+  int count = 0;
+  size_t list_cap = 0;      // nodes list and n were allocated for
+  void* m = nullptr;        // [psi_elems] Mom<R>: density, velocity
+  void* n = nullptr;        // [count] Mom<R>: density, momentum
+  float shift = 0.f;        // rho_shift the state was produced under
+};
+
 // Bound of the step kernels' device waits, and the test switch that makes
 // one wait run out.
 constexpr unsigned long long kDefaultWaitNs = 1000000000ull;  // 1 s
@@ -68,6 +83,7 @@ struct mlbm_lattice {
   int* err = nullptr;                      // device error flag (wait timeout)
   int step_kernel = 0;                     // MLBM_KERNEL_*
   mlbm::CompactState compact{};            // fluid-only layout (compact.cuh)
+  mlbm::MomentState mom{};                 // moment step (moments.cuh)
 
   unsigned long long wait_ns = mlbm::kDefaultWaitNs;  // bounded waits
   bool stall_test = false;  // the next step launch makes a wait run out
@@ -86,7 +102,8 @@ Geom make_geom(int lx, int ly, int lz);
 // (Re)build the update pass's tile shape and psi tensor map.
 mlbm_status setup_update(mlbm_lattice* lat, int rows, int planes);
 struct StepArgs;
-// The fluid-only layout (compact.cu).
+// The fluid-only layout (compact.cu); compact_leave and compact_sync_dense
+// also take a state held as moments to dense populations.
 mlbm_status compact_enter(mlbm_lattice* lat);   // dense -> compact state
 mlbm_status compact_leave(mlbm_lattice* lat);   // compact -> dense state
 mlbm_status compact_sync_dense(mlbm_lattice* lat);  // dense copy, stay compact
@@ -108,5 +125,18 @@ bool compact_band_supported(const mlbm_lattice* lat);
 // Whether the lattice's bands fit shared memory (tables built); where they
 // do not, BAND steps run as compact two-pass steps.
 bool compact_band_fits(mlbm_lattice* lat);
+// The moment step (moments.cu): tau = 1, any storage, whole lattices.
+bool moments_supported(const Geom& g);
+bool moments_apply(const mlbm_lattice* lat);
+mlbm_status moments_prepare(mlbm_lattice* lat);      // node list and buffers
+// One step; starts from moments, or from populations in the dense layout.
+template <typename T>
+mlbm_status launch_moment_step(mlbm_lattice* lat, const StepArgs& a,
+                               bool write_u, bool write_rho);
+mlbm_status moments_sync_dense(mlbm_lattice* lat);   // dense copy, stay
+mlbm_status moments_leave(mlbm_lattice* lat);        // moments -> dense state
+void moments_invalidate(mlbm_lattice* lat);           // the mask changed
+void moments_reset(mlbm_lattice* lat);                // a new initial state
+void moments_free(mlbm_lattice* lat);
 mlbm_status compact_set_band_shape(mlbm_lattice* lat, int rows, int planes);
 }  // namespace mlbm

@@ -12,6 +12,7 @@
 #include "compact.cuh"
 #include "band.cuh"
 #include "compact2.cuh"
+#include "launch.cuh"
 
 namespace mlbm {
 
@@ -147,6 +148,7 @@ bool compact_two_pass_supported(int lx, int ly, int lz, int storage) {
 mlbm_status compact_enter(mlbm_lattice* lat) {
   CompactState& c = lat->compact;
   if (c.active) return MLBM_OK;
+  if (mlbm_status st = moments_leave(lat)) return st;
   if (!c.two_pass_ok)
     return set_error(MLBM_ERR_ARG, "compact layout does not support this lattice");
   if (!c.built)
@@ -162,6 +164,7 @@ mlbm_status compact_enter(mlbm_lattice* lat) {
 }
 
 mlbm_status compact_sync_dense(mlbm_lattice* lat) {
+  if (lat->mom.active) return moments_sync_dense(lat);
   if (!lat->compact.active) return MLBM_OK;
   switch (lat->storage) {
     case MLBM_STORE_F32: return to_dense_t<float>(lat);
@@ -170,6 +173,7 @@ mlbm_status compact_sync_dense(mlbm_lattice* lat) {
 }
 
 mlbm_status compact_leave(mlbm_lattice* lat) {
+  if (lat->mom.active) return moments_leave(lat);
   if (!lat->compact.active) return MLBM_OK;
   if (mlbm_status st = compact_sync_dense(lat)) return st;
   lat->compact.active = false;
@@ -179,10 +183,12 @@ mlbm_status compact_leave(mlbm_lattice* lat) {
 void compact_invalidate(mlbm_lattice* lat) {
   lat->compact.built = false;
   lat->compact.active = false;
+  moments_invalidate(lat);
 }
 
 void compact_free(mlbm_lattice* lat) {
   CompactState& c = lat->compact;
+  moments_free(lat);
   cudaFree(c.cpop);
   cudaFree(c.cpop_alt);
   cudaFree(c.cinfo);
@@ -205,11 +211,7 @@ void own_range(const mlbm_lattice* lat, long long& kb, long long& ke) {
   }
 }
 
-// Launch a step kernel, with programmatic stream serialization when
-// `overlap`: it may then begin while the kernel before it in the stream
-// finishes, and waits for it at pdl_gate() (pair.cuh).  What a kernel reads
-// before its gate must not be written by the kernel launched right before
-// it, whose writes are visible only after the gate:
+// launch_overlapped (launch.cuh) under the gates' rule:
 //   k_cdensity reads the node table (cinfo, wtab) before its gate; the
 //     tables are written only in compact_enter, whose last kernel
 //     (k_convert) does not write them;
@@ -218,23 +220,6 @@ void own_range(const mlbm_lattice* lat, long long& kb, long long& ke) {
 //     (launch_compact_two_pass), which reads them only.  The slab pass API
 //     (launch_compact_pass) may run halo moves between the passes, so it
 //     launches without overlap.
-template <typename... KArgs, typename... Args>
-void launch_overlapped(bool overlap, void (*kernel)(KArgs...), unsigned grid,
-                       cudaStream_t stream, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kC2Threads);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = overlap ? 1 : 0;
-  // a failed launch is reported by the caller's cudaGetLastError
-  (void)cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 unsigned c2_grid(long long kb, long long ke, long long per_thread) {
   const long long threads = (ke - kb + per_thread - 1) / per_thread;
   return (unsigned)((threads + kC2Threads - 1) / kC2Threads);
@@ -251,7 +236,7 @@ void launch_c2_density(mlbm_lattice* lat, const StepArgs& a, bool wr, bool inj,
   float* rho = static_cast<float*>(lat->rho);
   float* psi = static_cast<float*>(lat->psi);
   auto kernel = wr ? k_cdensity<T, PHASE, true> : k_cdensity<T, PHASE, false>;
-  launch_overlapped(overlap, kernel, grid, lat->stream, cpop, cs,
+  launch_overlapped(overlap, kernel, grid, kC2Threads, lat->stream, cpop, cs,
                     (const uint2*)c.cinfo, (const uint2*)c.wtab, (int)kb,
                     (int)ke, rho, psi, lat->g, lat->phys, a, inj);
 }
@@ -266,7 +251,7 @@ void launch_c2_update(mlbm_lattice* lat, const StepArgs& a, bool wu, bool inj,
   const uint32_t cs = (uint32_t)c.cs;
   const float* psi = static_cast<const float*>(lat->psi);
   auto kernel = wu ? k_cupdate<T, PHASE, true> : k_cupdate<T, PHASE, false>;
-  launch_overlapped(overlap, kernel, grid, lat->stream, cpop, cs,
+  launch_overlapped(overlap, kernel, grid, kC2Threads, lat->stream, cpop, cs,
                     (const uint2*)c.cinfo,
                     (const uint2*)c.wtab, (int)kb, (int)ke, psi, lat->vel,
                     lat->g, lat->phys, a, inj);
@@ -276,20 +261,6 @@ bool inject_now(const mlbm_lattice* lat, const StepArgs& a) {
   const Phys& p = lat->phys;
   return p.rho_inject_period != 0ull &&
          (unsigned long long)a.step % p.rho_inject_period == 0ull;
-}
-}  // namespace
-
-namespace {
-// Launches into a stream that is being captured into a CUDA graph are plain:
-// the batched step's graphs with overlapped launches gave wrong states, so
-// the overlap is used in ordinary stream order only.
-bool stream_capturing(cudaStream_t stream) {
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(stream, &st) != cudaSuccess) {
-    cudaGetLastError();  // a query refused during another capture: be plain
-    return true;
-  }
-  return st != cudaStreamCaptureStatusNone;
 }
 }  // namespace
 

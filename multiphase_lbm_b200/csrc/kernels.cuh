@@ -167,7 +167,10 @@ __device__ __forceinline__ void collide(const Phys& p, R d, R psi_self,
   const R base = rsub(R(1), usq15);
   const R wd0 = rmul(weight<R>(0), d), wd1 = rmul(weight<R>(1), d),
           wd2 = rmul(weight<R>(4), d);
-  f[0] = rfma(rsub(rmul(wd0, base), f[0]), omega, f[0]);
+  // omega = 1: f_i + (feq_i - f_i) is feq_i, taken without the two roundings
+  // (what the moment step relies on, moments.cuh)
+  const bool eq = omega == R(1);
+  f[0] = eq ? rmul(wd0, base) : rfma(rsub(rmul(wd0, base), f[0]), omega, f[0]);
 #pragma unroll
   for (int i = 1; i <= 9; ++i) {
     R eu = R(0);
@@ -179,8 +182,8 @@ __device__ __forceinline__ void collide(const Phys& p, R d, R psi_self,
     const R wd = (i <= 3) ? wd1 : wd2;
     const R feq_i = rmul(wd, radd(sym, anti));
     const R feq_o = rmul(wd, rsub(sym, anti));
-    f[i] = rfma(rsub(feq_i, f[i]), omega, f[i]);
-    f[opp(i)] = rfma(rsub(feq_o, f[opp(i)]), omega, f[opp(i)]);
+    f[i] = eq ? feq_i : rfma(rsub(feq_i, f[i]), omega, f[i]);
+    f[opp(i)] = eq ? feq_o : rfma(rsub(feq_o, f[opp(i)]), omega, f[opp(i)]);
   }
 }
 

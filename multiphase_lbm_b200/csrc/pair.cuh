@@ -215,7 +215,8 @@ __device__ __forceinline__ void collide2(const Phys& p, float2 d, float2 psi_sel
   const float2 wd0 = p_mul(p_dup(weight<float>(0)), d),
                wd1 = p_mul(p_dup(weight<float>(1)), d),
                wd2 = p_mul(p_dup(weight<float>(4)), d);
-  f[0] = p_fma(p_sub(p_mul(wd0, base), f[0]), omega, f[0]);
+  const bool eq = p.omega == 1.f;  // as in collide(): f* = feq
+  f[0] = eq ? p_mul(wd0, base) : p_fma(p_sub(p_mul(wd0, base), f[0]), omega, f[0]);
 #pragma unroll
   for (int i = 1; i <= 9; ++i) {
     float2 eu = p_dup(0.f);
@@ -227,8 +228,8 @@ __device__ __forceinline__ void collide2(const Phys& p, float2 d, float2 psi_sel
     const float2 wd = (i <= 3) ? wd1 : wd2;
     const float2 feq_i = p_mul(wd, p_add(sym, anti));
     const float2 feq_o = p_mul(wd, p_sub(sym, anti));
-    f[i] = p_fma(p_sub(feq_i, f[i]), omega, f[i]);
-    f[opp(i)] = p_fma(p_sub(feq_o, f[opp(i)]), omega, f[opp(i)]);
+    f[i] = eq ? feq_i : p_fma(p_sub(feq_i, f[i]), omega, f[i]);
+    f[opp(i)] = eq ? feq_o : p_fma(p_sub(feq_o, f[opp(i)]), omega, f[opp(i)]);
   }
 }
 
