@@ -688,10 +688,10 @@ mlbm_status stats_enqueue(mlbm_lattice* lat, double* h, bool full) {
   // a lattice held in the fluid-only layout or as moments is walked through
   // its node table (no lanes idle on solid nodes); otherwise the dense grid
   const CompactState& c = lat->compact;
-  const uint2* nodes = lat->mom.active ? lat->mom.list
+  const uint2* nodes = lat->mom.active ? lat->mom.nodes
                        : c.active      ? c.cinfo
                                        : nullptr;
-  const long long nslots = lat->mom.active ? lat->mom.count : c.nfluid;
+  const long long nslots = lat->mom.active ? lat->mom.nnodes : c.nfluid;
   const bool fluid_list = nodes != nullptr;
   const dim3 grid(lat->g.px / 32, (lat->g.ly + 7) / 8,
                   (lat->g.lz + kStatZ - 1) / kStatZ);

@@ -34,18 +34,20 @@ struct CompactState {
   int band_slot = 0, band_slot_rows = -1, band_slot_nb = -1, band_slot_storage = -1;
 };
 
-// The moment step (moments.cuh): node list and buffers, built on first use.
+// The moment step (moments.cuh): lists and buffers, built on first use.
 struct MomentState {
-  bool list_built = false;  // list matches the current mask
-  bool words_current = false;  // and its neighbour words are lat->nbw's
+  bool list_built = false;  // the lists match the mask and the slabs
   bool no_room = false;     // a buffer was refused: population kernels run
   bool active = false;      // m holds the current state
-  void* buffer = nullptr;   // one allocation for m, n and list
-  uint2* list = nullptr;    // [count] fluid nodes (neighbour word, packed x, y, z)
-  int count = 0;
-  size_t list_cap = 0;      // nodes list and n were allocated for
-  void* m = nullptr;        // [psi_elems] Mom<R>: density, velocity
-  void* n = nullptr;        // [count] Mom<R>: density, momentum
+  void* buffer = nullptr;   // one allocation for all of the following
+  size_t buffer_bytes = 0;
+  void* m = nullptr;        // [pair_elems] MomPair<R>: density, velocity
+  void* psi = nullptr;      // [pair_elems] Two<R>
+  void* n = nullptr;        // [npairs] MomPair<R>: density, momentum
+  uint2* words = nullptr;   // [npairs] node pairs: neighbour words,
+  uint32_t* xyz = nullptr;  //          packed x, y, z
+  uint2* nodes = nullptr;   // [nnodes] fluid nodes (neighbour word, packed x, y, z)
+  int npairs = 0, nnodes = 0;
   float shift = 0.f;        // rho_shift the state was produced under
 };
 
@@ -128,15 +130,14 @@ bool compact_band_fits(mlbm_lattice* lat);
 // The moment step (moments.cu): tau = 1, any storage, whole lattices.
 bool moments_supported(const Geom& g);
 bool moments_apply(const mlbm_lattice* lat);
-mlbm_status moments_prepare(mlbm_lattice* lat);      // node list and buffers
+mlbm_status moments_prepare(mlbm_lattice* lat);      // lists and buffers
 // One step; starts from moments, or from populations in the dense layout.
 template <typename T>
 mlbm_status launch_moment_step(mlbm_lattice* lat, const StepArgs& a,
                                bool write_u, bool write_rho);
 mlbm_status moments_sync_dense(mlbm_lattice* lat);   // dense copy, stay
 mlbm_status moments_leave(mlbm_lattice* lat);        // moments -> dense state
-void moments_invalidate(mlbm_lattice* lat);           // the mask changed
-void moments_reset(mlbm_lattice* lat);                // a new initial state
+void moments_reset(mlbm_lattice* lat);  // a new mask or initial state
 void moments_free(mlbm_lattice* lat);
 mlbm_status compact_set_band_shape(mlbm_lattice* lat, int rows, int planes);
 }  // namespace mlbm

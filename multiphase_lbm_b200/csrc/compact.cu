@@ -183,7 +183,7 @@ mlbm_status compact_leave(mlbm_lattice* lat) {
 void compact_invalidate(mlbm_lattice* lat) {
   lat->compact.built = false;
   lat->compact.active = false;
-  moments_invalidate(lat);
+  moments_reset(lat);
 }
 
 void compact_free(mlbm_lattice* lat) {
@@ -236,7 +236,7 @@ void launch_c2_density(mlbm_lattice* lat, const StepArgs& a, bool wr, bool inj,
   float* rho = static_cast<float*>(lat->rho);
   float* psi = static_cast<float*>(lat->psi);
   auto kernel = wr ? k_cdensity<T, PHASE, true> : k_cdensity<T, PHASE, false>;
-  launch_overlapped(overlap, kernel, grid, kC2Threads, lat->stream, cpop, cs,
+  launch_overlapped(overlap, kernel, grid, kC2Threads, 0, lat->stream, cpop, cs,
                     (const uint2*)c.cinfo, (const uint2*)c.wtab, (int)kb,
                     (int)ke, rho, psi, lat->g, lat->phys, a, inj);
 }
@@ -251,7 +251,7 @@ void launch_c2_update(mlbm_lattice* lat, const StepArgs& a, bool wu, bool inj,
   const uint32_t cs = (uint32_t)c.cs;
   const float* psi = static_cast<const float*>(lat->psi);
   auto kernel = wu ? k_cupdate<T, PHASE, true> : k_cupdate<T, PHASE, false>;
-  launch_overlapped(overlap, kernel, grid, kC2Threads, lat->stream, cpop, cs,
+  launch_overlapped(overlap, kernel, grid, kC2Threads, 0, lat->stream, cpop, cs,
                     (const uint2*)c.cinfo,
                     (const uint2*)c.wtab, (int)kb, (int)ke, psi, lat->vel,
                     lat->g, lat->phys, a, inj);

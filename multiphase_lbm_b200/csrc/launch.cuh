@@ -12,11 +12,12 @@ namespace mlbm {
 // it, whose writes are visible only after the gate.
 template <typename... KArgs, typename... Args>
 void launch_overlapped(bool overlap, void (*kernel)(KArgs...), unsigned grid,
-                       unsigned block, cudaStream_t stream, Args... args) {
+                       unsigned block, size_t smem, cudaStream_t stream,
+                       Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -1,5 +1,4 @@
-// moments.cu -- host side of the moment step (moments.cuh): node list, buffers,
-// launches, and the way back to populations.
+// moments.cu -- host side of the moment step (moments.cuh): lists, buffers, launches, and the way back to populations.
 #include <cuda_runtime.h>
 
 #include <cub/cub.cuh>
@@ -12,70 +11,83 @@ namespace mlbm {
 
 namespace {
 
-unsigned blocks_of(long long n, int threads) {
-  return (unsigned)((n + threads - 1) / threads);
-}
-
 size_t up256(size_t n) { return (n + 255) / 256 * 256; }
 
-// The node list of the current mask, and the buffers (one allocation: m, n,
-// list).  Waits for the node count.
+// Pair list and node list of the current mask and slabs, and the
+// buffers (one allocation).  Waits for the counts.
 mlbm_status build_list(mlbm_lattice* lat) {
   MomentState& s = lat->mom;
   const Geom& g = lat->g;
-  const long long nwords = mom_tile_words(g);
-  uint32_t* start = nullptr;
+  const long long grid = TileGrid(g).count();
   size_t temp_bytes = 0;
-  uint32_t count = 0;
-  cudaError_t e = cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, start, start,
-                                                nwords + 1, lat->stream);
-  if (e != cudaSuccess) return cuda_fail(e, "moment list");
+  TileCount* counts = nullptr;
+  cudaError_t e = cub::DeviceScan::ExclusiveScan(
+      nullptr, temp_bytes, counts, counts, TileCountSum(), TileCount{0, 0},
+      grid + 1, lat->stream);
+  if (e != cudaSuccess) return cuda_fail(e, "moment lists");
   // scratch of the scan: the transfer buffer an upload has left (same
   // stream), else an allocation of its own
-  const size_t words_bytes = up256((size_t)(nwords + 1) * sizeof(uint32_t));
+  const size_t counts_bytes = up256((size_t)(grid + 1) * sizeof(TileCount));
   char* own = nullptr;
   char* buf = static_cast<char*>(lat->staging);
-  if (lat->staging_bytes < words_bytes + temp_bytes) {
-    e = cudaMalloc((void**)&own, words_bytes + temp_bytes);
-    if (e != cudaSuccess) return cuda_fail(e, "moment list");
+  if (lat->staging_bytes < counts_bytes + temp_bytes) {
+    e = cudaMalloc((void**)&own, counts_bytes + temp_bytes);
+    if (e != cudaSuccess) return cuda_fail(e, "moment lists");
     buf = own;
   }
-  start = reinterpret_cast<uint32_t*>(buf);
-  k_mom_counts<<<blocks_of(nwords + 1, 256), 256, 0, lat->stream>>>(
-      lat->mask, start, nwords, g);
-  e = cub::DeviceScan::ExclusiveSum(buf + words_bytes, temp_bytes, start, start,
-                                    nwords + 1, lat->stream);
+  counts = reinterpret_cast<TileCount*>(buf);
+  const unsigned threads = 32 * kPairRows;
+  k_mom_tiles<true><<<(unsigned)grid, threads, 0, lat->stream>>>(
+      lat->nbw, counts, nullptr, nullptr, nullptr, nullptr, g);
+  e = cub::DeviceScan::ExclusiveScan(buf + counts_bytes, temp_bytes, counts, counts,
+                                     TileCountSum(), TileCount{0, 0}, grid + 1,
+                                     lat->stream);
+  TileCount total{0, 0};
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(&count, start + nwords, sizeof count,
+    e = cudaMemcpyAsync(&total, counts + grid, sizeof total,
                         cudaMemcpyDeviceToHost, lat->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(lat->stream);
-  if (e == cudaSuccess && (!s.buffer || count > s.list_cap)) {
+  const size_t real = real_bytes(lat->storage);
+  const size_t m_bytes = up256((size_t)pair_elems(g) * 8 * real);
+  const size_t psi_bytes = up256((size_t)pair_elems(g) * 2 * real);
+  const size_t n_bytes = up256((size_t)total.pairs * 8 * real);
+  const size_t words_bytes = up256((size_t)total.pairs * sizeof(uint2));
+  const size_t xyz_bytes = up256((size_t)total.pairs * sizeof(uint32_t));
+  const size_t need = m_bytes + psi_bytes + n_bytes + words_bytes + xyz_bytes +
+                      (size_t)total.nodes * sizeof(uint2);
+  if (e == cudaSuccess && need > s.buffer_bytes) {
     cudaFree(s.buffer);
     s.buffer = nullptr;
-    s.list_cap = 0;
-    const size_t node = 4 * real_bytes(lat->storage);
-    const size_t m_bytes = up256((size_t)psi_elems(g) * node);
-    const size_t n_bytes = up256((size_t)count * node);
-    e = cudaMalloc(&s.buffer, m_bytes + n_bytes + (size_t)count * sizeof(uint2));
-    if (e == cudaSuccess) {
-      s.m = s.buffer;
-      s.n = static_cast<char*>(s.buffer) + m_bytes;
-      s.list = reinterpret_cast<uint2*>(static_cast<char*>(s.n) + n_bytes);
-      s.list_cap = count;
-    } else {
-      s.buffer = nullptr;
-    }
+    s.buffer_bytes = 0;
+    e = cudaMalloc(&s.buffer, need);
+    if (e == cudaSuccess) s.buffer_bytes = need;
+    else s.buffer = nullptr;
   }
-  if (e == cudaSuccess && count) {
-    k_mom_list<<<blocks_of(nwords * 32, 256), 256, 0, lat->stream>>>(
-        lat->mask, lat->nbw, start, s.list, nwords, g);
+  if (e == cudaSuccess) {
+    char* at = static_cast<char*>(s.buffer);
+    s.m = at;
+    s.psi = at += m_bytes;
+    s.n = at += psi_bytes;
+    s.words = reinterpret_cast<uint2*>(at += n_bytes);
+    s.xyz = reinterpret_cast<uint32_t*>(at += words_bytes);
+    s.nodes = reinterpret_cast<uint2*>(at + xyz_bytes);
+    s.npairs = (int)total.pairs;
+    s.nnodes = (int)total.nodes;
+    if (total.pairs)
+      k_mom_tiles<false><<<(unsigned)grid, threads, 0, lat->stream>>>(
+          lat->nbw, nullptr, counts, s.words, s.xyz, s.nodes, g);
     e = cudaGetLastError();
   }
   cudaFree(own);
-  if (e != cudaSuccess) return cuda_fail(e, "moment list");
-  s.count = (int)count;
-  s.list_built = s.words_current = true;
+  if (e != cudaSuccess) return cuda_fail(e, "moment lists");
+  s.list_built = true;
   return MLBM_OK;
+}
+
+PairList pair_list(const MomentState& s) { return PairList{s.words, s.xyz, s.npairs}; }
+
+unsigned pair_blocks(const MomentState& s) {
+  return (unsigned)((s.npairs + kMomThreads - 1) / kMomThreads);
 }
 
 template <typename T, bool WR>
@@ -83,38 +95,40 @@ void launch_gather(mlbm_lattice* lat, const StepArgs& a, bool inj, bool overlap)
   using R = typename Pop<T>::Real;
   MomentState& s = lat->mom;
   R* rho = static_cast<R*>(lat->rho);
-  R* psi = static_cast<R*>(lat->psi);
-  Mom<R>* n = static_cast<Mom<R>*>(s.n);
-  const unsigned grid = blocks_of(s.count, kMomThreads);
+  R* psi = static_cast<R*>(s.psi);
+  MomPair<R>* n = static_cast<MomPair<R>*>(s.n);
+  const unsigned grid = pair_blocks(s);
   if (s.active) {
-    launch_overlapped(overlap, k_mom_gather<T, WR>, grid, kMomThreads, lat->stream,
-                      (const Mom<R>*)s.m, (const uint2*)s.list, s.count, n, rho,
-                      psi, lat->g, lat->phys, a, inj, s.shift);
-  } else {
-    const T* pop = static_cast<const T*>(lat->pop);
-    if (lat->phase == 0)
-      k_mom_gather_pop<T, 0, WR><<<grid, kMomThreads, 0, lat->stream>>>(
-          pop, s.list, s.count, n, rho, psi, lat->g, lat->phys, a, inj);
-    else
-      k_mom_gather_pop<T, 1, WR><<<grid, kMomThreads, 0, lat->stream>>>(
-          pop, s.list, s.count, n, rho, psi, lat->g, lat->phys, a, inj);
+    launch_overlapped(overlap, k_mom_gather<T, WR>, grid, kMomThreads, 0, lat->stream,
+                      (const MomPair<R>*)s.m, pair_list(s), n, rho, psi, lat->g,
+                      lat->phys, a, inj, s.shift);
+    return;
   }
+  const Geom& g = lat->g;
+  k_mom_psi<R><<<dim3((g.lx + 31) / 32, (g.ly + 7) / 8, g.lz + 2), dim3(32, 8), 0,
+                 lat->stream>>>(static_cast<const R*>(lat->psi), psi, g);
+  const T* pop = static_cast<const T*>(lat->pop);
+  if (lat->phase == 0)
+    k_mom_gather_pop<T, 0, WR><<<grid, kMomThreads, 0, lat->stream>>>(
+        pop, pair_list(s), n, rho, psi, g, lat->phys, a, inj);
+  else
+    k_mom_gather_pop<T, 1, WR><<<grid, kMomThreads, 0, lat->stream>>>(
+        pop, pair_list(s), n, rho, psi, g, lat->phys, a, inj);
 }
 
 template <typename T>
 mlbm_status to_populations(mlbm_lattice* lat) {
   using R = typename Pop<T>::Real;
   const MomentState& s = lat->mom;
-  if (s.count == 0) return MLBM_OK;
-  const unsigned grid = blocks_of(s.count, kMomThreads);
-  const Mom<R>* m = static_cast<const Mom<R>*>(s.m);
+  if (s.npairs == 0) return MLBM_OK;
+  const MomPair<R>* m = static_cast<const MomPair<R>*>(s.m);
   T* pop = static_cast<T*>(lat->pop);
   if (lat->phase == 0)
-    k_mom_populations<T, 0><<<grid, kMomThreads, 0, lat->stream>>>(
-        m, s.list, s.count, pop, lat->g, s.shift);
+    k_mom_populations<T, 0><<<pair_blocks(s), kMomThreads, 0, lat->stream>>>(
+        m, pair_list(s), pop, lat->g, s.shift);
   else
-    k_mom_populations<T, 1><<<grid, kMomThreads, 0, lat->stream>>>(
-        m, s.list, s.count, pop, lat->g, s.shift);
+    k_mom_populations<T, 1><<<pair_blocks(s), kMomThreads, 0, lat->stream>>>(
+        m, pair_list(s), pop, lat->g, s.shift);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "populations of the moments");
   return MLBM_OK;
@@ -122,10 +136,10 @@ mlbm_status to_populations(mlbm_lattice* lat) {
 
 }  // namespace
 
-// Packed coordinates and 32-bit offsets bound the lattice.
+// Packed coordinates and 32-bit pair indexes bound the lattice.
 bool moments_supported(const Geom& g) {
   return g.lx <= kC2MaxX && g.ly <= kC2MaxY && g.lz <= kC2MaxZ &&
-         psi_elems(g) < (1LL << 31);
+         pair_elems(g) < (1LL << 31);
 }
 
 bool moments_apply(const mlbm_lattice* lat) {
@@ -135,17 +149,8 @@ bool moments_apply(const mlbm_lattice* lat) {
 
 mlbm_status moments_prepare(mlbm_lattice* lat) {
   MomentState& s = lat->mom;
-  mlbm_status st = MLBM_OK;
-  if (!s.list_built) {
-    st = build_list(lat);
-  } else if (!s.words_current) {
-    if (s.count)
-      k_mom_words<<<blocks_of(s.count, 256), 256, 0, lat->stream>>>(
-          lat->nbw, s.list, s.count, lat->g);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_fail(e, "moment list");
-    s.words_current = true;
-  }
+  if (s.list_built) return MLBM_OK;
+  const mlbm_status st = build_list(lat);
   if (st == MLBM_ERR_NOMEM) {
     s.no_room = true;
     cudaGetLastError();  // not an error of the step: it runs on populations
@@ -161,15 +166,14 @@ mlbm_status launch_moment_step(mlbm_lattice* lat, const StepArgs& a, bool write_
   const Phys& p = lat->phys;
   const bool inj = p.rho_inject_period != 0ull &&
                    (unsigned long long)a.step % p.rho_inject_period == 0ull;
-  if (s.count > 0) {
+  if (s.npairs > 0) {
     const bool overlap = !stream_capturing(lat->stream);
     if (write_rho) launch_gather<T, true>(lat, a, inj, overlap);
     else launch_gather<T, false>(lat, a, inj, overlap);
     auto collide = write_u ? k_mom_collide<R, true> : k_mom_collide<R, false>;
-    launch_overlapped(overlap, collide, blocks_of(s.count, kMomThreads),
-                      kMomThreads, lat->stream, (const Mom<R>*)s.n,
-                      (const uint2*)s.list, s.count, (const R*)lat->psi,
-                      (Mom<R>*)s.m, lat->vel, lat->g, lat->phys);
+    launch_overlapped(overlap, collide, pair_blocks(s), kMomThreads, 0, lat->stream,
+                      (const MomPair<R>*)s.n, pair_list(s), (const Two<R>*)s.psi,
+                      (MomPair<R>*)s.m, lat->vel, lat->g, lat->phys);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "moment step launch");
   }
@@ -196,21 +200,15 @@ mlbm_status moments_leave(mlbm_lattice* lat) {
   return MLBM_OK;
 }
 
-void moments_invalidate(mlbm_lattice* lat) {
-  lat->mom.list_built = false;
-  moments_reset(lat);
-}
-
 void moments_reset(mlbm_lattice* lat) {
-  lat->mom.words_current = false;
+  lat->mom.list_built = false;
   lat->mom.no_room = false;
   lat->mom.active = false;
 }
 
 void moments_free(mlbm_lattice* lat) {
-  MomentState& s = lat->mom;
-  cudaFree(s.buffer);
-  s = MomentState{};
+  cudaFree(lat->mom.buffer);
+  lat->mom = MomentState{};
 }
 
 }  // namespace mlbm

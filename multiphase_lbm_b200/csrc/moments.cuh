@@ -10,20 +10,31 @@
 // population kernels, at 16 bytes read and 16 written per node and pass in
 // place of 76.
 //
-// State between steps: m, one Mom per node in a dense array with a ghost
-// layer on every side (psi_index), so that the 18 neighbours of any node sit
-// at fixed offsets, periodic boundaries included.  Solid nodes' entries are
-// never read.  A step is
+// A step is
 //   gather   per fluid node: pulls f_i(x) = f*_i(x - e_i) of its neighbours
 //            (its own f*_opp(i) where x - e_i is solid: halfway
 //            bounce-back), sums rho and the momentum j, writes psi(rho) and
-//            n[k] = (rho, j);
+//            n = (rho, j);
 //   collide  per fluid node: Shan-Chen force from the neighbours' psi,
-//            u = (j + tau F)/rho, writes m = (rho, u) and its ghost copies.
-// n is indexed by the node's place k in the node list (k_mom_list): fluid
-// nodes only, ordered by tiles of 32 x kTileY x kTileZ nodes, so the nodes of
-// one block are neighbours in all three directions and share their loads in
-// L1 (list entry: neighbour word with NB_EDGE, packed coordinates).
+//            u = (j + tau F)/rho, writes m = (rho, u).
+//
+// Layout.  m and psi are dense and hold the nodes z and z + 1 (z even) next to
+// each other: element 2 * ((zp ly + y) px + x) + (z & 1), zp = (z + 2) / 2;
+// planes z = -1 and z = lz hold the periodic images of the last and the first
+// (x and y wrap by the offsets of a node's columns: with ghost copies in all
+// axes the stores of the images took longer than the rest of the collide).
+// A thread owns such a pair of nodes, so the moments of both, and of both
+// their neighbours in a column, are one 32-byte sector and one load; the 36
+// populations of a pair come from 28 nodes in 9 columns, 9 pair loads and 10
+// single ones, and what depends on the source node alone (1 - 1.5 u^2, the
+// weights times rho) is formed once for the up to three populations that the
+// pair takes from it.  Solid nodes' moments are never used.
+//
+// Threads run over a list of the pairs that hold fluid (a pair with one solid
+// node, 4-8 % of the nodes in the benchmarks' packings, idles half), ordered
+// by tiles of 32 x kTileY x kTileZ nodes so that a block's loads share lines
+// in all three directions.  In each tile the pairs whose neighbours are all
+// fluid come first: a warp of such pairs skips the bounce-back selects.
 //
 // FP16 storage keeps its meaning: a population read by the gather is rounded
 // to half(f* - t_i rho_shift) exactly as the population kernels store it.
@@ -36,84 +47,163 @@
 
 namespace mlbm {
 
-constexpr int kMomThreads = 256;
-constexpr int kTileY = 4, kTileZ = 4;  // node list tiles: 32 x kTileY x kTileZ
-// Bit of a node list entry's neighbour word: the node lies on a face of the
-// box, so its psi and moments have ghost copies.
-constexpr uint32_t NB_EDGE = 1u << 21;
+constexpr int kTileX = 32, kTileY = 8, kTileZ = 4;  // order of the pair list
+constexpr int kMomThreads = 128;
+
+// Neighbour words of the lists (k_build_nbr's, bits 0-20) also hold:
+constexpr uint32_t NB_EDGE = 1u << 21;   // z = 0 or lz - 1: has an image
+constexpr uint32_t NB_INNER = 1u << 22;  // a pair's first word: 36 fluid links,
+                                         // no slab nodes
+constexpr uint32_t kNbAllFluid = 0x7ffffu;  // the node and its 18 sources
 
 template <typename R>
 struct alignas(4 * sizeof(R)) Mom {
   R d, x, y, z;  // density; velocity (m) or momentum (n)
 };
-
-// Call st(index) for a node and each of its periodic ghost copies.
-template <typename St>
-__device__ __forceinline__ void for_ghosts(const Geom& g, int x, int y, int z,
-                                           St st) {
-  const int xs[3] = {x, x == 0 ? g.lx : INT_MIN, x == g.lx - 1 ? -1 : INT_MIN};
-  const int ys[3] = {y, y == 0 ? g.ly : INT_MIN, y == g.ly - 1 ? -1 : INT_MIN};
-  const int zs[3] = {z, z == 0 ? g.lz : INT_MIN, z == g.lz - 1 ? -1 : INT_MIN};
-#pragma unroll 1
-  for (int c = 0; c < 3; ++c) {
-    if (zs[c] == INT_MIN) continue;
-#pragma unroll 1
-    for (int b = 0; b < 3; ++b) {
-      if (ys[b] == INT_MIN) continue;
-#pragma unroll
-      for (int a = 0; a < 3; ++a)
-        if (xs[a] != INT_MIN) st((uint32_t)psi_index(g, xs[a], ys[b], zs[c]));
-    }
-  }
-}
-
-struct MomNode {
-  uint32_t nb;
-  int x, y, z;
-  uint32_t i;  // psi_index
+template <typename R>
+struct alignas(8 * sizeof(R)) MomPair {
+  Mom<R> a, b;  // z, z + 1
+};
+template <typename R>
+struct alignas(2 * sizeof(R)) Two {
+  R a, b;
 };
 
-__device__ __forceinline__ MomNode mom_node(const Geom& g, uint2 e) {
-  MomNode n;
-  n.nb = e.x;
-  n.x = (int)(e.y & 2047u);
-  n.y = (int)((e.y >> 11) & 2047u);
-  n.z = (int)(e.y >> 22);
-  n.i = (uint32_t)((n.z + 1) * (g.ly + 2) + n.y + 1) * (uint32_t)g.pxg +
-        (uint32_t)n.x + 4u;
-  return n;
+// Pair of node (x, y, z), 0 <= x < lx, 0 <= y < ly, -1 <= z <= lz.
+__host__ __device__ __forceinline__ uint32_t pair_index(const Geom& g, int x, int y,
+                                                        int z) {
+  return (uint32_t)(((z + 2) >> 1) * g.ly + y) * (uint32_t)g.px + (uint32_t)x;
+}
+// (an odd lz: one plane more, read for the node beside the box's last one)
+__host__ __device__ __forceinline__ long long pair_elems(const Geom& g) {
+  return (long long)((g.lz + 3) / 2 + 1) * g.ly * g.px;
+}
+__host__ __device__ __forceinline__ size_t node_element(const Geom& g, int x, int y,
+                                                        int z) {
+  return 2 * (size_t)pair_index(g, x, y, z) + (z & 1);
 }
 
-// f*_i = feq_i of a node with moments m, for a node reached against (flip)
-// or along direction i: collide()'s equilibrium, operation for operation.
+// Offsets, in pairs, of the columns around a pair's (periodic in x and y) and
+// of the planes below and above it.
+struct Columns {
+  int xm, xp, ym, yp, plane;
+  __device__ __forceinline__ Columns(const Geom& g, int x, int y) {
+    const int row = g.px;
+    xm = x == 0 ? g.lx - 1 : -1;
+    xp = x == g.lx - 1 ? 1 - g.lx : 1;
+    ym = y == 0 ? (g.ly - 1) * row : -row;
+    yp = y == g.ly - 1 ? (1 - g.ly) * row : row;
+    plane = g.ly * row;
+  }
+  __device__ __forceinline__ int at(int dx, int dy) const {
+    return (dx < 0 ? xm : dx > 0 ? xp : 0) + (dy < 0 ? ym : dy > 0 ? yp : 0);
+  }
+};
+
+// Whole pairs move with one access (FP32: 32 bytes).
+__device__ __forceinline__ MomPair<float> ld_pair(const MomPair<float>* p) {
+  MomPair<float> v;
+  asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(v.a.d), "=f"(v.a.x), "=f"(v.a.y), "=f"(v.a.z), "=f"(v.b.d),
+                 "=f"(v.b.x), "=f"(v.b.y), "=f"(v.b.z)
+               : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void st_pair(MomPair<float>* p, const MomPair<float>& v) {
+  asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p),
+               "f"(v.a.d), "f"(v.a.x), "f"(v.a.y), "f"(v.a.z), "f"(v.b.d),
+               "f"(v.b.x), "f"(v.b.y), "f"(v.b.z)
+               : "memory");
+}
+__device__ __forceinline__ MomPair<double> ld_pair(const MomPair<double>* p) {
+  return *p;
+}
+__device__ __forceinline__ void st_pair(MomPair<double>* p, const MomPair<double>& v) {
+  *p = v;
+}
+
+// Call st(element) for the image of a node with z = 0 or z = lz - 1 (both in a
+// box of one plane).
+template <typename St>
+__device__ __forceinline__ void for_images(const Geom& g, int x, int y, int z, St st) {
+  if (z == 0) st(node_element(g, x, y, g.lz));
+  if (z == g.lz - 1) st(node_element(g, x, y, -1));
+}
+
+// ---- the pair list --------------------------------------------------------------
+struct PairList {
+  const uint2* words;   // neighbour words of z and z + 1 (0: solid, outside)
+  const uint32_t* xyz;  // pack_xyz of the first node (z even)
+  int count;
+};
+struct PairAt {
+  uint32_t na, nb;
+  int x, y, z;
+  uint32_t at;  // pair_index
+};
+__device__ __forceinline__ PairAt pair_at(const Geom& g, const PairList& l, int k) {
+  const uint2 w = __ldg(l.words + k);
+  const uint32_t c = __ldg(l.xyz + k);
+  PairAt q;
+  q.na = w.x;
+  q.nb = w.y;
+  q.x = (int)(c & 2047u);
+  q.y = (int)((c >> 11) & 2047u);
+  q.z = (int)(c >> 22);
+  q.at = pair_index(g, q.x, q.y, q.z);
+  return q;
+}
+
+__host__ __device__ constexpr int direction(int dx, int dy, int dz) {
+  for (int i = 0; i < Q; ++i)
+    if (ex(i) == dx && ey(i) == dy && ez(i) == dz) return i;
+  return -1;
+}
+
+// ---- equilibrium ----------------------------------------------------------------
+// A node's moments with what every population of it shares.
 template <typename R>
-__device__ __forceinline__ R eq_population(int i, const Mom<R>& m, bool flip) {
-  const R usq15 = rmul(R(1.5), rfma(m.z, m.z, rfma(m.y, m.y, rmul(m.x, m.x))));
-  const R base = rsub(R(1), usq15);
-  if (i == 0) return rmul(rmul(weight<R>(0), m.d), base);
+struct Source {
+  Mom<R> m;
+  R base, wd1, wd2;  // 1 - 1.5 u^2; axis and diagonal weight times rho
+  __device__ __forceinline__ explicit Source(const Mom<R>& v) : m(v) {
+    base = rsub(R(1), rmul(R(1.5), rfma(v.z, v.z, rfma(v.y, v.y, rmul(v.x, v.x)))));
+    wd1 = rmul(weight<R>(1), v.d);
+    wd2 = rmul(weight<R>(4), v.d);
+  }
+};
+
+// feq_i of collide(), operation for operation.
+template <typename R>
+__device__ __forceinline__ R eq_population(int i, const Source<R>& s) {
+  if (i == 0) return rmul(rmul(weight<R>(0), s.m.d), s.base);
   R eu = R(0);
-  if (ex(i)) eu = ex(i) > 0 ? m.x : -m.x;
-  if (ey(i)) eu = ex(i) ? (ey(i) > 0 ? radd(eu, m.y) : rsub(eu, m.y))
-                        : (ey(i) > 0 ? m.y : -m.y);
-  if (ez(i)) eu = ex(i) || ey(i) ? (ez(i) > 0 ? radd(eu, m.z) : rsub(eu, m.z))
-                                 : (ez(i) > 0 ? m.z : -m.z);
-  eu = flip ? -eu : eu;
-  const R sym = rfma(rmul(R(4.5), eu), eu, base);
-  const R anti = rmul(R(3), eu);
-  const R wd = rmul(weight<R>(i), m.d);
-  return rmul(wd, radd(sym, anti));
+  if (ex(i)) eu = ex(i) > 0 ? s.m.x : -s.m.x;
+  if (ey(i)) eu = ex(i) ? (ey(i) > 0 ? radd(eu, s.m.y) : rsub(eu, s.m.y))
+                        : (ey(i) > 0 ? s.m.y : -s.m.y);
+  if (ez(i)) eu = ex(i) || ey(i) ? (ez(i) > 0 ? radd(eu, s.m.z) : rsub(eu, s.m.z))
+                                 : (ez(i) > 0 ? s.m.z : -s.m.z);
+  const R sym = rfma(rmul(R(4.5), eu), eu, s.base);
+  const bool axis = ex(i) * ex(i) + ey(i) * ey(i) + ez(i) * ez(i) == 1;
+  return rmul(axis ? s.wd1 : s.wd2, radd(sym, rmul(R(3), eu)));
 }
 
-// A population as the storage format T holds it: stored with shift s_st,
-// read back with shift s_ld (both t_i times a rho_shift).
+// Both nodes' population as the storage format T holds it: stored with shift
+// s_st, read back with shift s_ld (both t_i times a rho_shift).
 template <typename T>
-__device__ __forceinline__ typename Pop<T>::Real stored(
-    typename Pop<T>::Real f, typename Pop<T>::Real s_st,
-    typename Pop<T>::Real s_ld) {
-  T v;
-  Pop<T>::st(&v, f, s_st);
-  return Pop<T>::ld(&v, s_ld);
-}
+struct Stored {
+  using R = typename Pop<T>::Real;
+  static __device__ __forceinline__ Two<R> pass(Two<R> f, float, float) { return f; }
+};
+template <>
+struct Stored<__half> {
+  static __device__ __forceinline__ Two<float> pass(Two<float> f, float s_st,
+                                                    float s_ld) {
+    const float2 v = __half22float2(__float22half2_rn(
+        make_float2(__fsub_rn(f.a, s_st), __fsub_rn(f.b, s_st))));
+    return Two<float>{__fadd_rn(v.x, s_ld), __fadd_rn(v.y, s_ld)};
+  }
+};
 
 // Density injection with its step test hoisted out (inject_on for any R).
 template <typename R>
@@ -129,162 +219,269 @@ __device__ __forceinline__ R mom_inject(const Phys& p, const Geom& g,
   }
 }
 
-// rho and j of the populations f, in the order of sum_density() / collide();
-// injection and the slab density applied to rho.
+// One population into a node's sums, in the order of sum_density() / collide().
 template <typename R>
-__device__ __forceinline__ Mom<R> mom_sums(const Phys& p, const Geom& g,
-                                           const StepArgs& a, bool inj, int y,
-                                           const R (&f)[Q]) {
-  Mom<R> n{R(0), R(0), R(0), R(0)};
-#pragma unroll
-  for (int i = 0; i < Q; ++i) {
-    n.d = radd(n.d, f[i]);
-    if (ex(i)) n.x = ex(i) > 0 ? radd(n.x, f[i]) : rsub(n.x, f[i]);
-    if (ey(i)) n.y = ey(i) > 0 ? radd(n.y, f[i]) : rsub(n.y, f[i]);
-    if (ez(i)) n.z = ez(i) > 0 ? radd(n.z, f[i]) : rsub(n.z, f[i]);
-  }
-  n.d = mom_inject<R>(p, g, a, inj, y, n.d);
-  return n;
+__device__ __forceinline__ void mom_sum(int i, R f, Mom<R>& n) {
+  n.d = radd(n.d, f);
+  if (ex(i)) n.x = ex(i) > 0 ? radd(n.x, f) : rsub(n.x, f);
+  if (ey(i)) n.y = ey(i) > 0 ? radd(n.y, f) : rsub(n.y, f);
+  if (ez(i)) n.z = ez(i) > 0 ? radd(n.z, f) : rsub(n.z, f);
 }
 
-// What a gather leaves of one node.
+// What a gather leaves of one pair: its sums, after injection and the slabs'
+// densities, and psi (and rho).
 template <typename R, bool WRITE_RHO>
-__device__ __forceinline__ void mom_put(const MomNode& q, const Mom<R>& s,
-                                        Mom<R>* n, int k, R* rho, R* psi,
-                                        const Geom& g, const Phys& p) {
-  n[k] = s;
-  if (WRITE_RHO) rho[node_index(g, q.x, q.y, q.z)] = s.d;
-  const R v = psi_of<R>(p, s.d);
-  if (q.nb & NB_EDGE)
-    for_ghosts(g, q.x, q.y, q.z, [&](uint32_t i) { psi[i] = v; });
-  else
-    psi[q.i] = v;
+__device__ __forceinline__ void mom_put(const PairAt& q, MomPair<R> s,
+                                        MomPair<R>* n, int k, R* rho, R* psi,
+                                        const Geom& g, const Phys& p,
+                                        const StepArgs& a, bool inj) {
+  const int kind = nb_kind(q.na | q.nb);  // the same x: the same slab
+  if (kind) {
+    const R d = R(slab_density(p, kind));
+    s.a = s.b = Mom<R>{d, R(0), R(0), R(0)};
+  } else {
+    s.a.d = mom_inject<R>(p, g, a, inj, q.y, s.a.d);
+    s.b.d = mom_inject<R>(p, g, a, inj, q.y, s.b.d);
+  }
+  st_pair(n + k, s);
+  const R va = psi_of<R>(p, s.a.d), vb = psi_of<R>(p, s.b.d);
+  if (WRITE_RHO) {
+    const int at = (int)node_index(g, q.x, q.y, q.z);
+    if (q.na) rho[at] = s.a.d;
+    if (q.nb) rho[at + g.ly * g.px] = s.b.d;
+  }
+  if (q.na & q.nb & NB_SELF) {
+    *reinterpret_cast<Two<R>*>(psi + 2 * (size_t)q.at) = Two<R>{va, vb};
+  } else {  // a solid node keeps its psi, a ghost node its image's
+    psi[2 * (size_t)q.at + (q.na ? 0 : 1)] = q.na ? va : vb;
+  }
+  if ((q.na | q.nb) & NB_EDGE) {
+    if (q.na) for_images(g, q.x, q.y, q.z, [&](size_t i) { psi[i] = va; });
+    if (q.nb) for_images(g, q.x, q.y, q.z + 1, [&](size_t i) { psi[i] = vb; });
+  }
 }
 
-// Gather pass from moments.  m is read with plain loads only after the gate:
-// the launch before wrote it.
-template <typename T, bool WRITE_RHO>
-__device__ __forceinline__ void mom_gather(const Mom<typename Pop<T>::Real>* m,
-                                           uint2 e, int k,
-                                           Mom<typename Pop<T>::Real>* n,
-                                           typename Pop<T>::Real* rho,
-                                           typename Pop<T>::Real* psi,
-                                           const Geom& g, const Phys& p,
-                                           const StepArgs& a, bool inj,
-                                           float shift_st) {
+// ---- kernels ----------------------------------------------------------------------
+
+// The populations of one pair, in the order the sums take them.
+template <typename T, bool INNER>
+struct Gather {
   using R = typename Pop<T>::Real;
-  const MomNode q = mom_node(g, e);
-  Mom<R> s;
-  if (nb_kind(q.nb)) {
-    s = Mom<R>{R(slab_density(p, nb_kind(q.nb))), R(0), R(0), R(0)};
-  } else {
-    const int sy = g.pxg, sz = (g.ly + 2) * g.pxg;
-    const R st = R(shift_st), ld = R(p.rho_shift);
-    R f[Q];
-#pragma unroll
-    for (int i = 0; i < Q; ++i) {
-      const bool own = i == 0 || !((q.nb >> i) & 1u);
-      const int o = ex(i) + ey(i) * sy + ez(i) * sz;
-      const Mom<R> v = m[own ? q.i : q.i - o];
-      f[i] = stored<T>(eq_population<R>(i, v, i != 0 && own), st * weight<R>(i),
-                       ld * weight<R>(i));
-    }
-    s = mom_sums<R>(p, g, a, inj, q.y, f);
-  }
-  mom_put<R, WRITE_RHO>(q, s, n, k, rho, psi, g, p);
-}
+  const MomPair<R>* at;  // the pair's own moments
+  Columns col;
+  uint32_t na, nb;
+  float st, ld;
+  MomPair<R> own, sum;
 
-// Collide pass.
-template <typename R, bool WRITE_U>
-__device__ __forceinline__ void mom_collide(const Mom<R>* n, uint2 e, int k,
-                                            const R* psi, Mom<R>* m, float* vel,
-                                            const Geom& g, const Phys& p) {
-  const MomNode q = mom_node(g, e);
-  Mom<R> s = n[k];
-  if (nb_kind(q.nb)) {
-    s.x = s.y = s.z = R(0);
-  } else {
-    const int py = g.pxg, pz = (g.ly + 2) * g.pxg;
-    R sx = R(0), sy = R(0), sz = R(0);
-#pragma unroll
-    for (int i = 1; i < Q; ++i) {
-      const R wp = rmul(weight<R>(i), psi[q.i + (ex(i) + ey(i) * py + ez(i) * pz)]);
-      if (ex(i)) sx = ex(i) > 0 ? radd(sx, wp) : rsub(sx, wp);
-      if (ey(i)) sy = ey(i) > 0 ? radd(sy, wp) : rsub(sy, wp);
-      if (ez(i)) sz = ez(i) > 0 ? radd(sz, wp) : rsub(sz, wp);
+  // f_i of both nodes from the sources sa, sb
+  __device__ __forceinline__ Two<R> population(int i, const Source<R>& sa,
+                                               const Source<R>& sb) {
+    Two<R> f{eq_population<R>(i, sa), eq_population<R>(i, sb)};
+    if (!INNER && i) {
+      const int o = opp(i);
+      const R oa = eq_population<R>(o, Source<R>(own.a)),
+              ob = eq_population<R>(o, Source<R>(own.b));
+      f.a = (na >> i) & 1u ? f.a : oa;
+      f.b = (nb >> i) & 1u ? f.b : ob;
     }
-    const R gp = rmul(-R(p.G), psi[q.i]);
-    const R tau = R(p.tau);
-    const R inv_rho = rrcp(s.d);
-    s.x = rmul(rfma(tau, rmul(gp, sx), s.x), inv_rho);
-    s.y = rmul(rfma(tau, rmul(gp, sy), s.y), inv_rho);
-    s.z = rmul(rfma(tau, rmul(gp, sz), s.z), inv_rho);
+    return Stored<T>::pass(f, st * weight<float>(i), ld * weight<float>(i));
   }
-  if (WRITE_U) {
-    float* v = vel + 3 * node_index(g, q.x, q.y, q.z);
-    v[0] = (float)s.x;
-    v[1] = (float)s.y;
-    v[2] = (float)s.z;
+  // the three populations from the column (dx, dy): levels z - 1 .. z + 2
+  __device__ __forceinline__ void column(int dx, int dy, Two<R>& f0, Two<R>& up,
+                                         Two<R>& down) {
+    const MomPair<R>* c = at + col.at(dx, dy);
+    const MomPair<R> mid = dx || dy ? ld_pair(c) : own;
+    const Source<R> lo((c - col.plane)->b), a(mid.a), b(mid.b),
+        hi((c + col.plane)->a);
+    f0 = population(direction(-dx, -dy, 0), a, b);
+    up = population(direction(-dx, -dy, 1), lo, a);
+    down = population(direction(-dx, -dy, -1), b, hi);
   }
-  if (q.nb & NB_EDGE)
-    for_ghosts(g, q.x, q.y, q.z, [&](uint32_t i) { m[i] = s; });
-  else
-    m[q.i] = s;
-}
+  __device__ __forceinline__ Two<R> diagonal(int dx, int dy) {
+    const MomPair<R> mid = ld_pair(at + col.at(dx, dy));
+    return population(direction(-dx, -dy, 0), Source<R>(mid.a), Source<R>(mid.b));
+  }
+  __device__ __forceinline__ void add(int i, const Two<R>& f) {
+    mom_sum(i, f.a, sum.a);
+    mom_sum(i, f.b, sum.b);
+  }
+  __device__ __forceinline__ void run() {
+    own = ld_pair(at);
+    sum.a = sum.b = Mom<R>{R(0), R(0), R(0), R(0)};
+    Two<R> f0, f3, f12, f1, f6, f7, f2, f8, f9;
+    column(0, 0, f0, f12, f3);
+    add(0, f0);
+    column(1, 0, f1, f7, f6);
+    add(1, f1);
+    column(0, 1, f2, f9, f8);
+    add(2, f2);
+    add(3, f3);
+    add(4, diagonal(1, 1));
+    add(5, diagonal(1, -1));
+    add(6, f6);
+    add(7, f7);
+    add(8, f8);
+    add(9, f9);
+    Two<R> f10, f15, f16, f11, f17, f18;
+    column(-1, 0, f10, f15, f16);
+    add(10, f10);
+    column(0, -1, f11, f17, f18);
+    add(11, f11);
+    add(12, f12);
+    add(13, diagonal(-1, -1));
+    add(14, diagonal(-1, 1));
+    add(15, f15);
+    add(16, f16);
+    add(17, f17);
+    add(18, f18);
+  }
+};
 
-// ---- kernels ----------------------------------------------------------------
+template <typename T>
+constexpr int mom_gather_blocks() { return sizeof(typename Pop<T>::Real) == 8 ? 4 : 6; }
 
 template <typename T, bool WRITE_RHO>
-__global__ void __launch_bounds__(kMomThreads, 3)
-    k_mom_gather(const Mom<typename Pop<T>::Real>* m,
-                 const uint2* __restrict__ list, int count,
-                 Mom<typename Pop<T>::Real>* n, typename Pop<T>::Real* rho,
-                 typename Pop<T>::Real* psi, Geom g, Phys p, StepArgs a,
-                 bool inj, float shift_st) {
+__global__ void __launch_bounds__(kMomThreads, mom_gather_blocks<T>())
+    k_mom_gather(const MomPair<typename Pop<T>::Real>* m, PairList list,
+                 MomPair<typename Pop<T>::Real>* n, typename Pop<T>::Real* rho,
+                 typename Pop<T>::Real* psi, Geom g, Phys p, StepArgs a, bool inj,
+                 float shift_st) {
+  using R = typename Pop<T>::Real;
   const int k = blockIdx.x * kMomThreads + threadIdx.x;
-  if (k >= count) return;
-  const uint2 e = __ldg(list + k);
+  const bool some = k < list.count;
+  const PairAt q = pair_at(g, list, some ? k : list.count - 1);
+  const bool inner = __all_sync(~0u, q.na & NB_INNER);
   pdl_gate<true>();
-  mom_gather<T, WRITE_RHO>(m, e, k, n, rho, psi, g, p, a, inj, shift_st);
+  if (!some) return;
+  MomPair<R> s;
+  if (inner) {
+    Gather<T, true> c{m + q.at, Columns(g, q.x, q.y), q.na, q.nb, shift_st, p.rho_shift};
+    c.run();
+    s = c.sum;
+  } else {
+    Gather<T, false> c{m + q.at, Columns(g, q.x, q.y), q.na, q.nb, shift_st, p.rho_shift};
+    c.run();
+    s = c.sum;
+  }
+  mom_put<R, WRITE_RHO>(q, s, n, k, rho, psi, g, p, a, inj);
 }
 
 // The gather of a step that starts from populations (the dense layout in AA
 // phase PHASE): initial states, restored checkpoints, another tau before.
+template <typename T, int PHASE>
+__device__ __forceinline__ Mom<typename Pop<T>::Real> gather_node(
+    const T* __restrict__ pop, uint32_t nb, int x, int y, int z, const Geom& g,
+    const Phys& p) {
+  using R = typename Pop<T>::Real;
+  Mom<R> s{R(0), R(0), R(0), R(0)};
+  if (!(nb & NB_SELF) || nb_kind(nb)) return s;
+  Nbr w;
+  w.init(g, x, y, z);
+  R f[Q];
+  gather<T, PHASE>(pop, g.plane, w, nb, w.n, R(p.rho_shift), f);
+#pragma unroll
+  for (int i = 0; i < Q; ++i) mom_sum(i, f[i], s);
+  return s;
+}
+
 template <typename T, int PHASE, bool WRITE_RHO>
 __global__ void __launch_bounds__(kMomThreads)
-    k_mom_gather_pop(const T* __restrict__ pop, const uint2* __restrict__ list,
-                     int count, Mom<typename Pop<T>::Real>* n,
-                     typename Pop<T>::Real* rho, typename Pop<T>::Real* psi,
-                     Geom g, Phys p, StepArgs a, bool inj) {
+    k_mom_gather_pop(const T* __restrict__ pop, PairList list,
+                     MomPair<typename Pop<T>::Real>* n, typename Pop<T>::Real* rho,
+                     typename Pop<T>::Real* psi, Geom g, Phys p, StepArgs a,
+                     bool inj) {
   using R = typename Pop<T>::Real;
   const int k = blockIdx.x * kMomThreads + threadIdx.x;
-  if (k >= count) return;
-  const MomNode q = mom_node(g, __ldg(list + k));
-  Mom<R> s;
-  if (nb_kind(q.nb)) {
-    s = Mom<R>{R(slab_density(p, nb_kind(q.nb))), R(0), R(0), R(0)};
-  } else {
-    Nbr w;
-    w.init(g, q.x, q.y, q.z);
-    R f[Q];
-    gather<T, PHASE>(pop, g.plane, w, q.nb, w.n, R(p.rho_shift), f);
-    s = mom_sums<R>(p, g, a, inj, q.y, f);
-  }
-  mom_put<R, WRITE_RHO>(q, s, n, k, rho, psi, g, p);
+  if (k >= list.count) return;
+  const PairAt q = pair_at(g, list, k);
+  MomPair<R> s;
+  s.a = gather_node<T, PHASE>(pop, q.na, q.x, q.y, q.z, g, p);
+  s.b = gather_node<T, PHASE>(pop, q.nb, q.x, q.y, q.z + 1, g, p);
+  mom_put<R, WRITE_RHO>(q, s, n, k, rho, psi, g, p, a, inj);
+}
+
+// Force, velocity shift of one node: collide()'s, operation for operation.
+// s holds w_i psi sums; n the density and momentum.
+template <typename R>
+__device__ __forceinline__ void force_add(int i, R psi, R& sx, R& sy, R& sz) {
+  const R wp = rmul(weight<R>(i), psi);
+  if (ex(i)) sx = ex(i) > 0 ? radd(sx, wp) : rsub(sx, wp);
+  if (ey(i)) sy = ey(i) > 0 ? radd(sy, wp) : rsub(sy, wp);
+  if (ez(i)) sz = ez(i) > 0 ? radd(sz, wp) : rsub(sz, wp);
+}
+template <typename R>
+__device__ __forceinline__ Mom<R> shifted_velocity(const Phys& p, const Mom<R>& n,
+                                                   R psi, R sx, R sy, R sz,
+                                                   int kind) {
+  if (kind) return Mom<R>{n.d, R(0), R(0), R(0)};
+  const R gp = rmul(-R(p.G), psi), tau = R(p.tau), inv = rrcp(n.d);
+  return Mom<R>{n.d, rmul(rfma(tau, rmul(gp, sx), n.x), inv),
+                rmul(rfma(tau, rmul(gp, sy), n.y), inv),
+                rmul(rfma(tau, rmul(gp, sz), n.z), inv)};
 }
 
 // Blocks run in reverse list order: what the gather wrote last is still in L2
 // when the collide starts with it, and the next gather starts where the
 // collide ended.
 template <typename R, bool WRITE_U>
-__global__ void __launch_bounds__(kMomThreads, 4)
-    k_mom_collide(const Mom<R>* n, const uint2* __restrict__ list, int count,
-                  const R* psi, Mom<R>* m, float* vel, Geom g, Phys p) {
+__global__ void __launch_bounds__(kMomThreads, 8)
+    k_mom_collide(const MomPair<R>* n, PairList list, const Two<R>* psi,
+                  MomPair<R>* m, float* vel, Geom g, Phys p) {
   const int k = (int)(gridDim.x - 1 - blockIdx.x) * kMomThreads + threadIdx.x;
-  if (k >= count) return;
-  const uint2 e = __ldg(list + k);
+  if (k >= list.count) return;
+  const PairAt q = pair_at(g, list, k);
+  const Columns col(g, q.x, q.y);
   pdl_gate<true>();
-  mom_collide<R, WRITE_U>(n, e, k, psi, m, vel, g, p);
+  const MomPair<R> s = ld_pair(n + k);
+  const Two<R>* at = psi + q.at;
+  // psi of the columns: [dy + 1][dx + 1], levels z - 1, z, z + 1, z + 2
+  Two<R> mid[9];
+  R lo[9], hi[9];
+#pragma unroll
+  for (int j = 0; j < 9; ++j) {
+    const int dx = j % 3 - 1, dy = j / 3 - 1;
+    const Two<R>* c = at + col.at(dx, dy);
+    mid[j] = *c;
+    if (dx * dy == 0) {
+      lo[j] = (c - col.plane)->b;
+      hi[j] = (c + col.plane)->a;
+    }
+  }
+  R ax = R(0), ay = R(0), az = R(0), bx = R(0), by = R(0), bz = R(0);
+#pragma unroll
+  for (int i = 1; i < Q; ++i) {
+    const int j = (ey(i) + 1) * 3 + ex(i) + 1;
+    force_add(i, ez(i) == 0 ? mid[j].a : ez(i) > 0 ? mid[j].b : lo[j], ax, ay, az);
+    force_add(i, ez(i) == 0 ? mid[j].b : ez(i) > 0 ? hi[j] : mid[j].a, bx, by, bz);
+  }
+  const int kind = nb_kind(q.na | q.nb);
+  MomPair<R> u;
+  u.a = shifted_velocity<R>(p, s.a, mid[4].a, ax, ay, az, kind);
+  u.b = shifted_velocity<R>(p, s.b, mid[4].b, bx, by, bz, kind);
+  if (WRITE_U) {
+    const long long at0 = node_index(g, q.x, q.y, q.z);
+    float* v = vel + 3 * at0;
+    if (q.na) {
+      v[0] = (float)u.a.x;
+      v[1] = (float)u.a.y;
+      v[2] = (float)u.a.z;
+    }
+    v += 3ll * g.ly * g.px;
+    if (q.nb) {
+      v[0] = (float)u.b.x;
+      v[1] = (float)u.b.y;
+      v[2] = (float)u.b.z;
+    }
+  }
+  Mom<R>* mm = reinterpret_cast<Mom<R>*>(m);
+  if (q.na && q.nb)
+    st_pair(m + q.at, u);
+  else  // the other half may be a ghost node (odd lz)
+    mm[2 * (size_t)q.at + (q.na ? 0 : 1)] = q.na ? u.a : u.b;
+  if ((q.na | q.nb) & NB_EDGE) {
+    if (q.na) for_images(g, q.x, q.y, q.z, [&](size_t i) { mm[i] = u.a; });
+    if (q.nb) for_images(g, q.x, q.y, q.z + 1, [&](size_t i) { mm[i] = u.b; });
+  }
 }
 
 // The populations of the fluid nodes, in the dense layout in AA phase PHASE
@@ -292,86 +489,120 @@ __global__ void __launch_bounds__(kMomThreads, 4)
 // after the same steps, bit for bit.
 template <typename T, int PHASE>
 __global__ void __launch_bounds__(kMomThreads)
-    k_mom_populations(const Mom<typename Pop<T>::Real>* __restrict__ m,
-                      const uint2* __restrict__ list, int count,
-                      T* __restrict__ pop, Geom g, float shift_st) {
+    k_mom_populations(const MomPair<typename Pop<T>::Real>* __restrict__ m,
+                      PairList list, T* __restrict__ pop, Geom g, float shift_st) {
   using R = typename Pop<T>::Real;
   const int k = blockIdx.x * kMomThreads + threadIdx.x;
-  if (k >= count) return;
-  const MomNode q = mom_node(g, __ldg(list + k));
-  const Mom<R> v = m[q.i];
-  R f[Q];
+  if (k >= list.count) return;
+  const PairAt q = pair_at(g, list, k);
+  const MomPair<R> v = m[q.at];
+  for (int b = 0; b < 2; ++b) {
+    const uint32_t nb = b ? q.nb : q.na;
+    if (!nb) continue;
+    const Source<R> s(b ? v.b : v.a);
+    R f[Q];
 #pragma unroll
-  for (int i = 0; i < Q; ++i) f[i] = eq_population<R>(i, v, false);
-  Nbr w;
-  w.init(g, q.x, q.y, q.z);
-  scatter<T, PHASE ^ 1>(pop, g.plane, w, q.nb, w.n, R(shift_st), f);
+    for (int i = 0; i < Q; ++i) f[i] = eq_population<R>(i, s);
+    Nbr w;
+    w.init(g, q.x, q.y, q.z + b);
+    scatter<T, PHASE ^ 1>(pop, g.plane, w, nb, w.n, R(shift_st), f);
+  }
 }
 
-// ---- node list ----------------------------------------------------------------
-// Mask words in tile order: word t of the list's order -> (x / 32, y, z).
-__device__ __forceinline__ bool mom_tile_word(const Geom& g, long long t, int& w,
-                                              int& y, int& z) {
-  const int nty = (g.ly + kTileY - 1) / kTileY;
-  const int in = (int)(t % (kTileY * kTileZ));
-  long long tile = t / (kTileY * kTileZ);
-  w = (int)(tile % g.wpr);
-  tile /= g.wpr;
-  y = (int)(tile % nty) * kTileY + in % kTileY;
-  z = (int)(tile / nty) * kTileZ + in / kTileY;
-  return y < g.ly && z < g.lz;
-}
-__host__ __device__ __forceinline__ long long mom_tile_words(const Geom& g) {
-  return (long long)((g.ly + kTileY - 1) / kTileY) * ((g.lz + kTileZ - 1) / kTileZ) *
-         g.wpr * kTileY * kTileZ;
+// psi of every node into the paired layout, the images in z included (the
+// solid nodes' psi(rhos), which only initialisation writes).
+template <typename R>
+__global__ void k_mom_psi(const R* __restrict__ psi, R* __restrict__ out, Geom g) {
+  const int x = blockIdx.x * 32 + threadIdx.x;
+  const int y = blockIdx.y * blockDim.y + threadIdx.y;
+  const int z = (int)blockIdx.z - 1;
+  if (x >= g.lx || y >= g.ly) return;
+  out[node_element(g, x, y, z)] = psi[psi_index(g, x, y, z)];
 }
 
-static __global__ void k_mom_counts(const uint32_t* __restrict__ mask,
-                                    uint32_t* __restrict__ counts,
-                                    long long nwords, Geom g) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t > nwords) return;
-  int w, y, z;
-  uint32_t c = 0;
-  if (t < nwords && mom_tile_word(g, t, w, y, z))
-    c = __popc(mask[((long long)z * g.ly + y) * g.wpr + w]);
-  counts[t] = c;
+// ---- tiles and lists -----------------------------------------------------------
+struct TileGrid {
+  int nx, ny, nz;
+  __host__ __device__ explicit TileGrid(const Geom& g)
+      : nx((g.lx + kTileX - 1) / kTileX), ny((g.ly + kTileY - 1) / kTileY),
+        nz((g.lz + kTileZ - 1) / kTileZ) {}
+  __host__ __device__ long long count() const { return (long long)nx * ny * nz; }
+};
+
+constexpr int kPairRows = kTileY * kTileZ / 2;
+__device__ __forceinline__ uint32_t tile_word(const uint32_t* __restrict__ nbw,
+                                              const Geom& g, int x, int y, int z) {
+  if (x >= g.lx || y >= g.ly || z >= g.lz) return 0u;
+  const uint32_t nb = nbw[node_index(g, x, y, z)];
+  if (!(nb & NB_SELF)) return 0u;
+  return nb | (z == 0 || z == g.lz - 1 ? NB_EDGE : 0u);
 }
 
-__device__ __forceinline__ uint32_t mom_word(const uint32_t* __restrict__ nbw,
-                                             const Geom& g, int x, int y, int z) {
-  const bool edge = x == 0 || y == 0 || z == 0 || x == g.lx - 1 ||
-                    y == g.ly - 1 || z == g.lz - 1;
-  return nbw[node_index(g, x, y, z)] | (edge ? NB_EDGE : 0u);
-}
+// One block of kPairRows warps per tile (warp = row (y, z / 2), lane = x).
+// COUNT: counts[tile] = its pairs and nodes, for the host's scan.  Otherwise
+// the lists, at the places at[tile] that the scan gave.  nodes: the fluid
+// nodes one by one (neighbour word, packed coordinates), which the statistics
+// walk.
+struct TileCount {
+  uint32_t pairs, nodes;
+};
+struct TileCountSum {
+  __host__ __device__ TileCount operator()(const TileCount& a,
+                                           const TileCount& b) const {
+    return TileCount{a.pairs + b.pairs, a.nodes + b.nodes};
+  }
+};
 
-// The list's neighbour words again (a new initial state may move the slabs).
-static __global__ void k_mom_words(const uint32_t* __restrict__ nbw,
-                                   uint2* __restrict__ list, int count, Geom g) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count) return;
-  const uint32_t c = list[k].y;
-  list[k].x = mom_word(nbw, g, (int)(c & 2047u), (int)((c >> 11) & 2047u),
-                       (int)(c >> 22));
-}
-
-// One warp per mask word; start[t] = list place of the word's first node.
-static __global__ void k_mom_list(const uint32_t* __restrict__ mask,
-                                  const uint32_t* __restrict__ nbw,
-                                  const uint32_t* __restrict__ start,
-                                  uint2* __restrict__ list, long long nwords,
-                                  Geom g) {
-  const long long t =
-      ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32;
-  if (t >= nwords) return;
-  const int lane = threadIdx.x & 31;
-  int w, y, z;
-  if (!mom_tile_word(g, t, w, y, z)) return;
-  const uint32_t bits = mask[((long long)z * g.ly + y) * g.wpr + w];
-  if (!((bits >> lane) & 1u)) return;
-  const int x = 32 * w + lane;
-  list[start[t] + __popc(bits & low_bits(lane))] =
-      make_uint2(mom_word(nbw, g, x, y, z), pack_xyz(x, y, z));
+template <bool COUNT>
+__global__ void __launch_bounds__(32 * kPairRows)
+    k_mom_tiles(const uint32_t* __restrict__ nbw, TileCount* counts,
+                const TileCount* __restrict__ at, uint2* __restrict__ words,
+                uint32_t* __restrict__ xyz, uint2* __restrict__ nodes, Geom g) {
+  __shared__ uint32_t row_in[kPairRows], row_out[kPairRows], row_nodes[kPairRows];
+  const TileGrid tg(g);
+  const long long tile = blockIdx.x;
+  const int lane = threadIdx.x & 31, row = threadIdx.x / 32;
+  const int x = (int)(tile % tg.nx) * kTileX + lane,
+            y = (int)(tile / tg.nx % tg.ny) * kTileY + row % kTileY,
+            z = (int)(tile / ((long long)tg.nx * tg.ny)) * kTileZ + row / kTileY * 2;
+  const uint32_t na = tile_word(nbw, g, x, y, z), nb = tile_word(nbw, g, x, y, z + 1);
+  const bool any = (na | nb) != 0u;
+  const bool in = ((na & nb) & kNbAllFluid) == kNbAllFluid && !nb_kind(na);
+  const uint32_t bin = __ballot_sync(~0u, in), bout = __ballot_sync(~0u, any && !in);
+  const uint32_t ba = __ballot_sync(~0u, na != 0u), bb = __ballot_sync(~0u, nb != 0u);
+  if (lane == 0) {
+    row_in[row] = __popc(bin);
+    row_out[row] = __popc(bout);
+    row_nodes[row] = __popc(ba) + __popc(bb);
+  }
+  __syncthreads();
+  uint32_t inner = 0, outer = 0, count = 0, in0 = 0, out0 = 0, nodes0 = 0;
+  for (int r = 0; r < kPairRows; ++r) {
+    if (r == row) {
+      in0 = inner;
+      out0 = outer;
+      nodes0 = count;
+    }
+    inner += row_in[r];
+    outer += row_out[r];
+    count += row_nodes[r];
+  }
+  if (COUNT) {
+    if (threadIdx.x == 0) counts[tile] = TileCount{inner + outer, count};
+    return;
+  }
+  const TileCount w = at[tile];
+  const uint32_t below = (1u << lane) - 1u;
+  if (any) {
+    const uint32_t k = w.pairs + (in ? in0 + __popc(bin & below)
+                                     : inner + out0 + __popc(bout & below));
+    words[k] = make_uint2(na | (in ? NB_INNER : 0u), nb);
+    xyz[k] = pack_xyz(x, y, z);
+  }
+  const uint32_t k = w.nodes + nodes0;
+  if (na) nodes[k + __popc(ba & below)] = make_uint2(na, pack_xyz(x, y, z));
+  if (nb)
+    nodes[k + __popc(ba) + __popc(bb & below)] = make_uint2(nb, pack_xyz(x, y, z + 1));
 }
 
 }  // namespace mlbm
