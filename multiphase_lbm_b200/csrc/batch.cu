@@ -12,6 +12,7 @@
 #include "../../include/mlbm_batch.h"
 #include "batch.cuh"
 #include "batch_compact.cuh"
+#include "batch_moments.cuh"
 #include "capi_internal.h"
 
 using namespace mlbm;
@@ -47,6 +48,13 @@ struct mlbm_batch {
   long long* d_cpre = nullptr;
   int ccap = 0;
   int grid_c = 0, grid_cu = 0;
+  // moment mode (every domain with tau = 1): the domains are held as moments
+  // and every pass is one launch over all of them (batch_moments.cuh)
+  bool moments = false;
+  MomDomain* d_mdesc = nullptr;
+  MomBlock* d_mblocks = nullptr;
+  int mcap = 0, mblocks_cap = 0;
+  int grid_m = 0;
 };
 
 namespace {
@@ -151,6 +159,101 @@ mlbm_status rebuild_compact(mlbm_batch* b) {
   return MLBM_OK;
 }
 
+// Moment mode: tables of the domains, all held as moments.
+mlbm_status rebuild_moments(mlbm_batch* b) {
+  std::vector<MomDomain> desc;
+  std::vector<MomBlock> blocks;
+  for (size_t s = 0; s < b->dom.size(); ++s) {
+    const mlbm_lattice* lat = b->dom[s];
+    if (!lat) continue;
+    const MomentState& ms = lat->mom;
+    MomDomain d;
+    std::memset(&d, 0, sizeof d);
+    d.g = lat->g;
+    d.p = lat->phys;
+    d.m = ms.m;
+    d.n = ms.n;
+    d.psi = ms.psi;
+    d.rho = lat->rho;
+    d.list = PairList{ms.words, ms.xyz, ms.npairs};
+    d.step_origin = b->origin[s];
+    for (int k = 0; k < ms.npairs; k += kMomThreads)
+      blocks.push_back(MomBlock{(int)desc.size(), k});
+    desc.push_back(d);
+  }
+  const int n = (int)desc.size(), nb = (int)blocks.size();
+  if (n > kMaxBatch) return bfail(MLBM_ERR_ARG, "too many domains in a batch");
+  if (n > b->mcap) {
+    cudaFree(b->d_mdesc);
+    b->d_mdesc = nullptr;
+    b->mcap = 0;
+    const int cap = std::max(n, 64);
+    BCUDA(cudaMalloc(&b->d_mdesc, cap * sizeof(MomDomain)), "batch table");
+    b->mcap = cap;
+  }
+  if (nb > b->mblocks_cap) {
+    cudaFree(b->d_mblocks);
+    b->d_mblocks = nullptr;
+    b->mblocks_cap = 0;
+    BCUDA(cudaMalloc(&b->d_mblocks, (size_t)nb * sizeof(MomBlock)), "batch table");
+    b->mblocks_cap = nb;
+  }
+  if (n)
+    BCUDA(cudaMemcpyAsync(b->d_mdesc, desc.data(), n * sizeof(MomDomain),
+                          cudaMemcpyHostToDevice, b->stream), "batch table");
+  if (nb)
+    BCUDA(cudaMemcpyAsync(b->d_mblocks, blocks.data(), (size_t)nb * sizeof(MomBlock),
+                          cudaMemcpyHostToDevice, b->stream), "batch table");
+  BCUDA(cudaMemcpyAsync(b->d_step, &b->bstep, sizeof(long long),
+                        cudaMemcpyHostToDevice, b->stream), "batch step");
+  BCUDA(cudaStreamSynchronize(b->stream), "batch table");
+  b->nactive = n;
+  b->grid_m = nb;
+  b->dirty = false;
+  return MLBM_OK;
+}
+
+// Whether every domain can be held as moments; builds their lists and
+// buffers.  Where one's do not fit the device, none is.
+mlbm_status moments_mode(mlbm_batch* b, bool* on) {
+  *on = false;
+  for (const mlbm_lattice* lat : b->dom)
+    if (lat && !moments_apply(lat)) return MLBM_OK;
+  for (mlbm_lattice* lat : b->dom)
+    if (lat) {
+      const mlbm_status st = moments_prepare(lat);
+      if (st == MLBM_ERR_NOMEM) return MLBM_OK;
+      if (st) return st;
+    }
+  *on = true;
+  return MLBM_OK;
+}
+
+template <typename T>
+mlbm_status step_alone_t(mlbm_batch* b, int reverse, unsigned inject, bool write_rho) {
+  for (size_t s = 0; s < b->dom.size(); ++s) {
+    mlbm_lattice* lat = b->dom[s];
+    if (!lat) continue;
+    if (!lat->mom.active)
+      if (mlbm_status st = compact_leave(lat)) return st;
+    const StepArgs a{b->bstep - b->origin[s], reverse, inject};
+    if (mlbm_status st = launch_moment_step<T>(lat, a, false, write_rho)) return st;
+    lat->phase ^= 1;
+  }
+  b->bstep += 1;
+  return MLBM_OK;
+}
+
+// One step of every domain by its own launches: the step that takes new
+// domains from populations to moments.
+mlbm_status step_alone(mlbm_batch* b, int reverse, unsigned inject, bool write_rho) {
+  switch (b->storage) {
+    case MLBM_STORE_F32: return step_alone_t<float>(b, reverse, inject, write_rho);
+    case MLBM_STORE_F16: return step_alone_t<__half>(b, reverse, inject, write_rho);
+    default: return step_alone_t<double>(b, reverse, inject, write_rho);
+  }
+}
+
 bool compact_mode(const mlbm_batch* b) {
   if (b->storage == MLBM_STORE_F64) return false;
   for (mlbm_lattice* lat : b->dom)
@@ -160,6 +263,7 @@ bool compact_mode(const mlbm_batch* b) {
 
 mlbm_status rebuild(mlbm_batch* b) {
   drop_graph(b);
+  if (b->moments) return rebuild_moments(b);
   b->compact = compact_mode(b);
   if (b->compact) return rebuild_compact(b);
   // dense mode: the domains stay on (or return to) the dense layout
@@ -238,6 +342,15 @@ mlbm_status rebuild(mlbm_batch* b) {
 template <typename T>
 void launch_step(mlbm_batch* b, int delta, int reverse, unsigned inject,
                  bool write_rho) {
+  if (b->moments) {
+    if (b->grid_m == 0) return;
+    auto gather = write_rho ? k_batch_mom_gather<T, true> : k_batch_mom_gather<T, false>;
+    gather<<<b->grid_m, kMomThreads, 0, b->stream>>>(b->d_mdesc, b->d_mblocks,
+                                                     b->d_step, delta, reverse, inject);
+    k_batch_mom_collide<typename Pop<T>::Real>
+        <<<b->grid_m, kMomThreads, 0, b->stream>>>(b->d_mdesc, b->d_mblocks);
+    return;
+  }
   if constexpr (!std::is_same<T, double>::value) {
     if (b->compact) {
       if (write_rho)
@@ -367,6 +480,8 @@ mlbm_status mlbm_batch_destroy(mlbm_batch* b) {
   drop_graph(b);
   for (mlbm_lattice* lat : b->dom)
     if (lat) mlbm_lattice_destroy(lat);
+  cudaFree(b->d_mdesc);
+  cudaFree(b->d_mblocks);
   cudaFree(b->d_cdesc);
   cudaFree(b->d_cpre);
   cudaFree(b->d_desc);
@@ -468,10 +583,23 @@ mlbm_status mlbm_batch_iterate(mlbm_batch* b, int32_t nsteps, int32_t reverse,
   if (nsteps == 0) return MLBM_OK;
   mlbm::DeviceGuard restore_device;
   BCUDA(cudaSetDevice(b->device), "cudaSetDevice");
-  // a domain advanced on its own since may hold its state in another form
-  if (b->compact)
-    for (const mlbm_lattice* l : b->dom)
-      if (l && !l->compact.active) b->dirty = true;
+  // the domains' form: it follows a domain added or removed since, one whose
+  // parameters changed, one advanced on its own
+  bool moments = false;
+  if (mlbm_status st = moments_mode(b, &moments)) return st;
+  if (moments != b->moments) b->dirty = true;
+  b->moments = moments;
+  bool alone = false;
+  for (const mlbm_lattice* l : b->dom) {
+    if (!l) continue;
+    if (moments && (!l->mom.active || l->mom.shift != l->phys.rho_shift))
+      alone = b->dirty = true;
+    if (!moments && b->compact && !l->compact.active) b->dirty = true;
+  }
+  if (alone) {
+    if (mlbm_status st = step_alone(b, reverse, inject_type, nsteps == 1)) return st;
+    if (--nsteps == 0) return MLBM_OK;
+  }
   if (b->dirty)
     if (mlbm_status st = rebuild(b)) return st;
   if (b->nactive == 0) return MLBM_OK;
@@ -522,9 +650,7 @@ mlbm_status mlbm_batch_autotune(mlbm_batch* b, int32_t trial_steps,
                                 int32_t* out) {
   if (!b) return bfail(MLBM_ERR_ARG, "null batch");
   if (trial_steps < 1) trial_steps = 2;
-  if (b->dirty)
-    if (mlbm_status st = rebuild(b)) return st;
-  if (b->compact) {
+  if (compact_mode(b)) {
     // one thread per node (pair) per pass: no work-item shape to tune
     if (out) {
       out[0] = b->By_d;

@@ -337,21 +337,24 @@ struct Gather {
   }
 };
 
+// Resident blocks the registers are held to.  FP32: 64 registers (8-12 bytes
+// spilled) ran a 200^3 step in 117 us, 80 registers (6 blocks) in 122, 96 (5)
+// in 130, 51 (10 blocks, 68 bytes spilled) in 123.
 template <typename T>
-constexpr int mom_gather_blocks() { return sizeof(typename Pop<T>::Real) == 8 ? 4 : 6; }
+constexpr int mom_gather_blocks() { return sizeof(typename Pop<T>::Real) == 8 ? 4 : 8; }
 
-template <typename T, bool WRITE_RHO>
-__global__ void __launch_bounds__(kMomThreads, mom_gather_blocks<T>())
-    k_mom_gather(const MomPair<typename Pop<T>::Real>* m, PairList list,
-                 MomPair<typename Pop<T>::Real>* n, typename Pop<T>::Real* rho,
-                 typename Pop<T>::Real* psi, Geom g, Phys p, StepArgs a, bool inj,
-                 float shift_st) {
+// Gather pass of pair k of a list; every thread of the warp calls it.
+template <typename T, bool WRITE_RHO, bool PDL>
+__device__ __forceinline__ void mom_gather(
+    const MomPair<typename Pop<T>::Real>* m, const PairList& list, int k,
+    MomPair<typename Pop<T>::Real>* n, typename Pop<T>::Real* rho,
+    typename Pop<T>::Real* psi, const Geom& g, const Phys& p, const StepArgs& a,
+    bool inj, float shift_st) {
   using R = typename Pop<T>::Real;
-  const int k = blockIdx.x * kMomThreads + threadIdx.x;
   const bool some = k < list.count;
   const PairAt q = pair_at(g, list, some ? k : list.count - 1);
   const bool inner = __all_sync(~0u, q.na & NB_INNER);
-  pdl_gate<true>();
+  pdl_gate<PDL>();
   if (!some) return;
   MomPair<R> s;
   if (inner) {
@@ -364,6 +367,16 @@ __global__ void __launch_bounds__(kMomThreads, mom_gather_blocks<T>())
     s = c.sum;
   }
   mom_put<R, WRITE_RHO>(q, s, n, k, rho, psi, g, p, a, inj);
+}
+
+template <typename T, bool WRITE_RHO>
+__global__ void __launch_bounds__(kMomThreads, mom_gather_blocks<T>())
+    k_mom_gather(const MomPair<typename Pop<T>::Real>* m, PairList list,
+                 MomPair<typename Pop<T>::Real>* n, typename Pop<T>::Real* rho,
+                 typename Pop<T>::Real* psi, Geom g, Phys p, StepArgs a, bool inj,
+                 float shift_st) {
+  mom_gather<T, WRITE_RHO, true>(m, list, blockIdx.x * kMomThreads + threadIdx.x, n,
+                                 rho, psi, g, p, a, inj, shift_st);
 }
 
 // The gather of a step that starts from populations (the dense layout in AA
@@ -420,18 +433,14 @@ __device__ __forceinline__ Mom<R> shifted_velocity(const Phys& p, const Mom<R>& 
                 rmul(rfma(tau, rmul(gp, sz), n.z), inv)};
 }
 
-// Blocks run in reverse list order: what the gather wrote last is still in L2
-// when the collide starts with it, and the next gather starts where the
-// collide ended.
-template <typename R, bool WRITE_U>
-__global__ void __launch_bounds__(kMomThreads, 8)
-    k_mom_collide(const MomPair<R>* n, PairList list, const Two<R>* psi,
-                  MomPair<R>* m, float* vel, Geom g, Phys p) {
-  const int k = (int)(gridDim.x - 1 - blockIdx.x) * kMomThreads + threadIdx.x;
-  if (k >= list.count) return;
+// Collide pass of pair k of a list (k < list.count).
+template <typename R, bool WRITE_U, bool PDL>
+__device__ __forceinline__ void mom_collide(const MomPair<R>* n, const PairList& list,
+                                            int k, const Two<R>* psi, MomPair<R>* m,
+                                            float* vel, const Geom& g, const Phys& p) {
   const PairAt q = pair_at(g, list, k);
   const Columns col(g, q.x, q.y);
-  pdl_gate<true>();
+  pdl_gate<PDL>();
   const MomPair<R> s = ld_pair(n + k);
   const Two<R>* at = psi + q.at;
   // psi of the columns: [dy + 1][dx + 1], levels z - 1, z, z + 1, z + 2
@@ -482,6 +491,17 @@ __global__ void __launch_bounds__(kMomThreads, 8)
     if (q.na) for_images(g, q.x, q.y, q.z, [&](size_t i) { mm[i] = u.a; });
     if (q.nb) for_images(g, q.x, q.y, q.z + 1, [&](size_t i) { mm[i] = u.b; });
   }
+}
+
+// Blocks run in reverse list order: what the gather wrote last is still in L2
+// when the collide starts with it, and the next gather starts where the
+// collide ended.
+template <typename R, bool WRITE_U>
+__global__ void __launch_bounds__(kMomThreads, sizeof(R) == 8 ? 6 : 8)
+    k_mom_collide(const MomPair<R>* n, PairList list, const Two<R>* psi,
+                  MomPair<R>* m, float* vel, Geom g, Phys p) {
+  const int k = (int)(gridDim.x - 1 - blockIdx.x) * kMomThreads + threadIdx.x;
+  if (k < list.count) mom_collide<R, WRITE_U, true>(n, list, k, psi, m, vel, g, p);
 }
 
 // The populations of the fluid nodes, in the dense layout in AA phase PHASE
