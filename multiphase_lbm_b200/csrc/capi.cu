@@ -300,9 +300,8 @@ void launch_pop_out(mlbm_lattice* lat, O* out) {
 
 template <typename R, typename O>
 void launch_scalar_out(mlbm_lattice* lat, int field, O* out) {
-  k_scalar_to_ref<R, O><<<node_grid(lat->g), node_block(), 0, lat->stream>>>(
-      static_cast<const R*>(lat->rho), lat->mask, out, lat->g, lat->phys,
-      field);
+  k_scalar_to_ref<R, O><<<tile_grid(lat->g), tile_block(), 0, lat->stream>>>(
+      static_cast<const R*>(lat->rho), out, lat->g, lat->phys, field);
 }
 
 template <typename O>
@@ -321,7 +320,7 @@ mlbm_status field_out(mlbm_lattice* lat, int32_t field, O* dev_out) {
         return fail(MLBM_ERR_STATE,
                     "velocity not written: iterate with "
                     "MLBM_ITER_WRITE_VELOCITY first");
-      k_vel_to_ref<O><<<node_grid(lat->g), node_block(), 0, lat->stream>>>(
+      k_vel_to_ref<O><<<tile_grid(lat->g), tile_block(), 0, lat->stream>>>(
           lat->vel, dev_out, lat->g);
       break;
     case MLBM_FIELD_POPULATIONS:
@@ -523,7 +522,7 @@ static mlbm_status upload_mask_impl(mlbm_lattice* lat, const uint8_t* src,
   if (mlbm_status st = ensure_staging(lat, n)) return st;
   CUDA_TRY(cudaMemcpyAsync(lat->staging, src, n, kind, lat->stream),
            "mask upload copy");
-  k_pack_mask<<<node_grid(g), node_block(), 0, lat->stream>>>(
+  k_pack_mask<<<tile_grid(g), tile_block(), 0, lat->stream>>>(
       static_cast<const uint8_t*>(lat->staging), lat->mask, g);
   CUDA_TRY(cudaGetLastError(), "mask pack launch");
   CUDA_TRY(cudaStreamSynchronize(lat->stream), "mask upload");
@@ -541,7 +540,7 @@ static mlbm_status upload_rho_impl(mlbm_lattice* lat, const float* src,
   CUDA_TRY(cudaMemcpyAsync(lat->staging, src, n * sizeof(float), kind,
                            lat->stream),
            "rho upload copy");
-  k_rho_from_ref<<<node_grid(g), node_block(), 0, lat->stream>>>(
+  k_rho_from_ref<<<tile_grid(g), tile_block(), 0, lat->stream>>>(
       static_cast<const float*>(lat->staging), lat->rho_init, g);
   CUDA_TRY(cudaGetLastError(), "rho transpose launch");
   CUDA_TRY(cudaStreamSynchronize(lat->stream), "rho upload");
@@ -634,7 +633,7 @@ mlbm_status mlbm_download_field_device(mlbm_lattice* lat, int32_t field,
   if (field == MLBM_FIELD_FLUID) {
     if (dtype != MLBM_DTYPE_U8)
       return fail(MLBM_ERR_ARG, "the fluid mask downloads as MLBM_DTYPE_U8");
-    k_fluid_to_ref<<<node_grid(lat->g), node_block(), 0, lat->stream>>>(
+    k_fluid_to_ref<<<tile_grid(lat->g), tile_block(), 0, lat->stream>>>(
         lat->mask, static_cast<uint8_t*>(dev_out), lat->g);
     CUDA_TRY(cudaGetLastError(), "mask download launch");
     return MLBM_OK;
@@ -842,10 +841,10 @@ mlbm_status mlbm_plane_profile(mlbm_lattice* lat, int64_t* n_fluid_x,
   auto* nl = nf + lx;
   CUDA_TRY(cudaMemsetAsync(nf, 0, bytes, lat->stream), "profile clear");
   if (lat->storage == MLBM_STORE_F64)
-    k_plane_profile<double><<<node_grid(lat->g), node_block(), 0, lat->stream>>>(
+    k_plane_profile<double><<<profile_grid(lat->g), dim3(32, 8), 0, lat->stream>>>(
         static_cast<const double*>(lat->rho), lat->mask, lat->g, lat->phys, nf, nl);
   else
-    k_plane_profile<float><<<node_grid(lat->g), node_block(), 0, lat->stream>>>(
+    k_plane_profile<float><<<profile_grid(lat->g), dim3(32, 8), 0, lat->stream>>>(
         static_cast<const float*>(lat->rho), lat->mask, lat->g, lat->phys, nf, nl);
   CUDA_TRY(cudaGetLastError(), "profile launch");
   CUDA_TRY(cudaMemcpyAsync(n_fluid_x, nf, lx * 8, cudaMemcpyDeviceToHost,

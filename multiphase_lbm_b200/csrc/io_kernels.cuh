@@ -20,56 +20,97 @@ __device__ __forceinline__ long long ref_index(const Geom& g, int x, int y,
   const int y = blockIdx.y * blockDim.y + threadIdx.y; \
   const int z = blockIdx.z;
 
-// Pack a uint8 [x][y][z] fluid array into the bit mask; every warp covers one
-// aligned 32-node run of a row.
+// Both layouts are dense with opposite fastest axes, so a copy is a transpose
+// of the (x, z) planes: a block moves a 32 x 32 tile of one y through shared
+// memory, reading and writing runs of 32 values (one value per thread straight
+// across touched a sector per 4 bytes on one side: 56 us for the 64 MB of a
+// 200^3 FP32 field).  blockDim (32, kTileRows), grid (x tiles of every y, z
+// tiles): y has no place among the grid's short dimensions (up to 2^24 rows).
+constexpr int kTileRows = 8;
+#define MLBM_TILE_COORDS                                             \
+  const int xt = (int)(blockIdx.x % (unsigned)g.wpr), x0 = xt * 32;  \
+  const int y = (int)(blockIdx.x / (unsigned)g.wpr);                 \
+  const int z0 = blockIdx.y * 32, lane = threadIdx.x;
+
+inline dim3 tile_block() { return dim3(32, kTileRows, 1); }
+inline dim3 tile_grid(const Geom& g) {
+  return dim3((unsigned)g.wpr * (unsigned)g.ly, (g.lz + 31) / 32, 1);
+}
+
+// Pack a uint8 [x][y][z] fluid array into the bit mask.
 __global__ void k_pack_mask(const uint8_t* __restrict__ fluid_ref,
                             uint32_t* __restrict__ mask, Geom g) {
-  MLBM_NODE_COORDS
-  if (y >= g.ly) return;  // whole warp exits together (warp = one row run)
-  const bool f = (x < g.lx) && fluid_ref[ref_index(g, x, y, z)] != 0;
-  const uint32_t w = __ballot_sync(0xffffffffu, f);
-  if ((threadIdx.x & 31) == 0)
-    mask[((long long)z * g.ly + y) * g.wpr + (x >> 5)] = w;
+  __shared__ uint8_t t[32][33];
+  MLBM_TILE_COORDS
+  for (int r = threadIdx.y; r < 32; r += kTileRows) {
+    const int x = x0 + r, z = z0 + lane;
+    t[r][lane] = x < g.lx && z < g.lz && fluid_ref[ref_index(g, x, y, z)] != 0;
+  }
+  __syncthreads();
+  for (int r = threadIdx.y; r < 32 && z0 + r < g.lz; r += kTileRows) {
+    const uint32_t w = __ballot_sync(0xffffffffu, t[lane][r] != 0);
+    if (lane == 0) mask[((long long)(z0 + r) * g.ly + y) * g.wpr + xt] = w;
+  }
 }
 
 __global__ void k_rho_from_ref(const float* __restrict__ rho_ref,
                                float* __restrict__ rho_int, Geom g) {
-  MLBM_NODE_COORDS
-  if (x >= g.lx || y >= g.ly) return;
-  rho_int[node_index(g, x, y, z)] = rho_ref[ref_index(g, x, y, z)];
+  __shared__ float t[32][33];
+  MLBM_TILE_COORDS
+  for (int r = threadIdx.y; r < 32; r += kTileRows) {
+    const int x = x0 + r, z = z0 + lane;
+    if (x < g.lx && z < g.lz) t[r][lane] = rho_ref[ref_index(g, x, y, z)];
+  }
+  __syncthreads();
+  if (x0 + lane >= g.lx) return;
+  for (int r = threadIdx.y; r < 32 && z0 + r < g.lz; r += kTileRows)
+    rho_int[node_index(g, x0 + lane, y, z0 + r)] = t[lane][r];
 }
 
-// field: 0 rho, 1 pressure, 2 psi, 5 fluid (as 0/1) -> reference layout.
+// field: 0 rho, 1 pressure, 2 psi -> reference layout.
 template <typename R, typename O>
-__global__ void k_scalar_to_ref(const R* __restrict__ rho,
-                                const uint32_t* __restrict__ mask,
-                                O* __restrict__ out, Geom g, Phys p,
-                                int field) {
-  MLBM_NODE_COORDS
-  if (x >= g.lx || y >= g.ly) return;
-  const R r = rho[node_index(g, x, y, z)];
-  R v;
-  if (field == 0) v = r;
-  else if (field == 1) v = pressure_of<R>(p, r);
-  else if (field == 2) v = psi_of<R>(p, r);
-  else v = R(fluid_at(mask, g, x, y, z) ? 1 : 0);
-  out[ref_index(g, x, y, z)] = (O)v;
+__global__ void k_scalar_to_ref(const R* __restrict__ rho, O* __restrict__ out,
+                                Geom g, Phys p, int field) {
+  __shared__ O t[32][33];
+  MLBM_TILE_COORDS
+  for (int r = threadIdx.y; r < 32; r += kTileRows) {
+    const int x = x0 + lane, z = z0 + r;
+    if (x >= g.lx || z >= g.lz) continue;
+    const R v = rho[node_index(g, x, y, z)];
+    t[lane][r] = (O)(field == 0 ? v : field == 1 ? pressure_of<R>(p, v) : psi_of<R>(p, v));
+  }
+  __syncthreads();
+  if (z0 + lane >= g.lz) return;
+  for (int r = threadIdx.y; r < 32 && x0 + r < g.lx; r += kTileRows)
+    out[ref_index(g, x0 + r, y, z0 + lane)] = t[r][lane];
 }
 
 __global__ void k_fluid_to_ref(const uint32_t* __restrict__ mask,
                                uint8_t* __restrict__ out, Geom g) {
-  MLBM_NODE_COORDS
-  if (x >= g.lx || y >= g.ly) return;
-  out[ref_index(g, x, y, z)] = fluid_at(mask, g, x, y, z) ? 1 : 0;
+  MLBM_TILE_COORDS
+  if (z0 + lane >= g.lz) return;
+  // a warp writes 32 z of one x; its 32 mask words serve the tile's 32 x
+  const uint32_t w = mask[((long long)(z0 + lane) * g.ly + y) * g.wpr + xt];
+  for (int r = threadIdx.y; r < 32 && x0 + r < g.lx; r += kTileRows)
+    out[ref_index(g, x0 + r, y, z0 + lane)] = (w >> r) & 1u;
 }
 
+// The three components of a node stay together: runs of 96 values.
 template <typename O>
 __global__ void k_vel_to_ref(const float* __restrict__ vel,
                              O* __restrict__ out, Geom g) {
-  MLBM_NODE_COORDS
-  if (x >= g.lx || y >= g.ly) return;
-  const long long n = node_index(g, x, y, z), r = ref_index(g, x, y, z);
-  for (int c = 0; c < 3; ++c) out[3 * r + c] = (O)vel[3 * n + c];
+  __shared__ float t[32][97];  // [z][3 x + c]
+  MLBM_TILE_COORDS
+  const int nx = min(32, g.lx - x0), nz = min(32, g.lz - z0);
+  for (int r = threadIdx.y; r < nz; r += kTileRows) {
+    const float* src = vel + 3 * node_index(g, x0, y, z0 + r);
+    for (int c = lane; c < 3 * nx; c += 32) t[r][c] = src[c];
+  }
+  __syncthreads();
+  for (int r = threadIdx.y; r < nx; r += kTileRows) {
+    O* dst = out + 3 * ref_index(g, x0 + r, y, z0);
+    for (int c = lane; c < 3 * nz; c += 32) dst[c] = (O)t[c / 3][3 * r + c % 3];
+  }
 }
 
 // Post-collision populations f*_i in the reference layout [x][y][z][19].
@@ -349,17 +390,46 @@ __global__ void __launch_bounds__(kStatThreads)
   stat_last_block(sc, gridDim.x, err, threadIdx.x, FULL);
 }
 
-// Per-x-plane fluid / liquid node counts (integer atomics: deterministic).
+// Per-x-plane fluid / liquid node counts (integers: deterministic).  A thread
+// counts a column of kProfileRows rows (y, z) at its x, a block adds its
+// columns up and adds one number per plane (two atomics per fluid node on lx
+// counters took 210 us at 200^3).  blockDim (32, 8), grid x tiles of
+// every row group.
+constexpr int kProfileRows = 64;
 template <typename R>
 __global__ void k_plane_profile(const R* __restrict__ rho,
                                 const uint32_t* __restrict__ mask, Geom g,
                                 Phys p, unsigned long long* __restrict__ nf,
                                 unsigned long long* __restrict__ nl) {
-  MLBM_NODE_COORDS
-  if (x >= g.lx || y >= g.ly) return;
-  if (!fluid_at(mask, g, x, y, z)) return;
-  atomicAdd(nf + x, 1ull);
-  if (rho[node_index(g, x, y, z)] > R(p.rhol_spinodal)) atomicAdd(nl + x, 1ull);
+  __shared__ unsigned sf[8][32], sl[8][32];
+  const int lane = threadIdx.x, w = (int)(blockIdx.x % (unsigned)g.wpr);
+  const int x = w * 32 + lane;
+  const long long rows = (long long)g.ly * g.lz;
+  const long long r0 =
+      ((long long)(blockIdx.x / (unsigned)g.wpr) * 8 + threadIdx.y) * kProfileRows;
+  unsigned f = 0, l = 0;
+#pragma unroll 4
+  for (long long r = r0; r < min(r0 + kProfileRows, rows); ++r) {
+    const bool fl = (mask[r * g.wpr + w] >> lane) & 1u;
+    f += fl;
+    // padding columns are never fluid, and lie inside the array
+    l += fl && rho[r * g.px + x] > R(p.rhol_spinodal);
+  }
+  sf[threadIdx.y][lane] = f;
+  sl[threadIdx.y][lane] = l;
+  __syncthreads();
+  if (threadIdx.y) return;
+  for (int j = 1; j < 8; ++j) {
+    f += sf[j][lane];
+    l += sl[j][lane];
+  }
+  if (x >= g.lx) return;
+  if (f) atomicAdd(nf + x, (unsigned long long)f);
+  if (l) atomicAdd(nl + x, (unsigned long long)l);
+}
+inline dim3 profile_grid(const Geom& g) {
+  const long long rows = (long long)g.ly * g.lz;
+  return dim3((unsigned)(g.wpr * ((rows + 8 * kProfileRows - 1) / (8 * kProfileRows))));
 }
 
 }  // namespace mlbm
