@@ -102,7 +102,7 @@ __device__ __forceinline__ void batch_update_node(const DomainDesc& d,
     const R* ps = static_cast<const R*>(d.psi) + psi_index(g, x, y, z);
     const long long sy = g.pxg, sz = (long long)(g.ly + 2) * g.pxg;
     R ux, uy, uz;
-    collide<R>(
+    collide<T, R>(
         d.p, dd, __ldg(ps),
         [&](int i) { return __ldg(ps + ex(i) + ey(i) * sy + ez(i) * sz); }, f,
         ux, uy, uz);

@@ -18,9 +18,9 @@ namespace mlbm {
 struct MomDomain {
   Geom g;
   Phys p;
-  void* m;      // MomPair<R>, paired dense layout
+  void* m;      // Mom<R>, dense (node_element)
   void* n;      // MomPair<R>, pair list
-  void* psi;    // R, paired dense layout
+  void* psi;    // R, dense (node_element)
   void* rho;    // R, dense
   PairList list;
   long long step_origin;
@@ -42,8 +42,9 @@ __global__ void __launch_bounds__(kMomThreads, mom_gather_blocks<T>())
   const StepArgs a{*step + delta - D.step_origin, reverse, inject_type};
   const bool inj = D.p.rho_inject_period != 0ull &&
                    (unsigned long long)a.step % D.p.rho_inject_period == 0ull;
+  const int k = b.first + (int)threadIdx.x;
   mom_gather<T, WRITE_RHO, false>(
-      static_cast<const MomPair<R>*>(D.m), D.list, b.first + (int)threadIdx.x,
+      static_cast<const Mom<R>*>(D.m), D.list, k,
       static_cast<MomPair<R>*>(D.n), static_cast<R*>(D.rho),
       static_cast<R*>(D.psi), D.g, D.p, a, inj, D.p.rho_shift);
 }
@@ -57,8 +58,8 @@ __global__ void __launch_bounds__(kMomThreads, sizeof(R) == 8 ? 6 : 8)
   const int k = b.first + (int)threadIdx.x;
   if (k < D.list.count)
     mom_collide<R, false, false>(static_cast<const MomPair<R>*>(D.n), D.list, k,
-                                 static_cast<const Two<R>*>(D.psi),
-                                 static_cast<MomPair<R>*>(D.m), nullptr, D.g, D.p);
+                                 static_cast<const R*>(D.psi),
+                                 static_cast<Mom<R>*>(D.m), nullptr, D.g, D.p);
 }
 
 }  // namespace mlbm

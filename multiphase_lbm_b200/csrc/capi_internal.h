@@ -41,8 +41,8 @@ struct MomentState {
   bool active = false;      // m holds the current state
   void* buffer = nullptr;   // one allocation for all of the following
   size_t buffer_bytes = 0;
-  void* m = nullptr;        // [pair_elems] MomPair<R>: density, velocity
-  void* psi = nullptr;      // [pair_elems] Two<R>
+  void* m = nullptr;        // [node_elems] Mom<R>: density, velocity
+  void* psi = nullptr;      // [node_elems] R
   void* n = nullptr;        // [npairs] MomPair<R>: density, momentum
   uint2* words = nullptr;   // [npairs] node pairs: neighbour words,
   uint32_t* xyz = nullptr;  //          packed x, y, z

@@ -126,9 +126,32 @@ __device__ __forceinline__ float slab_density(const Phys& p, int kind) {
   return kind == 1 ? p.rho_inlet : p.rho_outlet;
 }
 
+// The equilibrium at omega = 1 (f* = feq), feq_i = t_i rho (base + 3 eu +
+// 4.5 eu^2) with base = 1 - 1.5 u^2 and eu = e_i . u, as every kernel forms it
+// for storage T.  FP32 and FP64 take the shorter chain of fused operations;
+// FP16 storage keeps the chain of the general update, whose last bits decide
+// which half a population is rounded to.
+template <typename T>
+struct Equilibrium {
+  using R = typename Pop<T>::Real;
+  static __device__ __forceinline__ R base(R usq) { return rfma(R(-1.5), usq, R(1)); }
+  static __device__ __forceinline__ R term(R base, R eu) {
+    return rfma(eu, rfma(R(4.5), eu, R(3)), base);
+  }
+};
+template <>
+struct Equilibrium<__half> {
+  static __device__ __forceinline__ float base(float usq) {
+    return rsub(1.f, rmul(1.5f, usq));
+  }
+  static __device__ __forceinline__ float term(float base, float eu) {
+    return radd(rfma(rmul(4.5f, eu), eu, base), rmul(3.f, eu));
+  }
+};
+
 // Force, velocity shift and BGK relaxation of one interior fluid node
 // (include/iteration_device.cuh:69-206).  psi_nb(i) returns psi at x + e_i.
-template <typename R, typename PsiNb>
+template <typename T, typename R, typename PsiNb>
 __device__ __forceinline__ void collide(const Phys& p, R d, R psi_self,
                                         PsiNb psi_nb, R (&f)[Q], R& ux, R& uy,
                                         R& uz) {
@@ -158,32 +181,45 @@ __device__ __forceinline__ void collide(const Phys& p, R d, R psi_self,
   ux = rmul(rfma(tau, Fx, ux), inv_rho);
   uy = rmul(rfma(tau, Fy, uy), inv_rho);
   uz = rmul(rfma(tau, Fz, uz), inv_rho);
-  const R usq15 =
-      rmul(R(1.5), rfma(uz, uz, rfma(uy, uy, rmul(ux, ux))));
+  const R usq = rfma(uz, uz, rfma(uy, uy, rmul(ux, ux)));
   const R omega = R(p.omega);
-  // BGK, include/iteration_device.cuh:162-174:
-  //   f_i += (t_i rho (1 + 3 eu + 4.5 eu^2 - 1.5 u^2) - f_i) / tau
-  // evaluated for the pairs (i, opp(i)), whose eu differ only in sign.
-  const R base = rsub(R(1), usq15);
   const R wd0 = rmul(weight<R>(0), d), wd1 = rmul(weight<R>(1), d),
           wd2 = rmul(weight<R>(4), d);
-  // omega = 1: f_i + (feq_i - f_i) is feq_i, taken without the two roundings
-  // (what the moment step relies on, moments.cuh)
-  const bool eq = omega == R(1);
-  f[0] = eq ? rmul(wd0, base) : rfma(rsub(rmul(wd0, base), f[0]), omega, f[0]);
-#pragma unroll
-  for (int i = 1; i <= 9; ++i) {
+  auto e_dot_u = [&](int i) {
     R eu = R(0);
     if (ex(i)) eu = ex(i) > 0 ? radd(eu, ux) : rsub(eu, ux);
     if (ey(i)) eu = ey(i) > 0 ? radd(eu, uy) : rsub(eu, uy);
     if (ez(i)) eu = ez(i) > 0 ? radd(eu, uz) : rsub(eu, uz);
+    return eu;
+  };
+  // omega = 1: f_i + (feq_i - f_i) is feq_i, taken without the two roundings
+  // (what the moment step relies on, moments.cuh)
+  if (omega == R(1)) {
+    const R base = Equilibrium<T>::base(usq);
+    f[0] = rmul(wd0, base);
+#pragma unroll
+    for (int i = 1; i <= 9; ++i) {
+      const R eu = e_dot_u(i), wd = (i <= 3) ? wd1 : wd2;
+      f[i] = rmul(wd, Equilibrium<T>::term(base, eu));
+      f[opp(i)] = rmul(wd, Equilibrium<T>::term(base, -eu));
+    }
+    return;
+  }
+  // BGK, include/iteration_device.cuh:162-174:
+  //   f_i += (t_i rho (1 + 3 eu + 4.5 eu^2 - 1.5 u^2) - f_i) / tau
+  // evaluated for the pairs (i, opp(i)), whose eu differ only in sign.
+  const R base = rsub(R(1), rmul(R(1.5), usq));
+  f[0] = rfma(rsub(rmul(wd0, base), f[0]), omega, f[0]);
+#pragma unroll
+  for (int i = 1; i <= 9; ++i) {
+    const R eu = e_dot_u(i);
     const R sym = rfma(rmul(R(4.5), eu), eu, base);
     const R anti = rmul(R(3), eu);
     const R wd = (i <= 3) ? wd1 : wd2;
     const R feq_i = rmul(wd, radd(sym, anti));
     const R feq_o = rmul(wd, rsub(sym, anti));
-    f[i] = eq ? feq_i : rfma(rsub(feq_i, f[i]), omega, f[i]);
-    f[opp(i)] = eq ? feq_o : rfma(rsub(feq_o, f[opp(i)]), omega, f[opp(i)]);
+    f[i] = rfma(rsub(feq_i, f[i]), omega, f[i]);
+    f[opp(i)] = rfma(rsub(feq_o, f[opp(i)]), omega, f[opp(i)]);
   }
 }
 

@@ -48,8 +48,8 @@ mlbm_status build_list(mlbm_lattice* lat) {
                         cudaMemcpyDeviceToHost, lat->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(lat->stream);
   const size_t real = real_bytes(lat->storage);
-  const size_t m_bytes = up256((size_t)pair_elems(g) * 8 * real);
-  const size_t psi_bytes = up256((size_t)pair_elems(g) * 2 * real);
+  const size_t m_bytes = up256((size_t)node_elems(g) * 4 * real);
+  const size_t psi_bytes = up256((size_t)node_elems(g) * real);
   const size_t n_bytes = up256((size_t)total.pairs * 8 * real);
   const size_t words_bytes = up256((size_t)total.pairs * sizeof(uint2));
   const size_t xyz_bytes = up256((size_t)total.pairs * sizeof(uint32_t));
@@ -100,7 +100,7 @@ void launch_gather(mlbm_lattice* lat, const StepArgs& a, bool inj, bool overlap)
   const unsigned grid = pair_blocks(s);
   if (s.active) {
     launch_overlapped(overlap, k_mom_gather<T, WR>, grid, kMomThreads, 0, lat->stream,
-                      (const MomPair<R>*)s.m, pair_list(s), n, rho, psi, lat->g,
+                      (const Mom<R>*)s.m, pair_list(s), n, rho, psi, lat->g,
                       lat->phys, a, inj, s.shift);
     return;
   }
@@ -121,7 +121,7 @@ mlbm_status to_populations(mlbm_lattice* lat) {
   using R = typename Pop<T>::Real;
   const MomentState& s = lat->mom;
   if (s.npairs == 0) return MLBM_OK;
-  const MomPair<R>* m = static_cast<const MomPair<R>*>(s.m);
+  const Mom<R>* m = static_cast<const Mom<R>*>(s.m);
   T* pop = static_cast<T*>(lat->pop);
   if (lat->phase == 0)
     k_mom_populations<T, 0><<<pair_blocks(s), kMomThreads, 0, lat->stream>>>(
@@ -136,10 +136,10 @@ mlbm_status to_populations(mlbm_lattice* lat) {
 
 }  // namespace
 
-// Packed coordinates and 32-bit pair indexes bound the lattice.
+// Packed coordinates and 32-bit node indexes bound the lattice.
 bool moments_supported(const Geom& g) {
   return g.lx <= kC2MaxX && g.ly <= kC2MaxY && g.lz <= kC2MaxZ &&
-         pair_elems(g) < (1LL << 31);
+         node_elems(g) < (1LL << 31);
 }
 
 bool moments_apply(const mlbm_lattice* lat) {
@@ -172,8 +172,8 @@ mlbm_status launch_moment_step(mlbm_lattice* lat, const StepArgs& a, bool write_
     else launch_gather<T, false>(lat, a, inj, overlap);
     auto collide = write_u ? k_mom_collide<R, true> : k_mom_collide<R, false>;
     launch_overlapped(overlap, collide, pair_blocks(s), kMomThreads, 0, lat->stream,
-                      (const MomPair<R>*)s.n, pair_list(s), (const Two<R>*)s.psi,
-                      (MomPair<R>*)s.m, lat->vel, lat->g, lat->phys);
+                      (const MomPair<R>*)s.n, pair_list(s), (const R*)s.psi, (Mom<R>*)s.m,
+                      lat->vel, lat->g, lat->phys);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "moment step launch");
   }

@@ -18,23 +18,27 @@
 //   collide  per fluid node: Shan-Chen force from the neighbours' psi,
 //            u = (j + tau F)/rho, writes m = (rho, u).
 //
-// Layout.  m and psi are dense and hold the nodes z and z + 1 (z even) next to
-// each other: element 2 * ((zp ly + y) px + x) + (z & 1), zp = (z + 2) / 2;
+// Layout.  m and psi are dense, node (x, y, z) at ((z + 1) ly + y) px + x;
 // planes z = -1 and z = lz hold the periodic images of the last and the first
 // (x and y wrap by the offsets of a node's columns: with ghost copies in all
 // axes the stores of the images took longer than the rest of the collide).
-// A thread owns such a pair of nodes, so the moments of both, and of both
-// their neighbours in a column, are one 32-byte sector and one load; the 36
-// populations of a pair come from 28 nodes in 9 columns, 9 pair loads and 10
-// single ones, and what depends on the source node alone (1 - 1.5 u^2, the
-// weights times rho) is formed once for the up to three populations that the
-// pair takes from it.  Solid nodes' moments are never used.
+// A thread owns the nodes z and z + 1 (z even): the 36 populations of the pair
+// come from 28 nodes in 9 columns, and what depends on the source node alone
+// (1 - 1.5 u^2, the weights times rho) is formed once for the up to three
+// populations that the pair takes from it.  Solid nodes' moments are never
+// used.  Threads run over a list of the pairs that hold fluid (a pair with one
+// solid node, 4-8 % of the nodes in the benchmarks' packings, idles half),
+// ordered by tiles of 32 x kTileY x kTileZ nodes and by rows within, so that a
+// block's loads share lines in all three directions.
 //
-// Threads run over a list of the pairs that hold fluid (a pair with one solid
-// node, 4-8 % of the nodes in the benchmarks' packings, idles half), ordered
-// by tiles of 32 x kTileY x kTileZ nodes so that a block's loads share lines
-// in all three directions.  In each tile the pairs whose neighbours are all
-// fluid come first: a warp of such pairs skips the bounce-back selects.
+// What bounds it: the cache lines a warp's loads touch.  A warp of the list
+// spans 2-3 runs of fluid along x, so a 16-byte load of its lanes touches 6
+// lines where a full row would touch 4.  Tried, at 200^3 FP32 (us per step,
+// 110 as it is): the two nodes of a pair side by side with 32-byte loads
+// 117 (19 requests in place of 28, but 9.7 lines each); pairs whose neighbours
+// are all fluid listed first in each tile, to skip their bounce-back selects,
+// 119 (the runs break up: 7.9 lines); tiles staged in shared memory with
+// packed FP32 arithmetic 190 (bank conflicts take the place of the lines).
 //
 // FP16 storage keeps its meaning: a population read by the gather is rounded
 // to half(f* - t_i rho_shift) exactly as the population kernels store it.
@@ -52,9 +56,6 @@ constexpr int kMomThreads = 128;
 
 // Neighbour words of the lists (k_build_nbr's, bits 0-20) also hold:
 constexpr uint32_t NB_EDGE = 1u << 21;   // z = 0 or lz - 1: has an image
-constexpr uint32_t NB_INNER = 1u << 22;  // a pair's first word: 36 fluid links,
-                                         // no slab nodes
-constexpr uint32_t kNbAllFluid = 0x7ffffu;  // the node and its 18 sources
 
 template <typename R>
 struct alignas(4 * sizeof(R)) Mom {
@@ -65,26 +66,22 @@ struct alignas(8 * sizeof(R)) MomPair {
   Mom<R> a, b;  // z, z + 1
 };
 template <typename R>
-struct alignas(2 * sizeof(R)) Two {
+struct Two {
   R a, b;
 };
 
-// Pair of node (x, y, z), 0 <= x < lx, 0 <= y < ly, -1 <= z <= lz.
-__host__ __device__ __forceinline__ uint32_t pair_index(const Geom& g, int x, int y,
-                                                        int z) {
-  return (uint32_t)(((z + 2) >> 1) * g.ly + y) * (uint32_t)g.px + (uint32_t)x;
+// Node (x, y, z), 0 <= x < lx, 0 <= y < ly, -1 <= z <= lz, of m and psi.
+__host__ __device__ __forceinline__ uint32_t node_element(const Geom& g, int x, int y,
+                                                          int z) {
+  return (uint32_t)((z + 1) * g.ly + y) * (uint32_t)g.px + (uint32_t)x;
 }
-// (an odd lz: one plane more, read for the node beside the box's last one)
-__host__ __device__ __forceinline__ long long pair_elems(const Geom& g) {
-  return (long long)((g.lz + 3) / 2 + 1) * g.ly * g.px;
-}
-__host__ __device__ __forceinline__ size_t node_element(const Geom& g, int x, int y,
-                                                        int z) {
-  return 2 * (size_t)pair_index(g, x, y, z) + (z & 1);
+// (one plane more, read for the node beside the box's last one when lz is odd)
+__host__ __device__ __forceinline__ long long node_elems(const Geom& g) {
+  return (long long)(g.lz + 3) * g.ly * g.px;
 }
 
-// Offsets, in pairs, of the columns around a pair's (periodic in x and y) and
-// of the planes below and above it.
+// Offsets of the columns around a node's (periodic in x and y) and of the
+// plane above it.
 struct Columns {
   int xm, xp, ym, yp, plane;
   __device__ __forceinline__ Columns(const Geom& g, int x, int y) {
@@ -139,7 +136,7 @@ struct PairList {
 struct PairAt {
   uint32_t na, nb;
   int x, y, z;
-  uint32_t at;  // pair_index
+  uint32_t at;  // node_element of the first node
 };
 __device__ __forceinline__ PairAt pair_at(const Geom& g, const PairList& l, int k) {
   const uint2 w = __ldg(l.words + k);
@@ -150,7 +147,7 @@ __device__ __forceinline__ PairAt pair_at(const Geom& g, const PairList& l, int 
   q.x = (int)(c & 2047u);
   q.y = (int)((c >> 11) & 2047u);
   q.z = (int)(c >> 22);
-  q.at = pair_index(g, q.x, q.y, q.z);
+  q.at = node_element(g, q.x, q.y, q.z);
   return q;
 }
 
@@ -162,20 +159,23 @@ __host__ __device__ constexpr int direction(int dx, int dy, int dz) {
 
 // ---- equilibrium ----------------------------------------------------------------
 // A node's moments with what every population of it shares.
-template <typename R>
+template <typename T>
 struct Source {
+  using R = typename Pop<T>::Real;
   Mom<R> m;
-  R base, wd1, wd2;  // 1 - 1.5 u^2; axis and diagonal weight times rho
+  R base, wd1, wd2;  // of Equilibrium; axis and diagonal weight times rho
   __device__ __forceinline__ explicit Source(const Mom<R>& v) : m(v) {
-    base = rsub(R(1), rmul(R(1.5), rfma(v.z, v.z, rfma(v.y, v.y, rmul(v.x, v.x)))));
+    base = Equilibrium<T>::base(rfma(v.z, v.z, rfma(v.y, v.y, rmul(v.x, v.x))));
     wd1 = rmul(weight<R>(1), v.d);
     wd2 = rmul(weight<R>(4), v.d);
   }
 };
 
 // feq_i of collide(), operation for operation.
-template <typename R>
-__device__ __forceinline__ R eq_population(int i, const Source<R>& s) {
+template <typename T>
+__device__ __forceinline__ typename Pop<T>::Real eq_population(int i,
+                                                               const Source<T>& s) {
+  using R = typename Pop<T>::Real;
   if (i == 0) return rmul(rmul(weight<R>(0), s.m.d), s.base);
   R eu = R(0);
   if (ex(i)) eu = ex(i) > 0 ? s.m.x : -s.m.x;
@@ -183,9 +183,8 @@ __device__ __forceinline__ R eq_population(int i, const Source<R>& s) {
                         : (ey(i) > 0 ? s.m.y : -s.m.y);
   if (ez(i)) eu = ex(i) || ey(i) ? (ez(i) > 0 ? radd(eu, s.m.z) : rsub(eu, s.m.z))
                                  : (ez(i) > 0 ? s.m.z : -s.m.z);
-  const R sym = rfma(rmul(R(4.5), eu), eu, s.base);
   const bool axis = ex(i) * ex(i) + ey(i) * ey(i) + ez(i) * ez(i) == 1;
-  return rmul(axis ? s.wd1 : s.wd2, radd(sym, rmul(R(3), eu)));
+  return rmul(axis ? s.wd1 : s.wd2, Equilibrium<T>::term(s.base, eu));
 }
 
 // Both nodes' population as the storage format T holds it: stored with shift
@@ -250,37 +249,34 @@ __device__ __forceinline__ void mom_put(const PairAt& q, MomPair<R> s,
     if (q.na) rho[at] = s.a.d;
     if (q.nb) rho[at + g.ly * g.px] = s.b.d;
   }
-  if (q.na & q.nb & NB_SELF) {
-    *reinterpret_cast<Two<R>*>(psi + 2 * (size_t)q.at) = Two<R>{va, vb};
-  } else {  // a solid node keeps its psi, a ghost node its image's
-    psi[2 * (size_t)q.at + (q.na ? 0 : 1)] = q.na ? va : vb;
-  }
+  if (q.na) psi[q.at] = va;
+  if (q.nb) psi[q.at + g.ly * g.px] = vb;
   if ((q.na | q.nb) & NB_EDGE) {
-    if (q.na) for_images(g, q.x, q.y, q.z, [&](size_t i) { psi[i] = va; });
-    if (q.nb) for_images(g, q.x, q.y, q.z + 1, [&](size_t i) { psi[i] = vb; });
+    if (q.na) for_images(g, q.x, q.y, q.z, [&](uint32_t i) { psi[i] = va; });
+    if (q.nb) for_images(g, q.x, q.y, q.z + 1, [&](uint32_t i) { psi[i] = vb; });
   }
 }
 
 // ---- kernels ----------------------------------------------------------------------
 
 // The populations of one pair, in the order the sums take them.
-template <typename T, bool INNER>
+template <typename T>
 struct Gather {
   using R = typename Pop<T>::Real;
-  const MomPair<R>* at;  // the pair's own moments
+  const Mom<R>* at;  // the first node's own moments
   Columns col;
   uint32_t na, nb;
   float st, ld;
   MomPair<R> own, sum;
 
   // f_i of both nodes from the sources sa, sb
-  __device__ __forceinline__ Two<R> population(int i, const Source<R>& sa,
-                                               const Source<R>& sb) {
-    Two<R> f{eq_population<R>(i, sa), eq_population<R>(i, sb)};
-    if (!INNER && i) {
+  __device__ __forceinline__ Two<R> population(int i, const Source<T>& sa,
+                                               const Source<T>& sb) {
+    Two<R> f{eq_population<T>(i, sa), eq_population<T>(i, sb)};
+    if (i) {
       const int o = opp(i);
-      const R oa = eq_population<R>(o, Source<R>(own.a)),
-              ob = eq_population<R>(o, Source<R>(own.b));
+      const R oa = eq_population<T>(o, Source<T>(own.a)),
+              ob = eq_population<T>(o, Source<T>(own.b));
       f.a = (na >> i) & 1u ? f.a : oa;
       f.b = (nb >> i) & 1u ? f.b : ob;
     }
@@ -289,24 +285,24 @@ struct Gather {
   // the three populations from the column (dx, dy): levels z - 1 .. z + 2
   __device__ __forceinline__ void column(int dx, int dy, Two<R>& f0, Two<R>& up,
                                          Two<R>& down) {
-    const MomPair<R>* c = at + col.at(dx, dy);
-    const MomPair<R> mid = dx || dy ? ld_pair(c) : own;
-    const Source<R> lo((c - col.plane)->b), a(mid.a), b(mid.b),
-        hi((c + col.plane)->a);
+    const Mom<R>* c = at + col.at(dx, dy);
+    const Source<T> lo(c[-col.plane]), a(dx || dy ? c[0] : own.a),
+        b(dx || dy ? c[col.plane] : own.b), hi(c[2 * col.plane]);
     f0 = population(direction(-dx, -dy, 0), a, b);
     up = population(direction(-dx, -dy, 1), lo, a);
     down = population(direction(-dx, -dy, -1), b, hi);
   }
   __device__ __forceinline__ Two<R> diagonal(int dx, int dy) {
-    const MomPair<R> mid = ld_pair(at + col.at(dx, dy));
-    return population(direction(-dx, -dy, 0), Source<R>(mid.a), Source<R>(mid.b));
+    const Mom<R>* c = at + col.at(dx, dy);
+    return population(direction(-dx, -dy, 0), Source<T>(c[0]), Source<T>(c[col.plane]));
   }
   __device__ __forceinline__ void add(int i, const Two<R>& f) {
     mom_sum(i, f.a, sum.a);
     mom_sum(i, f.b, sum.b);
   }
   __device__ __forceinline__ void run() {
-    own = ld_pair(at);
+    own.a = at[0];
+    own.b = at[col.plane];
     sum.a = sum.b = Mom<R>{R(0), R(0), R(0), R(0)};
     Two<R> f0, f3, f12, f1, f6, f7, f2, f8, f9;
     column(0, 0, f0, f12, f3);
@@ -337,46 +333,38 @@ struct Gather {
   }
 };
 
-// Resident blocks the registers are held to.  FP32: 64 registers (8-12 bytes
-// spilled) ran a 200^3 step in 117 us, 80 registers (6 blocks) in 122, 96 (5)
-// in 130, 51 (10 blocks, 68 bytes spilled) in 123.
+// Resident blocks the registers are held to.  FP32: 72 registers ran a 200^3
+// step in 109 us and a 96^3 one in 14.9, 64 registers (8 blocks) in 112 and
+// 15.4, 80 (6) in 111 and 15.2, 51 (10) in 121 and 17.9.
 template <typename T>
-constexpr int mom_gather_blocks() { return sizeof(typename Pop<T>::Real) == 8 ? 4 : 8; }
+constexpr int mom_gather_blocks() { return sizeof(typename Pop<T>::Real) == 8 ? 4 : 7; }
 
-// Gather pass of pair k of a list; every thread of the warp calls it.
+// Gather pass of pair k of a list.  A thread past its end passes the gate with
+// the others (a branch around the gate cost 4 % of the step).
 template <typename T, bool WRITE_RHO, bool PDL>
 __device__ __forceinline__ void mom_gather(
-    const MomPair<typename Pop<T>::Real>* m, const PairList& list, int k,
+    const Mom<typename Pop<T>::Real>* m, const PairList& list, int k,
     MomPair<typename Pop<T>::Real>* n, typename Pop<T>::Real* rho,
     typename Pop<T>::Real* psi, const Geom& g, const Phys& p, const StepArgs& a,
     bool inj, float shift_st) {
   using R = typename Pop<T>::Real;
   const bool some = k < list.count;
   const PairAt q = pair_at(g, list, some ? k : list.count - 1);
-  const bool inner = __all_sync(~0u, q.na & NB_INNER);
   pdl_gate<PDL>();
   if (!some) return;
-  MomPair<R> s;
-  if (inner) {
-    Gather<T, true> c{m + q.at, Columns(g, q.x, q.y), q.na, q.nb, shift_st, p.rho_shift};
-    c.run();
-    s = c.sum;
-  } else {
-    Gather<T, false> c{m + q.at, Columns(g, q.x, q.y), q.na, q.nb, shift_st, p.rho_shift};
-    c.run();
-    s = c.sum;
-  }
-  mom_put<R, WRITE_RHO>(q, s, n, k, rho, psi, g, p, a, inj);
+  Gather<T> c{m + q.at, Columns(g, q.x, q.y), q.na, q.nb, shift_st, p.rho_shift};
+  c.run();
+  mom_put<R, WRITE_RHO>(q, c.sum, n, k, rho, psi, g, p, a, inj);
 }
 
 template <typename T, bool WRITE_RHO>
 __global__ void __launch_bounds__(kMomThreads, mom_gather_blocks<T>())
-    k_mom_gather(const MomPair<typename Pop<T>::Real>* m, PairList list,
+    k_mom_gather(const Mom<typename Pop<T>::Real>* m, PairList list,
                  MomPair<typename Pop<T>::Real>* n, typename Pop<T>::Real* rho,
                  typename Pop<T>::Real* psi, Geom g, Phys p, StepArgs a, bool inj,
                  float shift_st) {
-  mom_gather<T, WRITE_RHO, true>(m, list, blockIdx.x * kMomThreads + threadIdx.x, n,
-                                 rho, psi, g, p, a, inj, shift_st);
+  const int k = blockIdx.x * kMomThreads + threadIdx.x;
+  mom_gather<T, WRITE_RHO, true>(m, list, k, n, rho, psi, g, p, a, inj, shift_st);
 }
 
 // The gather of a step that starts from populations (the dense layout in AA
@@ -436,24 +424,24 @@ __device__ __forceinline__ Mom<R> shifted_velocity(const Phys& p, const Mom<R>& 
 // Collide pass of pair k of a list (k < list.count).
 template <typename R, bool WRITE_U, bool PDL>
 __device__ __forceinline__ void mom_collide(const MomPair<R>* n, const PairList& list,
-                                            int k, const Two<R>* psi, MomPair<R>* m,
+                                            int k, const R* psi, Mom<R>* m,
                                             float* vel, const Geom& g, const Phys& p) {
   const PairAt q = pair_at(g, list, k);
   const Columns col(g, q.x, q.y);
   pdl_gate<PDL>();
   const MomPair<R> s = ld_pair(n + k);
-  const Two<R>* at = psi + q.at;
+  const R* at = psi + q.at;
   // psi of the columns: [dy + 1][dx + 1], levels z - 1, z, z + 1, z + 2
   Two<R> mid[9];
   R lo[9], hi[9];
 #pragma unroll
   for (int j = 0; j < 9; ++j) {
     const int dx = j % 3 - 1, dy = j / 3 - 1;
-    const Two<R>* c = at + col.at(dx, dy);
-    mid[j] = *c;
+    const R* c = at + col.at(dx, dy);
+    mid[j] = Two<R>{c[0], c[col.plane]};
     if (dx * dy == 0) {
-      lo[j] = (c - col.plane)->b;
-      hi[j] = (c + col.plane)->a;
+      lo[j] = c[-col.plane];
+      hi[j] = c[2 * col.plane];
     }
   }
   R ax = R(0), ay = R(0), az = R(0), bx = R(0), by = R(0), bz = R(0);
@@ -482,14 +470,11 @@ __device__ __forceinline__ void mom_collide(const MomPair<R>* n, const PairList&
       v[2] = (float)u.b.z;
     }
   }
-  Mom<R>* mm = reinterpret_cast<Mom<R>*>(m);
-  if (q.na && q.nb)
-    st_pair(m + q.at, u);
-  else  // the other half may be a ghost node (odd lz)
-    mm[2 * (size_t)q.at + (q.na ? 0 : 1)] = q.na ? u.a : u.b;
+  if (q.na) m[q.at] = u.a;
+  if (q.nb) m[q.at + col.plane] = u.b;
   if ((q.na | q.nb) & NB_EDGE) {
-    if (q.na) for_images(g, q.x, q.y, q.z, [&](size_t i) { mm[i] = u.a; });
-    if (q.nb) for_images(g, q.x, q.y, q.z + 1, [&](size_t i) { mm[i] = u.b; });
+    if (q.na) for_images(g, q.x, q.y, q.z, [&](uint32_t i) { m[i] = u.a; });
+    if (q.nb) for_images(g, q.x, q.y, q.z + 1, [&](uint32_t i) { m[i] = u.b; });
   }
 }
 
@@ -498,8 +483,8 @@ __device__ __forceinline__ void mom_collide(const MomPair<R>* n, const PairList&
 // collide ended.
 template <typename R, bool WRITE_U>
 __global__ void __launch_bounds__(kMomThreads, sizeof(R) == 8 ? 6 : 8)
-    k_mom_collide(const MomPair<R>* n, PairList list, const Two<R>* psi,
-                  MomPair<R>* m, float* vel, Geom g, Phys p) {
+    k_mom_collide(const MomPair<R>* n, PairList list, const R* psi, Mom<R>* m,
+                  float* vel, Geom g, Phys p) {
   const int k = (int)(gridDim.x - 1 - blockIdx.x) * kMomThreads + threadIdx.x;
   if (k < list.count) mom_collide<R, WRITE_U, true>(n, list, k, psi, m, vel, g, p);
 }
@@ -509,20 +494,19 @@ __global__ void __launch_bounds__(kMomThreads, sizeof(R) == 8 ? 6 : 8)
 // after the same steps, bit for bit.
 template <typename T, int PHASE>
 __global__ void __launch_bounds__(kMomThreads)
-    k_mom_populations(const MomPair<typename Pop<T>::Real>* __restrict__ m,
+    k_mom_populations(const Mom<typename Pop<T>::Real>* __restrict__ m,
                       PairList list, T* __restrict__ pop, Geom g, float shift_st) {
   using R = typename Pop<T>::Real;
   const int k = blockIdx.x * kMomThreads + threadIdx.x;
   if (k >= list.count) return;
   const PairAt q = pair_at(g, list, k);
-  const MomPair<R> v = m[q.at];
   for (int b = 0; b < 2; ++b) {
     const uint32_t nb = b ? q.nb : q.na;
     if (!nb) continue;
-    const Source<R> s(b ? v.b : v.a);
+    const Source<T> s(m[q.at + b * g.ly * g.px]);
     R f[Q];
 #pragma unroll
-    for (int i = 0; i < Q; ++i) f[i] = eq_population<R>(i, s);
+    for (int i = 0; i < Q; ++i) f[i] = eq_population<T>(i, s);
     Nbr w;
     w.init(g, q.x, q.y, q.z + b);
     scatter<T, PHASE ^ 1>(pop, g.plane, w, nb, w.n, R(shift_st), f);
@@ -578,7 +562,7 @@ __global__ void __launch_bounds__(32 * kPairRows)
     k_mom_tiles(const uint32_t* __restrict__ nbw, TileCount* counts,
                 const TileCount* __restrict__ at, uint2* __restrict__ words,
                 uint32_t* __restrict__ xyz, uint2* __restrict__ nodes, Geom g) {
-  __shared__ uint32_t row_in[kPairRows], row_out[kPairRows], row_nodes[kPairRows];
+  __shared__ uint32_t row_pairs[kPairRows], row_nodes[kPairRows];
   const TileGrid tg(g);
   const long long tile = blockIdx.x;
   const int lane = threadIdx.x & 31, row = threadIdx.x / 32;
@@ -587,36 +571,31 @@ __global__ void __launch_bounds__(32 * kPairRows)
             z = (int)(tile / ((long long)tg.nx * tg.ny)) * kTileZ + row / kTileY * 2;
   const uint32_t na = tile_word(nbw, g, x, y, z), nb = tile_word(nbw, g, x, y, z + 1);
   const bool any = (na | nb) != 0u;
-  const bool in = ((na & nb) & kNbAllFluid) == kNbAllFluid && !nb_kind(na);
-  const uint32_t bin = __ballot_sync(~0u, in), bout = __ballot_sync(~0u, any && !in);
+  const uint32_t bp = __ballot_sync(~0u, any);
   const uint32_t ba = __ballot_sync(~0u, na != 0u), bb = __ballot_sync(~0u, nb != 0u);
   if (lane == 0) {
-    row_in[row] = __popc(bin);
-    row_out[row] = __popc(bout);
+    row_pairs[row] = __popc(bp);
     row_nodes[row] = __popc(ba) + __popc(bb);
   }
   __syncthreads();
-  uint32_t inner = 0, outer = 0, count = 0, in0 = 0, out0 = 0, nodes0 = 0;
+  uint32_t pairs = 0, count = 0, pairs0 = 0, nodes0 = 0;
   for (int r = 0; r < kPairRows; ++r) {
     if (r == row) {
-      in0 = inner;
-      out0 = outer;
+      pairs0 = pairs;
       nodes0 = count;
     }
-    inner += row_in[r];
-    outer += row_out[r];
+    pairs += row_pairs[r];
     count += row_nodes[r];
   }
   if (COUNT) {
-    if (threadIdx.x == 0) counts[tile] = TileCount{inner + outer, count};
+    if (threadIdx.x == 0) counts[tile] = TileCount{pairs, count};
     return;
   }
   const TileCount w = at[tile];
   const uint32_t below = (1u << lane) - 1u;
   if (any) {
-    const uint32_t k = w.pairs + (in ? in0 + __popc(bin & below)
-                                     : inner + out0 + __popc(bout & below));
-    words[k] = make_uint2(na | (in ? NB_INNER : 0u), nb);
+    const uint32_t k = w.pairs + pairs0 + __popc(bp & below);
+    words[k] = make_uint2(na, nb);
     xyz[k] = pack_xyz(x, y, z);
   }
   const uint32_t k = w.nodes + nodes0;

@@ -177,10 +177,37 @@ __device__ __forceinline__ void pair_scatter(T* cpop, uint32_t cs, int k,
   }
 }
 
+// Equilibrium (kernels.cuh) of two nodes: base, and the terms of a direction
+// and of its opposite (term(base, -eu), in the operations that give its bits).
+template <typename T>
+struct Equilibrium2 {
+  static __device__ __forceinline__ float2 base(float2 usq) {
+    return p_fma(p_dup(-1.5f), usq, p_dup(1.f));
+  }
+  static __device__ __forceinline__ float2 term(float2 base, float2 eu) {
+    return p_fma(eu, p_fma(p_dup(4.5f), eu, p_dup(3.f)), base);
+  }
+  static __device__ __forceinline__ float2 opposite(float2 base, float2 eu) {
+    return p_fma(eu, p_fma(p_dup(4.5f), eu, p_dup(-3.f)), base);
+  }
+};
+template <>
+struct Equilibrium2<__half> {
+  static __device__ __forceinline__ float2 base(float2 usq) {
+    return p_sub(p_dup(1.f), p_mul(p_dup(1.5f), usq));
+  }
+  static __device__ __forceinline__ float2 term(float2 base, float2 eu) {
+    return p_add(p_fma(p_mul(p_dup(4.5f), eu), eu, base), p_mul(p_dup(3.f), eu));
+  }
+  static __device__ __forceinline__ float2 opposite(float2 base, float2 eu) {
+    return p_sub(p_fma(p_mul(p_dup(4.5f), eu), eu, base), p_mul(p_dup(3.f), eu));
+  }
+};
+
 // Force, velocity shift and BGK of two interior fluid nodes: collide() of
 // kernels.cuh, operation for operation, in packed form.  psi_nb(i) returns
 // psi at x + e_i of both nodes.
-template <typename PsiNb>
+template <typename T, typename PsiNb>
 __device__ __forceinline__ void collide2(const Phys& p, float2 d, float2 psi_self,
                                          PsiNb psi_nb, float2 (&f)[Q],
                                          float2& ux, float2& uy, float2& uz) {
@@ -208,28 +235,41 @@ __device__ __forceinline__ void collide2(const Phys& p, float2 d, float2 psi_sel
   ux = p_mul(p_fma(tau, Fx, ux), inv_rho);
   uy = p_mul(p_fma(tau, Fy, uy), inv_rho);
   uz = p_mul(p_fma(tau, Fz, uz), inv_rho);
-  const float2 usq15 =
-      p_mul(p_dup(1.5f), p_fma(uz, uz, p_fma(uy, uy, p_mul(ux, ux))));
+  const float2 usq = p_fma(uz, uz, p_fma(uy, uy, p_mul(ux, ux)));
   const float2 omega = p_dup(p.omega);
-  const float2 base = p_sub(p_dup(1.f), usq15);
   const float2 wd0 = p_mul(p_dup(weight<float>(0)), d),
                wd1 = p_mul(p_dup(weight<float>(1)), d),
                wd2 = p_mul(p_dup(weight<float>(4)), d);
-  const bool eq = p.omega == 1.f;  // as in collide(): f* = feq
-  f[0] = eq ? p_mul(wd0, base) : p_fma(p_sub(p_mul(wd0, base), f[0]), omega, f[0]);
-#pragma unroll
-  for (int i = 1; i <= 9; ++i) {
+  auto e_dot_u = [&](int i) {
     float2 eu = p_dup(0.f);
     if (ex(i)) eu = ex(i) > 0 ? p_add(eu, ux) : p_sub(eu, ux);
     if (ey(i)) eu = ey(i) > 0 ? p_add(eu, uy) : p_sub(eu, uy);
     if (ez(i)) eu = ez(i) > 0 ? p_add(eu, uz) : p_sub(eu, uz);
+    return eu;
+  };
+  if (p.omega == 1.f) {  // as in collide(): f* = feq
+    const float2 base = Equilibrium2<T>::base(usq);
+    f[0] = p_mul(wd0, base);
+#pragma unroll
+    for (int i = 1; i <= 9; ++i) {
+      const float2 eu = e_dot_u(i), wd = (i <= 3) ? wd1 : wd2;
+      f[i] = p_mul(wd, Equilibrium2<T>::term(base, eu));
+      f[opp(i)] = p_mul(wd, Equilibrium2<T>::opposite(base, eu));
+    }
+    return;
+  }
+  const float2 base = p_sub(p_dup(1.f), p_mul(p_dup(1.5f), usq));
+  f[0] = p_fma(p_sub(p_mul(wd0, base), f[0]), omega, f[0]);
+#pragma unroll
+  for (int i = 1; i <= 9; ++i) {
+    const float2 eu = e_dot_u(i);
     const float2 sym = p_fma(p_mul(p_dup(4.5f), eu), eu, base);
     const float2 anti = p_mul(p_dup(3.f), eu);
     const float2 wd = (i <= 3) ? wd1 : wd2;
     const float2 feq_i = p_mul(wd, p_add(sym, anti));
     const float2 feq_o = p_mul(wd, p_sub(sym, anti));
-    f[i] = eq ? feq_i : p_fma(p_sub(feq_i, f[i]), omega, f[i]);
-    f[opp(i)] = eq ? feq_o : p_fma(p_sub(feq_o, f[opp(i)]), omega, f[opp(i)]);
+    f[i] = p_fma(p_sub(feq_i, f[i]), omega, f[i]);
+    f[opp(i)] = p_fma(p_sub(feq_o, f[opp(i)]), omega, f[opp(i)]);
   }
 }
 
@@ -378,7 +418,7 @@ __device__ __forceinline__ void pair_update(T* cpop, uint32_t cs,
     const uint32_t pb = (uint32_t)psi_index(g, q.b.x, q.b.y, q.b.z);
     const int sy = g.pxg, sz = (g.ly + 2) * g.pxg;
     pr.ready();
-    collide2(
+    collide2<T>(
         p, d, make_float2(pr.self(pa), pr.self(pb)),
         [&](int i) {
           const int o = ex(i) + ey(i) * sy + ez(i) * sz;

@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(256)
         const R* p0 = ring + slot_of(z) * slot_elems;
         const R* pp = ring + slot_of(z + 1) * slot_elems;
         const int c = (ly_ + 1) * kBoxX + (tid & 31) + 4;
-        collide<R>(
+        collide<T, R>(
             p, d, p0[c],
             [&](int i) {
               const R* pl = ez(i) < 0 ? pm : (ez(i) > 0 ? pp : p0);
