@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(kBandThreads, 1)
         const int ca = (na.y - y0 + 1) * P + na.x + 1;
         const int cb = (nbn.y - y0 + 1) * P + nbn.x + 1;
         collide2<T>(
-            p, d, make_float2(s0[ca], s0[cb]),
+            p.omega == 1.f, p, d, make_float2(s0[ca], s0[cb]),
             [&](int i) {
               const float* pl = ez(i) < 0 ? sm : (ez(i) > 0 ? spl : s0);
               const int o = ey(i) * P + ex(i);

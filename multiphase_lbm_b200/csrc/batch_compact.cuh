@@ -18,6 +18,8 @@
 #include "compact2.cuh"
 #include "lattice.cuh"
 
+#include <type_traits>
+
 namespace mlbm {
 
 constexpr int kBCThreads = 256;
@@ -102,14 +104,19 @@ __global__ void __launch_bounds__(kBCThreads, 3)
   const bool inj = bc_inject(D.p, a.step);
   const long long k = 2 * ((b - upre[d]) * kBCThreads + threadIdx.x);
   if (k >= D.nfluid) return;
-  if (ph == 0)
-    pair_update<T, 0, false>(static_cast<T*>(D.cpop), D.cs, D.cinfo, D.wtab,
-                             (int)k, D.nfluid, PsiPlain{D.psi}, nullptr, D.g,
-                             D.p, a, inj);
-  else
-    pair_update<T, 1, false>(static_cast<T*>(D.cpop), D.cs, D.cinfo, D.wtab,
-                             (int)k, D.nfluid, PsiPlain{D.psi}, nullptr, D.g,
-                             D.p, a, inj);
+  auto update = [&](auto phase, auto eq) {
+    pair_update<T, decltype(phase)::value, false, decltype(eq)::value>(
+        static_cast<T*>(D.cpop), D.cs, D.cinfo, D.wtab, (int)k, D.nfluid,
+        PsiPlain{D.psi}, nullptr, D.g, D.p, a, inj);
+  };
+  using std::integral_constant;
+  if (D.p.omega == 1.f) {  // a batch with other taus beside
+    if (ph == 0) update(integral_constant<int, 0>(), std::true_type());
+    else update(integral_constant<int, 1>(), std::true_type());
+  } else {
+    if (ph == 0) update(integral_constant<int, 0>(), std::false_type());
+    else update(integral_constant<int, 1>(), std::false_type());
+  }
 }
 
 }  // namespace mlbm

@@ -30,6 +30,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <utility>
 #include <vector>
 
 #include "../../include/mlbm_driver.h"
@@ -59,20 +60,32 @@ struct Dims {
   }
 };
 
-// class: 1 liquid, 2 gas, 0 neither (solid or in between)
+// Periodic wrap of a coordinate at most one step outside.
+__device__ __forceinline__ int wrap(int v, int n) {
+  return v < 0 ? v + n : v >= n ? v - n : v;
+}
+
+// class: 1 liquid, 2 gas, 0 neither (solid or in between).  A node starts under
+// the first node of its run of the class along z within the warp, so that the
+// links along z are those between warps only.
 __global__ void k_classify(const float* __restrict__ rho,
                            const uint8_t* __restrict__ fluid, Dims d,
                            float rhol, float rhog, uint8_t* __restrict__ cls,
                            int* __restrict__ parent) {
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= d.n) return;
   uint8_t c = 0;
-  if (fluid[k]) {
+  if (k < d.n && fluid[k]) {
     const float r = rho[k];
     c = r > rhol ? 1 : (r < rhog ? 2 : 0);
   }
+  const int lane = threadIdx.x & 31;
+  const int before = __shfl_up_sync(~0u, (int)c, 1);
+  const unsigned starts =
+      __ballot_sync(~0u, lane == 0 || before != c || k % d.lz == 0);
+  if (k >= d.n) return;
   cls[k] = c;
-  parent[k] = (int)k;
+  const unsigned upto = starts & (~0u >> (31 - lane));
+  parent[k] = (int)k - (lane - (31 - __clz(upto)));
 }
 
 __device__ __forceinline__ int uf_find(const int* parent, int a) {
@@ -102,6 +115,9 @@ __device__ __forceinline__ void uf_unite(int* parent, int a, int b) {
 }
 
 // Each node unites with its +x, +y, +z neighbours (periodic) of its class.
+// Along z only across warps and around the box (k_classify linked the rest);
+// along x and y not where the node before it along z, of the same run, has the
+// same link to the same run.
 __global__ void k_unite(const uint8_t* __restrict__ cls, Dims d,
                         int* __restrict__ parent) {
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -110,23 +126,35 @@ __global__ void k_unite(const uint8_t* __restrict__ cls, Dims d,
   if (!c) return;
   int x, y, z;
   d.xyz(k, x, y, z);
-  const long long q[3] = {d.idx(x + 1 < d.lx ? x + 1 : 0, y, z),
-                          d.idx(x, y + 1 < d.ly ? y + 1 : 0, z),
-                          d.idx(x, y, z + 1 < d.lz ? z + 1 : 0)};
+  const bool run = (threadIdx.x & 31) != 0 && z != 0 && cls[k - 1] == c;
+  const long long q[2] = {d.idx(x + 1 < d.lx ? x + 1 : 0, y, z),
+                          d.idx(x, y + 1 < d.ly ? y + 1 : 0, z)};
 #pragma unroll
-  for (int j = 0; j < 3; ++j)
-    if (q[j] != k && cls[q[j]] == c) uf_unite(parent, (int)k, (int)q[j]);
+  for (int j = 0; j < 2; ++j)
+    if (q[j] != k && cls[q[j]] == c && !(run && cls[q[j] - 1] == c))
+      uf_unite(parent, (int)k, (int)q[j]);
+  if (z + 1 < d.lz) {
+    if ((threadIdx.x & 31) == 31 && cls[k + 1] == c)
+      uf_unite(parent, (int)k, (int)k + 1);
+  } else if (d.lz > 1 && cls[k - z] == c) {
+    uf_unite(parent, (int)k, (int)(k - z));
+  }
 }
 
-// Flatten every node onto its root and count the members of every root.
+// Flatten every node onto its root and count the members of every root: one
+// atomic per root in a warp (one per node on a few roots took 407 us of the
+// 1.4 ms at 128^3).
 __global__ void k_flatten(const uint8_t* __restrict__ cls, Dims d,
                           int* __restrict__ parent, int* __restrict__ size) {
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= d.n) return;
-  if (!cls[k]) return;
-  const int r = uf_find(parent, (int)k);
-  parent[k] = r;
-  atomicAdd(size + r, 1);
+  int r = -1;
+  if (k < d.n && cls[k]) {
+    r = uf_find(parent, (int)k);
+    parent[k] = r;
+  }
+  const unsigned same = __match_any_sync(~0u, r);
+  if (r >= 0 && __ffs(same) - 1 == (int)(threadIdx.x & 31))
+    atomicAdd(size + r, __popc(same));
 }
 
 // keep[k] = 1 for a root of a cluster of class c with >= kMinCluster nodes.
@@ -163,15 +191,23 @@ __global__ void k_boundary(const uint8_t* __restrict__ fluid,
                            const uint8_t* __restrict__ cls, Dims d, float rhol,
                            unsigned long long* __restrict__ counts) {
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= d.n || cls[k] != 1) return;
-  int x, y, z;
-  d.xyz(k, x, y, z);
-  for (int i = 1; i < 19; ++i) {
-    const int nx = (x - c_ex[i] + d.lx) % d.lx, ny = (y - c_ey[i] + d.ly) % d.ly,
-              nz = (z - c_ez[i] + d.lz) % d.lz;
-    const long long q = d.idx(nx, ny, nz);
-    if (!fluid[q]) { atomicAdd(counts, 1ull); return; }
-    if (rho[q] < rhol) { atomicAdd(counts + 1, 1ull); return; }
+  int first = 0;  // 1 solid, 2 not liquid
+  if (k < d.n && cls[k] == 1) {
+    int x, y, z;
+    d.xyz(k, x, y, z);
+    for (int i = 1; i < 19 && !first; ++i) {
+      const int nx = wrap(x - c_ex[i], d.lx), ny = wrap(y - c_ey[i], d.ly),
+                nz = wrap(z - c_ez[i], d.lz);
+      const long long q = d.idx(nx, ny, nz);
+      if (!fluid[q]) first = 1;
+      else if (rho[q] < rhol) first = 2;
+    }
+  }
+  const unsigned solid = __ballot_sync(~0u, first == 1),
+                 vapour = __ballot_sync(~0u, first == 2);
+  if ((threadIdx.x & 31) == 0) {
+    if (solid) atomicAdd(counts, (unsigned long long)__popc(solid));
+    if (vapour) atomicAdd(counts + 1, (unsigned long long)__popc(vapour));
   }
 }
 
@@ -183,25 +219,53 @@ __global__ void k_solid_pairs(const int* __restrict__ label,
                               unsigned long long* __restrict__ keys,
                               unsigned long long* __restrict__ n_keys) {
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= d.n) return;
-  const int L = label[k];
-  if (!L) return;
-  int x, y, z;
-  d.xyz(k, x, y, z);
-  const long long q[6] = {d.idx(x > 0 ? x - 1 : d.lx - 1, y, z),
-                          d.idx(x, y > 0 ? y - 1 : d.ly - 1, z),
-                          d.idx(x, y, z > 0 ? z - 1 : d.lz - 1),
-                          d.idx(x < d.lx - 1 ? x + 1 : 0, y, z),
-                          d.idx(x, y < d.ly - 1 ? y + 1 : 0, z),
-                          d.idx(x, y, z < d.lz - 1 ? z + 1 : 0)};
+  const int L = k < d.n ? label[k] : 0;
+  unsigned long long key[6];
+  int mine = 0;
+  if (L) {
+    int x, y, z;
+    d.xyz(k, x, y, z);
+    const long long q[6] = {d.idx(x > 0 ? x - 1 : d.lx - 1, y, z),
+                            d.idx(x, y > 0 ? y - 1 : d.ly - 1, z),
+                            d.idx(x, y, z > 0 ? z - 1 : d.lz - 1),
+                            d.idx(x < d.lx - 1 ? x + 1 : 0, y, z),
+                            d.idx(x, y < d.ly - 1 ? y + 1 : 0, z),
+                            d.idx(x, y, z < d.lz - 1 ? z + 1 : 0)};
 #pragma unroll
-  for (int j = 0; j < 6; ++j) {
-    const int64_t sn = solid_number[q[j]];
-    if (sn == 0 || label[q[j]] == L) continue;
-    const unsigned long long slot = atomicAdd(n_keys, 1ull);
-    if (EMIT)
-      keys[slot] = ((unsigned long long)(unsigned)L << 32) | (unsigned)(uint32_t)sn;
+    for (int j = 0; j < 6; ++j) {
+      key[j] = 0;  // no key: L > 0
+      if (label[q[j]] == L) continue;
+      const int64_t sn = solid_number[q[j]];
+      if (sn == 0) continue;
+      key[j] = ((unsigned long long)(unsigned)L << 32) | (unsigned)(uint32_t)sn;
+      ++mine;
+    }
   }
+  // one atomic per warp; a lane's keys follow those of the lanes before it
+  const int lane = threadIdx.x & 31;
+  int upto = mine;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int v = __shfl_up_sync(~0u, upto, off);
+    if (lane >= off) upto += v;
+  }
+  const int total = __shfl_sync(~0u, upto, 31);
+  if (!total) return;
+  unsigned long long slot = 0;
+  if (lane == 31) slot = atomicAdd(n_keys, (unsigned long long)total);
+  slot = __shfl_sync(~0u, slot, 31) + (unsigned)(upto - mine);
+  if (EMIT && L) {
+#pragma unroll
+    for (int j = 0; j < 6; ++j)
+      if (key[j]) keys[slot++] = key[j];
+  }
+}
+
+// Cluster numbers as the caller's type.
+__global__ void k_widen(const int* __restrict__ label, long long n,
+                        int64_t* __restrict__ out) {
+  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < n) out[k] = label[k];
 }
 
 // Distinct pairs and distinct clusters among sorted keys.
@@ -292,18 +356,31 @@ mlbm_status cl_fail(cudaError_t e, const char* where) {
   return set_error(MLBM_ERR_CUDA, msg);
 }
 
-// Device buffers of one call, freed on every return path.
+// Device buffers of one call, freed on every return path.  take() lays buffers
+// out one after the other, alloc() makes them one allocation (an allocation
+// and its release cost about half a millisecond of host time, whatever its
+// size).
 struct ClBuffers {
   std::vector<void*> ptrs;
+  std::vector<std::pair<void**, size_t>> parts;
+  size_t bytes = 0;
   ~ClBuffers() {
     for (void* p : ptrs) cudaFree(p);
   }
   template <typename T>
-  cudaError_t alloc(T** p, size_t count) {
+  void take(T** p, size_t count) {
+    parts.emplace_back(reinterpret_cast<void**>(p), bytes);
+    bytes += (count * sizeof(T) + 255) / 256 * 256;
+  }
+  cudaError_t alloc() {
     void* v = nullptr;
-    const cudaError_t e = cudaMalloc(&v, count * sizeof(T) + 16);
-    if (e == cudaSuccess) ptrs.push_back(v);
-    *p = static_cast<T*>(v);
+    const cudaError_t e = cudaMalloc(&v, bytes);
+    if (e == cudaSuccess) {
+      ptrs.push_back(v);
+      for (auto& q : parts) *q.first = static_cast<char*>(v) + q.second;
+    }
+    parts.clear();
+    bytes = 0;
     return e;
   }
 };
@@ -342,31 +419,35 @@ extern "C" mlbm_status mlbm_cluster_stats_gpu(
                               // [5..8] sums, [9] liquid nodes
   unsigned* d_flags;          // [0] faces, [1] max radius bits
   int* d_occ;
-  CL_TRY(b.alloc(&d_rho, n), "cluster_stats_gpu buffers");
-  CL_TRY(b.alloc(&d_fluid, n), "cluster_stats_gpu buffers");
-  CL_TRY(b.alloc(&d_cls, n), "cluster_stats_gpu buffers");
-  CL_TRY(b.alloc(&d_parent, n), "cluster_stats_gpu buffers");
-  CL_TRY(b.alloc(&d_size, n), "cluster_stats_gpu buffers");
-  CL_TRY(b.alloc(&d_keep, n), "cluster_stats_gpu buffers");
-  CL_TRY(b.alloc(&d_prefix, n), "cluster_stats_gpu buffers");
-  CL_TRY(b.alloc(&d_liq, n), "cluster_stats_gpu buffers");
-  CL_TRY(b.alloc(&d_gas, n), "cluster_stats_gpu buffers");
-  CL_TRY(b.alloc(&d_cnt, 16), "cluster_stats_gpu buffers");
-  CL_TRY(b.alloc(&d_flags, 4), "cluster_stats_gpu buffers");
-  CL_TRY(b.alloc(&d_occ, (size_t)lx + ly + lz), "cluster_stats_gpu buffers");
+  size_t scan_bytes = 0;
+  d_keep = d_prefix = nullptr;
+  CL_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, d_keep, d_prefix, (int)n),
+         "cluster_stats_gpu scan");
+  unsigned char* d_scan;
+  b.take(&d_rho, n);
+  b.take(&d_fluid, n);
+  b.take(&d_cls, n);
+  b.take(&d_parent, n);
+  b.take(&d_keep, n);
+  b.take(&d_prefix, n);
+  b.take(&d_liq, n);
+  b.take(&d_gas, n);
+  // zeroed together: sizes, counters, flags, occupied planes
+  b.take(&d_size, n);
+  b.take(&d_cnt, 16);
+  b.take(&d_flags, 4);
+  b.take(&d_occ, (size_t)lx + ly + lz);
+  b.take(&d_scan, scan_bytes);
+  // the solid numbers, and the labels on their way out
+  if (solid_number || liq_labels_out || gas_labels_out) b.take(&d_sn, n);
+  CL_TRY(b.alloc(), "cluster_stats_gpu buffers");
   CL_TRY(cudaMemcpy(d_rho, rho, n * sizeof(float), cudaMemcpyHostToDevice),
          "cluster_stats_gpu upload");
   CL_TRY(cudaMemcpy(d_fluid, is_fluid, n, cudaMemcpyHostToDevice),
          "cluster_stats_gpu upload");
-  if (solid_number) {
-    CL_TRY(b.alloc(&d_sn, n), "cluster_stats_gpu buffers");
-    CL_TRY(cudaMemcpy(d_sn, solid_number, n * sizeof(int64_t), cudaMemcpyHostToDevice),
-           "cluster_stats_gpu upload");
-  }
-  CL_TRY(cudaMemset(d_size, 0, n * sizeof(int)), "cluster_stats_gpu");
-  CL_TRY(cudaMemset(d_cnt, 0, 16 * sizeof(unsigned long long)), "cluster_stats_gpu");
-  CL_TRY(cudaMemset(d_flags, 0, 4 * sizeof(unsigned)), "cluster_stats_gpu");
-  CL_TRY(cudaMemset(d_occ, 0, ((size_t)lx + ly + lz) * sizeof(int)), "cluster_stats_gpu");
+  CL_TRY(cudaMemset(d_size, 0,
+                    reinterpret_cast<char*>(d_scan) - reinterpret_cast<char*>(d_size)),
+         "cluster_stats_gpu");
 
   // components of both classes, each rooted at its first node in the scan
   k_classify<<<grid, 256>>>(d_rho, d_fluid, d, rhol, rhog, d_cls, d_parent);
@@ -374,13 +455,11 @@ extern "C" mlbm_status mlbm_cluster_stats_gpu(
   k_flatten<<<grid, 256>>>(d_cls, d, d_parent, d_size);
   CL_TRY(cudaGetLastError(), "cluster_stats_gpu labelling");
 
+  if (solid_number)
+    CL_TRY(cudaMemcpy(d_sn, solid_number, n * sizeof(int64_t), cudaMemcpyHostToDevice),
+           "cluster_stats_gpu upload");
+
   // cluster numbers of the kept clusters, per class
-  size_t scan_bytes = 0;
-  CL_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, d_keep, d_prefix, (int)n),
-         "cluster_stats_gpu scan");
-  void* d_scan;
-  CL_TRY(b.alloc(reinterpret_cast<unsigned char**>(&d_scan), scan_bytes),
-         "cluster_stats_gpu buffers");
   long long counts[2] = {0, 0};
   for (int c = 1; c <= 2; ++c) {
     int* lab = c == 1 ? d_liq : d_gas;
@@ -414,7 +493,7 @@ extern "C" mlbm_status mlbm_cluster_stats_gpu(
   // cluster order and wet coordination number from the distinct
   // (liquid cluster, solid number) pairs, :535-561
   unsigned long long pairs = 0, touching = 0;
-  if (d_sn && liq_count > 0) {
+  if (solid_number && liq_count > 0) {
     k_solid_pairs<false><<<grid, 256>>>(d_liq, d_sn, d, nullptr, d_cnt + 2);
     unsigned long long m = 0;
     CL_TRY(cudaMemcpy(&m, d_cnt + 2, sizeof m, cudaMemcpyDeviceToHost),
@@ -422,19 +501,23 @@ extern "C" mlbm_status mlbm_cluster_stats_gpu(
     if (m >= (1ull << 31))
       return set_error(MLBM_ERR_ARG, "cluster_stats_gpu: too many cluster-solid contacts");
     if (m > 0) {
-      unsigned long long *d_keys, *d_sorted;
-      CL_TRY(b.alloc(&d_keys, m), "cluster_stats_gpu pairs");
-      CL_TRY(b.alloc(&d_sorted, m), "cluster_stats_gpu pairs");
-      CL_TRY(cudaMemset(d_cnt + 2, 0, sizeof(unsigned long long)), "cluster_stats_gpu");
-      k_solid_pairs<true><<<grid, 256>>>(d_liq, d_sn, d, d_keys, d_cnt + 2);
+      unsigned long long *d_keys = nullptr, *d_sorted = nullptr;
+      unsigned char* d_sort;
+      // the low half is a solid number, the high half a cluster number
+      int bits = 32;
+      while (bits < 64 && (liq_count >> (bits - 32)) != 0) ++bits;
       size_t sort_bytes = 0;
       CL_TRY(cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, d_keys, d_sorted,
-                                            (int)m),
+                                            (int)m, 0, bits),
              "cluster_stats_gpu sort");
-      unsigned char* d_sort;
-      CL_TRY(b.alloc(&d_sort, sort_bytes), "cluster_stats_gpu sort");
+      b.take(&d_keys, m);
+      b.take(&d_sorted, m);
+      b.take(&d_sort, sort_bytes);
+      CL_TRY(b.alloc(), "cluster_stats_gpu pairs");
+      CL_TRY(cudaMemset(d_cnt + 2, 0, sizeof(unsigned long long)), "cluster_stats_gpu");
+      k_solid_pairs<true><<<grid, 256>>>(d_liq, d_sn, d, d_keys, d_cnt + 2);
       CL_TRY(cub::DeviceRadixSort::SortKeys(d_sort, sort_bytes, d_keys, d_sorted,
-                                            (int)m),
+                                            (int)m, 0, bits),
              "cluster_stats_gpu sort");
       k_count_distinct<<<(unsigned)((m + 255) / 256), 256>>>(d_sorted, (long long)m,
                                                              d_cnt + 3);
@@ -492,11 +575,9 @@ extern "C" mlbm_status mlbm_cluster_stats_gpu(
   for (int c = 0; c < 2; ++c) {
     int64_t* dst = c == 0 ? liq_labels_out : gas_labels_out;
     if (!dst) continue;
-    std::vector<int> h((size_t)n);
-    CL_TRY(cudaMemcpy(h.data(), c == 0 ? d_liq : d_gas, n * sizeof(int),
-                      cudaMemcpyDeviceToHost),
+    k_widen<<<grid, 256>>>(c == 0 ? d_liq : d_gas, n, d_sn);
+    CL_TRY(cudaMemcpy(dst, d_sn, n * sizeof(int64_t), cudaMemcpyDeviceToHost),
            "cluster_stats_gpu labels");
-    for (long long k = 0; k < n; ++k) dst[k] = h[k];
   }
   CL_TRY(cudaGetLastError(), "cluster_stats_gpu");
   return MLBM_OK;

@@ -250,7 +250,9 @@ void launch_c2_update(mlbm_lattice* lat, const StepArgs& a, bool wu, bool inj,
   T* cpop = static_cast<T*>(c.cpop);
   const uint32_t cs = (uint32_t)c.cs;
   const float* psi = static_cast<const float*>(lat->psi);
-  auto kernel = wu ? k_cupdate<T, PHASE, true> : k_cupdate<T, PHASE, false>;
+  const bool eq = lat->phys.omega == 1.f;
+  auto kernel = wu ? (eq ? k_cupdate<T, PHASE, true, true> : k_cupdate<T, PHASE, true, false>)
+                   : (eq ? k_cupdate<T, PHASE, false, true> : k_cupdate<T, PHASE, false, false>);
   launch_overlapped(overlap, kernel, grid, kC2Threads, 0, lat->stream, cpop, cs,
                     (const uint2*)c.cinfo,
                     (const uint2*)c.wtab, (int)kb, (int)ke, psi, lat->vel,

@@ -115,6 +115,7 @@ namespace mlbm {
 // bench that beat 3, 4 and 6 CTAs per SM.  Both kernels advance the compact
 // indices [kbeg, nfluid): the whole lattice, or the own planes of a slab
 // lattice (kbeg is a plane start, so it is even).
+// EQ: omega is 1 (collide2).
 template <int PHASE>
 constexpr int c2_nodes_per_thread() { return PHASE == 0 ? 1 : 2; }
 constexpr int c2_update_nodes_per_thread() { return 2; }
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(kC2Threads, 5)
                                         rho_out, psi, g, p, a, inj);
 }
 
-template <typename T, int PHASE, bool WRITE_U>
+template <typename T, int PHASE, bool WRITE_U, bool EQ>
 __global__ void __launch_bounds__(kC2Threads, 3)
     k_cupdate(T* __restrict__ cpop, uint32_t cs, const uint2* __restrict__ cinfo,
               const uint2* __restrict__ wtab, int kbeg, int nfluid,
@@ -148,7 +149,7 @@ __global__ void __launch_bounds__(kC2Threads, 3)
   const long long k = kbeg + c2_update_nodes_per_thread() *
                                  ((long long)blockIdx.x * kC2Threads + threadIdx.x);
   if (k >= nfluid) return;
-  pair_update<T, PHASE, WRITE_U, PsiPlain, true>(cpop, cs, cinfo, wtab, (int)k,
+  pair_update<T, PHASE, WRITE_U, EQ, PsiPlain, true>(cpop, cs, cinfo, wtab, (int)k,
                                                  nfluid, PsiPlain{psi}, vel, g,
                                                  p, a, inj);
 }

@@ -205,11 +205,14 @@ struct Equilibrium2<__half> {
 };
 
 // Force, velocity shift and BGK of two interior fluid nodes: collide() of
-// kernels.cuh, operation for operation, in packed form.  psi_nb(i) returns
+// kernels.cuh, operation for operation, in packed form; eq: omega is 1 (a
+// constant where the caller knows it: tested here, it costs the general
+// update 1.4 %).  psi_nb(i) returns
 // psi at x + e_i of both nodes.
 template <typename T, typename PsiNb>
-__device__ __forceinline__ void collide2(const Phys& p, float2 d, float2 psi_self,
-                                         PsiNb psi_nb, float2 (&f)[Q],
+__device__ __forceinline__ void collide2(bool eq, const Phys& p, float2 d,
+                                         float2 psi_self, PsiNb psi_nb,
+                                         float2 (&f)[Q],
                                          float2& ux, float2& uy, float2& uz) {
   float2 sx = p_dup(0.f), sy = p_dup(0.f), sz = p_dup(0.f);
 #pragma unroll
@@ -247,7 +250,7 @@ __device__ __forceinline__ void collide2(const Phys& p, float2 d, float2 psi_sel
     if (ez(i)) eu = ez(i) > 0 ? p_add(eu, uz) : p_sub(eu, uz);
     return eu;
   };
-  if (p.omega == 1.f) {  // as in collide(): f* = feq
+  if (eq) {  // as in collide(): f* = feq
     const float2 base = Equilibrium2<T>::base(usq);
     f[0] = p_mul(wd0, base);
 #pragma unroll
@@ -376,8 +379,15 @@ __device__ __forceinline__ void pair_density(const T* cpop, uint32_t cs,
   if (q.two) store_psi<float>(psi, g, q.b.x, q.b.y, q.b.z, psi_of<float>(p, d.y));
 }
 
+// Shared memory of the gather/push update: one array for every form of
+// pair_update in a kernel.
+__device__ __forceinline__ uint32_t (*parked_addresses())[kC2Threads] {
+  __shared__ uint32_t parked[2 * Q][kC2Threads];
+  return parked;
+}
+
 // Update pass of one pair (the work of k_cupdate for two nodes).
-template <typename T, int PHASE, bool WRITE_U, class PsiR, bool PDL = false>
+template <typename T, int PHASE, bool WRITE_U, bool EQ, class PsiR, bool PDL = false>
 __device__ __forceinline__ void pair_update(T* cpop, uint32_t cs,
                                             const uint2* __restrict__ cinfo,
                                             const uint2* __restrict__ wtab,
@@ -393,8 +403,8 @@ __device__ __forceinline__ void pair_update(T* cpop, uint32_t cs,
   // collision they leave too few for 3 CTAs per SM.  Each node's addresses
   // are parked right after its own gather, so only 19 are live at a time.
   // (k_cupdate: 1-D blocks of kC2Threads.)
-  __shared__ uint32_t parked[PHASE == 0 ? 2 * Q : 1][PHASE == 0 ? kC2Threads : 1];
   if (PHASE == 0) {
+    uint32_t(*parked)[kC2Threads] = parked_addresses();
     aa_addresses0(wtab, g, cs, q.a, A);
 #pragma unroll
     for (int e = 0; e < Q; ++e) {
@@ -419,7 +429,7 @@ __device__ __forceinline__ void pair_update(T* cpop, uint32_t cs,
     const int sy = g.pxg, sz = (g.ly + 2) * g.pxg;
     pr.ready();
     collide2<T>(
-        p, d, make_float2(pr.self(pa), pr.self(pb)),
+        EQ, p, d, make_float2(pr.self(pa), pr.self(pb)),
         [&](int i) {
           const int o = ex(i) + ey(i) * sy + ez(i) * sz;
           return make_float2(pr.nb(pa + o, i), pr.nb(pb + o, i));
@@ -447,7 +457,7 @@ __device__ __forceinline__ void pair_update(T* cpop, uint32_t cs,
     vel[3 * nb + 2] = uz.y;
   }
   if (PHASE == 0) {
-    const volatile uint32_t(*pk)[PHASE == 0 ? kC2Threads : 1] = parked;
+    const volatile uint32_t(*pk)[kC2Threads] = parked_addresses();
 #pragma unroll
     for (int e = 0; e < Q; ++e) {
       A[e] = pk[e][threadIdx.x];
