@@ -5,6 +5,7 @@
 // returned as mlbm_status with a message kept per host thread; nothing here
 // exits or falls back to the CPU.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 #include <type_traits>
 
 #include <cstdarg>
@@ -49,6 +50,21 @@ mlbm_status cuda_fail(cudaError_t e, const char* where) {
   if (e == cudaErrorMemoryAllocation)
     return fail(MLBM_ERR_NOMEM, "%s: %s", where, cudaGetErrorString(e));
   return fail(MLBM_ERR_CUDA, "%s: %s", where, cudaGetErrorString(e));
+}
+
+void prefault(void* p, size_t bytes) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  if (at.type != cudaMemoryTypeUnregistered) return;
+  const uintptr_t page = 4096, a = ((uintptr_t)p + page - 1) / page * page,
+                  b = ((uintptr_t)p + bytes) / page * page;
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+  if (b > a) (void)madvise((void*)a, b - a, MADV_POPULATE_WRITE);
 }
 
 size_t pop_elem_bytes(int storage) {
@@ -361,6 +377,9 @@ mlbm_status check_device_error(mlbm_lattice* lat) {
 
 mlbm_status ensure_staging(mlbm_lattice* lat, size_t bytes) {
   if (lat->staging_bytes >= bytes) return MLBM_OK;
+  // room for a scalar field at once: mask, density and result follow
+  const Geom& g = lat->g;
+  bytes = std::max(bytes, (size_t)g.lx * g.ly * g.lz * real_bytes(lat->storage));
   if (lat->staging) cudaFree(lat->staging);
   lat->staging = nullptr;
   lat->staging_bytes = 0;
@@ -444,22 +463,32 @@ mlbm_status mlbm_lattice_create(int32_t lx, int32_t ly, int32_t lz,
   lat->compact.two_pass_ok = compact_two_pass_supported(lx, ly, lz, storage);
   const size_t np = (size_t)lat->g.plane;
   const size_t mask_words = (size_t)lz * ly * lat->g.wpr;
-  cudaError_t e = cudaSuccess;
-  auto alloc = [&](void** p, size_t bytes) {
-    if (e == cudaSuccess) e = cudaMalloc(p, bytes);
-  };
-  alloc(&lat->pop, np * Q * pop_elem_bytes(storage));
-  alloc(&lat->rho, np * real_bytes(storage));
-  alloc(&lat->psi, (size_t)psi_elems(lat->g) * real_bytes(storage));
-  alloc((void**)&lat->rho_init, np * sizeof(float));
-  alloc((void**)&lat->mask, mask_words * sizeof(uint32_t));
-  alloc((void**)&lat->nbw, np * sizeof(uint32_t));
-  alloc((void**)&lat->err, sizeof(int));
-  if (e == cudaSuccess)
-    e = cudaMemset(lat->psi, 0, (size_t)psi_elems(lat->g) * real_bytes(storage));
-  if (e == cudaSuccess) e = cudaMemset(lat->err, 0, sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(lat->mask, 0, mask_words * 4);
-  if (e == cudaSuccess) e = cudaMemset(lat->rho_init, 0, np * sizeof(float));
+  // one allocation for all buffers (an allocation and its release cost about
+  // half a millisecond of host time, whatever its size); what starts as zeros
+  // lies together
+  auto up = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+  const size_t pop_bytes = up(np * Q * pop_elem_bytes(storage));
+  const size_t rho_bytes = up(np * real_bytes(storage));
+  const size_t nbw_bytes = up(np * sizeof(uint32_t));
+  const size_t psi_bytes = up((size_t)psi_elems(lat->g) * real_bytes(storage));
+  const size_t init_bytes = up(np * sizeof(float));
+  const size_t mask_bytes = up(mask_words * sizeof(uint32_t));
+  const size_t zeros = psi_bytes + init_bytes + mask_bytes + up(sizeof(int));
+  cudaError_t e =
+      cudaMalloc(&lat->buffer, pop_bytes + rho_bytes + nbw_bytes + zeros);
+  if (e == cudaSuccess) {
+    char* at = static_cast<char*>(lat->buffer);
+    lat->pop = at;
+    lat->rho = at += pop_bytes;
+    lat->nbw = reinterpret_cast<uint32_t*>(at += rho_bytes);
+    lat->psi = at += nbw_bytes;
+    lat->rho_init = reinterpret_cast<float*>(at + psi_bytes);
+    lat->mask = reinterpret_cast<uint32_t*>(at + psi_bytes + init_bytes);
+    lat->err = reinterpret_cast<int*>(at + psi_bytes + init_bytes + mask_bytes);
+    e = cudaMemset(at, 0, zeros);
+  } else {
+    lat->buffer = nullptr;
+  }
   if (e != cudaSuccess) {
     mlbm_lattice_destroy(lat);
     cudaGetLastError();
@@ -478,16 +507,10 @@ mlbm_status mlbm_lattice_destroy(mlbm_lattice* lat) {
   mlbm::DeviceGuard restore_device;
   cudaSetDevice(lat->device);
   if (lat->stream_owned_sync) cudaStreamSynchronize(lat->stream);
-  cudaFree(lat->pop);
-  cudaFree(lat->rho);
-  cudaFree(lat->psi);
-  cudaFree(lat->rho_init);
-  cudaFree(lat->mask);
+  cudaFree(lat->buffer);
   cudaFree(lat->vel);
-  cudaFree(lat->nbw);
   cudaFree(lat->staging);
   cudaFree(lat->stats_scratch);
-  cudaFree(lat->err);
   compact_free(lat);
   delete lat;
   return MLBM_OK;
@@ -659,6 +682,7 @@ mlbm_status mlbm_download_field(mlbm_lattice* lat, int32_t field,
   if (mlbm_status st = ensure_staging(lat, bytes)) return st;
   if (mlbm_status st = mlbm_download_field_device(lat, field, dtype, lat->staging))
     return st;
+  prefault(host_out, bytes);  // while the device works
   // cudaMemcpyDefault: host_out may be pageable, pinned or managed memory
   CUDA_TRY(cudaMemcpyAsync(host_out, lat->staging, bytes, cudaMemcpyDefault,
                            lat->stream),

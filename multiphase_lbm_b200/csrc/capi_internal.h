@@ -65,6 +65,7 @@ struct mlbm_lattice {
   cudaStream_t stream = nullptr;
   bool stream_owned_sync = true;
 
+  void* buffer = nullptr;       // one allocation for pop .. nbw and err
   void* pop = nullptr;          // 19 planes of g.plane elements (T)
   void* rho = nullptr;          // density, R per node
   void* psi = nullptr;          // pseudopotential, R per node

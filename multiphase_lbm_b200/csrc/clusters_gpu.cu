@@ -454,6 +454,9 @@ extern "C" mlbm_status mlbm_cluster_stats_gpu(
   k_unite<<<grid, 256>>>(d_cls, d, d_parent);
   k_flatten<<<grid, 256>>>(d_cls, d, d_parent, d_size);
   CL_TRY(cudaGetLastError(), "cluster_stats_gpu labelling");
+  // while the device labels: the pages that the labels go to
+  if (liq_labels_out) prefault(liq_labels_out, n * sizeof(int64_t));
+  if (gas_labels_out) prefault(gas_labels_out, n * sizeof(int64_t));
 
   if (solid_number)
     CL_TRY(cudaMemcpy(d_sn, solid_number, n * sizeof(int64_t), cudaMemcpyHostToDevice),

@@ -4,6 +4,8 @@
 
 #include <cuda_runtime.h>
 
+#include <cstddef>
+
 #include "../../include/mlbm.h"
 
 namespace mlbm {
@@ -24,6 +26,11 @@ struct DeviceGuard {
   DeviceGuard(const DeviceGuard&) = delete;
   DeviceGuard& operator=(const DeviceGuard&) = delete;
 };
+
+// Have the pages of an ordinary host buffer in place before a copy from the
+// device fills it (its contents stay): a copy into pages that are not takes
+// them one fault at a time with the device idle.
+void prefault(void* p, size_t bytes);
 
 // Record `msg` as the calling thread's last error and return `st`.
 mlbm_status set_error(mlbm_status st, const char* msg);
