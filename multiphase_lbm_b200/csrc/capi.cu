@@ -473,15 +473,17 @@ mlbm_status mlbm_lattice_create(int32_t lx, int32_t ly, int32_t lz,
   const size_t psi_bytes = up((size_t)psi_elems(lat->g) * real_bytes(storage));
   const size_t init_bytes = up(np * sizeof(float));
   const size_t mask_bytes = up(mask_words * sizeof(uint32_t));
+  const size_t words_bytes = up(2 * mask_words * sizeof(uint32_t));
   const size_t zeros = psi_bytes + init_bytes + mask_bytes + up(sizeof(int));
   cudaError_t e =
-      cudaMalloc(&lat->buffer, pop_bytes + rho_bytes + nbw_bytes + zeros);
+      cudaMalloc(&lat->buffer, pop_bytes + rho_bytes + nbw_bytes + words_bytes + zeros);
   if (e == cudaSuccess) {
     char* at = static_cast<char*>(lat->buffer);
     lat->pop = at;
     lat->rho = at += pop_bytes;
     lat->nbw = reinterpret_cast<uint32_t*>(at += rho_bytes);
-    lat->psi = at += nbw_bytes;
+    lat->stat_words = reinterpret_cast<uint32_t*>(at += nbw_bytes);
+    lat->psi = at += words_bytes;
     lat->rho_init = reinterpret_cast<float*>(at + psi_bytes);
     lat->mask = reinterpret_cast<uint32_t*>(at + psi_bytes + init_bytes);
     lat->err = reinterpret_cast<int*>(at + psi_bytes + init_bytes + mask_bytes);
@@ -697,7 +699,7 @@ namespace {
 
 // Enqueue the phase statistics reduction and the copy of its ST_COUNT + 1
 // doubles (the last one the device error flag) to host memory `h`; `full`
-// false: the bulk columns only (stat_node<R, false>).
+// false: the bulk columns only (k_stats_nodes<R, false>).
 mlbm_status stats_enqueue(mlbm_lattice* lat, double* h, bool full) {
   if (mlbm_status st = check_lat(lat)) return st;
   if (!h) return fail(MLBM_ERR_ARG, "null output");
@@ -708,42 +710,14 @@ mlbm_status stats_enqueue(mlbm_lattice* lat, double* h, bool full) {
                 "gather the slabs' own planes first");
   DeviceGuard restore_device;
   if (mlbm_status st = activate(lat)) return st;
-  // a lattice held in the fluid-only layout or as moments is walked through
-  // its node table (no lanes idle on solid nodes); otherwise the dense grid
-  const CompactState& c = lat->compact;
-  const uint2* nodes = lat->mom.active ? lat->mom.nodes
-                       : c.active      ? c.cinfo
-                                       : nullptr;
-  const long long nslots = lat->mom.active ? lat->mom.nnodes : c.nfluid;
-  const bool fluid_list = nodes != nullptr;
-  const dim3 grid(lat->g.px / 32, (lat->g.ly + 7) / 8,
-                  (lat->g.lz + kStatZ - 1) / kStatZ);
-  // The fluid-list form runs one wave of resident blocks over even spans of
-  // the node table (spans of whole 256-slot rounds; one block at least: the
-  // last block to finish writes the results).
-  long long nblocks = (long long)grid.x * grid.y * grid.z, span = 0;
-  if (fluid_list) {
-    // Both forms use the full form's wave: the spans, and with them the
-    // order of every sum, are then the same, so the bulk columns come out
-    // bit-identical.
-    if (lat->stats_wave <= 0) {
-      int per_sm = 0, nsm = 0;
-      CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                   &per_sm, k_stats_fluid<float, true>, kStatThreads, 0),
-               "stats occupancy");
-      CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount,
-                                      lat->device),
-               "stats occupancy");
-      lat->stats_wave = std::max(1, per_sm * nsm);
-    }
-    const long long rounds =
-        std::max(1LL, (nslots + kStatThreads - 1) / kStatThreads);
-    nblocks = std::min<long long>(lat->stats_wave, rounds);
-    span = (rounds + nblocks - 1) / nblocks * kStatThreads;
-    nblocks = std::max(1LL, (nslots + span - 1) / span);
-  }
-  // slot 0: the arrival counter; the block records; the results
-  const size_t need = (1 + (size_t)nblocks * ST_COUNT + ST_COUNT + 1) * sizeof(double);
+  // up to four blocks per SM: every record is folded again by one block
+  const int nwords = (int)((long long)lat->g.lz * lat->g.ly * lat->g.wpr);
+  constexpr int kPer = kStatThreads / 32 * kStatWords;
+  const unsigned nodes = (unsigned)std::min(592, (nwords + kPer - 1) / kPer);
+  const unsigned bound = (unsigned)((nwords + kStatThreads - 1) / kStatThreads);
+  // the counters; the block records; the results
+  const size_t records = (size_t)nodes * ST_COUNT;
+  const size_t need = (kStatCounters + records + ST_COUNT + 1) * sizeof(double);
   if (lat->stats_scratch_bytes < need) {
     // a larger area: earlier calls may still be reading the old one
     CUDA_TRY(cudaStreamSynchronize(lat->stream), "stats");
@@ -751,36 +725,31 @@ mlbm_status stats_enqueue(mlbm_lattice* lat, double* h, bool full) {
     lat->stats_scratch = nullptr;
     lat->stats_scratch_bytes = 0;
     CUDA_TRY(cudaMalloc((void**)&lat->stats_scratch, need), "stats scratch");
-    CUDA_TRY(cudaMemsetAsync(lat->stats_scratch, 0, sizeof(double), lat->stream),
+    CUDA_TRY(cudaMemsetAsync(lat->stats_scratch, 0, kStatCounters * sizeof(double),
+                             lat->stream),
              "stats counter");
     lat->stats_scratch_bytes = need;
   }
   StatScratch sc;
   sc.counter = reinterpret_cast<unsigned*>(lat->stats_scratch);
-  sc.records = lat->stats_scratch + 1;
-  sc.out = sc.records + (size_t)nblocks * ST_COUNT;
+  sc.boundary = reinterpret_cast<unsigned long long*>(lat->stats_scratch + 1);
+  sc.records = lat->stats_scratch + kStatCounters;
+  sc.out = sc.records + records;
   double* fin = sc.out;
-  if (fluid_list && lat->storage == MLBM_STORE_F64) {
-    auto kernel = full ? k_stats_fluid<double, true> : k_stats_fluid<double, false>;
-    kernel<<<(unsigned)nblocks, kStatThreads, 0, lat->stream>>>(
-        static_cast<const double*>(lat->rho), nodes, nslots, span, lat->g,
-        lat->phys, sc, lat->err);
-  } else if (fluid_list) {
-    auto kernel = full ? k_stats_fluid<float, true> : k_stats_fluid<float, false>;
-    kernel<<<(unsigned)nblocks, kStatThreads, 0, lat->stream>>>(
-        static_cast<const float*>(lat->rho), nodes, nslots, span, lat->g,
-        lat->phys, sc, lat->err);
-  } else if (lat->storage == MLBM_STORE_F64) {
-    auto kernel = full ? k_stats_partial<double, true> : k_stats_partial<double, false>;
-    kernel<<<grid, dim3(32, 8), 0, lat->stream>>>(
-        static_cast<const double*>(lat->rho), lat->nbw, lat->g, lat->phys, sc,
-        lat->err);
-  } else {
-    auto kernel = full ? k_stats_partial<float, true> : k_stats_partial<float, false>;
-    kernel<<<grid, dim3(32, 8), 0, lat->stream>>>(
-        static_cast<const float*>(lat->rho), lat->nbw, lat->g, lat->phys, sc,
-        lat->err);
-  }
+  uint32_t* liquid = lat->stat_words;
+  uint32_t* low = liquid + nwords;
+  auto launch = [&](auto real) {
+    using R = decltype(real);
+    auto kernel = full ? k_stats_nodes<R, true> : k_stats_nodes<R, false>;
+    kernel<<<nodes, kStatThreads, 0, lat->stream>>>(static_cast<const R*>(lat->rho),
+                                                    lat->mask, nwords, lat->phys, sc,
+                                                    liquid, low, lat->err);
+  };
+  if (lat->storage == MLBM_STORE_F64) launch(double());
+  else launch(float());
+  if (full)
+    k_stats_boundary<<<bound, kStatThreads, 0, lat->stream>>>(
+        lat->mask, liquid, low, nwords, lat->g, nodes, sc, lat->err);
   CUDA_TRY(cudaGetLastError(), "stats launch");
   CUDA_TRY(cudaMemcpyAsync(h, fin, (ST_COUNT + 1) * sizeof(double),
                            cudaMemcpyDeviceToHost, lat->stream),
@@ -871,11 +840,18 @@ mlbm_status mlbm_plane_profile(mlbm_lattice* lat, int64_t* n_fluid_x,
     k_plane_profile<float><<<profile_grid(lat->g), dim3(32, 8), 0, lat->stream>>>(
         static_cast<const float*>(lat->rho), lat->mask, lat->g, lat->phys, nf, nl);
   CUDA_TRY(cudaGetLastError(), "profile launch");
-  CUDA_TRY(cudaMemcpyAsync(n_fluid_x, nf, lx * 8, cudaMemcpyDeviceToHost,
-                           lat->stream), "profile copy");
-  CUDA_TRY(cudaMemcpyAsync(n_liquid_x, nl, lx * 8, cudaMemcpyDeviceToHost,
-                           lat->stream), "profile copy");
+  // one copy for both counts (two small pageable copies wait twice)
+  std::vector<int64_t> h;
+  try {
+    h.resize(2 * (size_t)lx);
+  } catch (const std::bad_alloc&) {
+    return fail(MLBM_ERR_NOMEM, "profile: host buffer");
+  }
+  CUDA_TRY(cudaMemcpyAsync(h.data(), nf, bytes, cudaMemcpyDeviceToHost, lat->stream),
+           "profile copy");
   CUDA_TRY(cudaStreamSynchronize(lat->stream), "profile");
+  std::memcpy(n_fluid_x, h.data(), bytes / 2);
+  std::memcpy(n_liquid_x, h.data() + lx, bytes / 2);
   return MLBM_OK;
 }
 

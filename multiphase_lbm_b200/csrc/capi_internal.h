@@ -46,8 +46,7 @@ struct MomentState {
   void* n = nullptr;        // [npairs] MomPair<R>: density, momentum
   uint2* words = nullptr;   // [npairs] node pairs: neighbour words,
   uint32_t* xyz = nullptr;  //          packed x, y, z
-  uint2* nodes = nullptr;   // [nnodes] fluid nodes (neighbour word, packed x, y, z)
-  int npairs = 0, nnodes = 0;
+  int npairs = 0;
   float shift = 0.f;        // rho_shift the state was produced under
 };
 
@@ -75,9 +74,9 @@ struct mlbm_lattice {
   float* vel = nullptr;         // [node][3], written on request
   void* staging = nullptr;      // reference-layout transfer buffer
   size_t staging_bytes = 0;
+  uint32_t* stat_words = nullptr;  // [2][mask words] bits of the statistics pass
   double* stats_scratch = nullptr;
   size_t stats_scratch_bytes = 0;
-  int stats_wave = 0;           // resident blocks of the statistics kernel
 
   // update pass: z-march tiles and the TMA descriptor of the psi tensor
   mlbm::ZMarch zm{};

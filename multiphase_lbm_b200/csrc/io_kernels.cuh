@@ -149,8 +149,7 @@ __global__ void k_pop_to_ref(const T* __restrict__ pop,
 enum { ST_NF, ST_NL, ST_NV, ST_NLS, ST_NLV, ST_MASS, ST_PL, ST_PV, ST_RL,
        ST_RV, ST_MINR, ST_MAXR, ST_MINP, ST_MAXP, ST_COUNT };
 
-constexpr int kStatThreads = 256;  // blockDim (32, 8)
-constexpr int kStatZ = 16;         // planes per block
+constexpr int kStatThreads = 256;
 
 __device__ __forceinline__ double stat_op(int k, double v, double o) {
   return (k == ST_MINR || k == ST_MINP) ? fmin(v, o)
@@ -163,59 +162,7 @@ __device__ __forceinline__ double stat_identity(int k) {
                                            : 0.0;
 }
 
-// The statistics of one fluid node folded into acc.  The liquid boundary
-// test reads the node's neighbour word (bit i: x - e_i is fluid) and the
-// density of every fluid neighbour, then takes the first neighbour
-// (i = 1..18) that is solid or not liquid, as calc_cluster does.  FULL =
-// false folds only the bulk columns (stat_bulk_column): no boundary test and
-// no pressure; those columns get the same operations in the same order
-// either way, so they come out bit-identical.
-template <typename R, bool FULL = true>
-__device__ __forceinline__ void stat_node(double (&acc)[ST_COUNT],
-                                          const R* __restrict__ rho,
-                                          const Geom& g, const Phys& p, int x,
-                                          int y, int z, uint32_t nb, R r) {
-  const R rhol = R(p.rhol_spinodal), rhog = R(p.rhog_spinodal);
-  const R pr = FULL ? pressure_of<R>(p, r) : R(0);
-  acc[ST_NF] += 1.0;
-  acc[ST_MASS] += (double)r;
-  if (r > rhol) {
-    acc[ST_NL] += 1.0;
-    if (FULL) acc[ST_PL] += (double)pr;
-    acc[ST_RL] += (double)r;
-    if (FULL) {
-      Nbr a;
-      a.init(g, x, y, z);
-      // all 18 neighbour densities as independent loads (every periodic
-      // index lies inside the array, solid nodes included), then the masks:
-      // a load under each direction's branch would wait on the one before
-      R nr[Q];
-#pragma unroll
-      for (int i = 1; i < Q; ++i) nr[i] = __ldg(rho + a.idx(-ex(i), -ey(i), -ez(i)));
-      const uint32_t solid = ~nb & 0x7fffeu;  // directions 1..18
-      uint32_t low = 0u;
-#pragma unroll
-      for (int i = 1; i < Q; ++i) low |= (nr[i] < rhol ? 1u : 0u) << i;
-      const uint32_t other = low & nb & 0x7fffeu;
-      const uint32_t first = (solid | other) & (0u - (solid | other));
-      if (first & solid) acc[ST_NLS] += 1.0;
-      else if (first) acc[ST_NLV] += 1.0;
-    }
-  } else if (r < rhog) {
-    acc[ST_NV] += 1.0;
-    if (FULL) acc[ST_PV] += (double)pr;
-    acc[ST_RV] += (double)r;
-  }
-  acc[ST_MINR] = fmin(acc[ST_MINR], (double)r);
-  acc[ST_MAXR] = fmax(acc[ST_MAXR], (double)r);
-  if (FULL) {
-    acc[ST_MINP] = fmin(acc[ST_MINP], (double)pr);
-    acc[ST_MAXP] = fmax(acc[ST_MAXP], (double)pr);
-  }
-}
-
-// The columns that the bulk statistics (FULL = false) compute; the others
-// are written as 0.
+// The columns that the bulk statistics compute; the others are written as 0.
 __host__ __device__ constexpr bool stat_bulk_column(int k) {
   return k == ST_NF || k == ST_NL || k == ST_NV || k == ST_MASS ||
          k == ST_RL || k == ST_RV || k == ST_MINR || k == ST_MAXR;
@@ -245,37 +192,40 @@ __device__ __forceinline__ void stat_block_reduce(double (&acc)[ST_COUNT],
   }
 }
 
-// Scratch of one statistics reduction (8-byte slots): slot 0 the arrival
-// counter (zero between calls), then the block records (ST_COUNT each),
-// then the ST_COUNT results and the device error flag.
+// Scratch of one statistics reduction (8-byte slots): the arrival counter and
+// the two boundary counts (zero between calls), then the block records
+// (ST_COUNT each), then the ST_COUNT results and the device error flag.
 struct StatScratch {
   unsigned* counter;
+  unsigned long long* boundary;  // liquid-solid, liquid-vapour
   double* records;
   double* out;
 };
+constexpr int kStatCounters = 3;
 
-// Called by every thread of a block once the block's record is written
-// (stat_block_reduce).  The last block to arrive folds all records -- in a
-// fixed order, so the result does not depend on which block is last: thread
-// t folds records t, t + 256, ... ascending, then the warps' shuffle trees,
-// then the warps in order -- writes the results and the device error flag
-// and re-arms the counter.  Records are read through L2 (ld.global.cg):
-// other SMs wrote them.  256 threads.
-__device__ __forceinline__ void stat_last_block(StatScratch s, unsigned nblocks,
+// Called by every thread of a block once the block's part is in the scratch.
+// The last of `arrivals` blocks to arrive folds the `nrecords` records (of this
+// launch or of the one before) -- in a fixed order, so the result does not
+// depend on which block is last: thread t folds records t, t + 256, ...
+// ascending, then the warps' shuffle trees, then the warps in order -- writes
+// the results and the device error flag and re-arms the counters.  Records are
+// read through L2 (ld.global.cg): other SMs wrote them.  256 threads.
+__device__ __forceinline__ void stat_last_block(StatScratch s, unsigned arrivals,
+                                                unsigned nrecords,
                                                 const int* __restrict__ err,
                                                 int tid, bool full) {
   __shared__ bool last;
   __shared__ double sh[kStatThreads / 32][ST_COUNT];
   __threadfence();
   __syncthreads();
-  if (tid == 0) last = atomicAdd(s.counter, 1u) == nblocks - 1;
+  if (tid == 0) last = atomicAdd(s.counter, 1u) == arrivals - 1;
   __syncthreads();
   if (!last) return;
   __threadfence();
   double v[ST_COUNT];
 #pragma unroll
   for (int k = 0; k < ST_COUNT; ++k) v[k] = stat_identity(k);
-  for (unsigned b = tid; b < nblocks; b += kStatThreads) {
+  for (unsigned b = tid; b < nrecords; b += kStatThreads) {
     const double* rec = s.records + (size_t)b * ST_COUNT;
     double r[ST_COUNT];
 #pragma unroll
@@ -294,6 +244,8 @@ __device__ __forceinline__ void stat_last_block(StatScratch s, unsigned nblocks,
   if (tid < ST_COUNT) {
     double r = sh[0][tid];
     for (int w = 1; w < kStatThreads / 32; ++w) r = stat_op(tid, r, sh[w][tid]);
+    if (full && (tid == ST_NLS || tid == ST_NLV))
+      r = (double)atomicExch(s.boundary + (tid - ST_NLS), 0ull);
     s.out[tid] = full || stat_bulk_column(tid) ? r : 0.0;  // not computed: 0
   }
   if (tid == 0) {
@@ -302,92 +254,159 @@ __device__ __forceinline__ void stat_last_block(StatScratch s, unsigned nblocks,
   }
 }
 
-// Dense form: one block per 32 x 8 nodes of an (x, y) plane and kStatZ
-// planes; each thread folds its column of nodes, z ascending.
-template <typename R, bool FULL = true>
-__global__ void __launch_bounds__(kStatThreads)
-    k_stats_partial(const R* __restrict__ rho, const uint32_t* __restrict__ nbw,
-                    Geom g, Phys p, StatScratch sc, const int* __restrict__ err) {
-  double acc[ST_COUNT];
-#pragma unroll
-  for (int k = 0; k < ST_COUNT; ++k) acc[k] = stat_identity(k);
-  const int x = blockIdx.x * 32 + threadIdx.x;
-  const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  const int z0 = blockIdx.z * kStatZ, z1 = min(z0 + kStatZ, g.lz);
-  if (x < g.lx && y < g.ly) {
-    // eight planes' node words and densities in flight at once (4: 1 %
-    // slower end to end; 8 planes per block with more blocks: 5 % slower)
-    constexpr int U = 8;
+// Sums, counts and extrema of the fluid nodes.  A warp takes kStatWords x 32
+// nodes at a time -- the padded rows make the nodes of consecutive mask words
+// consecutive densities -- with all their loads in flight: no node needs a
+// table entry first (walking the fluid nodes' table, two dependent loads a
+// node, took 35 us at 200^3, the 18 neighbours' densities of the boundary test
+// another 32; 31 and 23 us for both parts now).  What bounds it: instruction
+// issue, 71 per 32 nodes.
+// Counts are integers and extrema are in the densities' type; sums are FP64,
+// each lane over its nodes in order, then the fixed trees of
+// stat_block_reduce.  FULL: the pressures too, and for the boundary test the
+// words of the liquid nodes and of the fluid nodes below rhol; the fold is then
+// k_stats_boundary's.
+constexpr int kStatWords = 16;
+template <typename R, bool FULL>
+__global__ void __launch_bounds__(kStatThreads, sizeof(R) == 8 ? 2 : 4)
+    k_stats_nodes(const R* __restrict__ rho, const uint32_t* __restrict__ mask,
+                  int nwords, Phys p, StatScratch sc, uint32_t* __restrict__ liquid,
+                  uint32_t* __restrict__ low, const int* __restrict__ err) {
+  const int lane = threadIdx.x & 31;
+  const int warp = blockIdx.x * (kStatThreads / 32) + threadIdx.x / 32;
+  const int warps = gridDim.x * (kStatThreads / 32);
+  const R rhol = R(p.rhol_spinodal), rhog = R(p.rhog_spinodal);
+  unsigned nf = 0, nl = 0, nv = 0;
+  double mass = 0, pl = 0, pv = 0, rl = 0, rv = 0;
+  R minr = R(INFINITY), maxr = R(-INFINITY), minp = minr, maxp = maxr;
 #pragma unroll 1
-    for (int zb = z0; zb < z1; zb += U) {
-      uint32_t nbv[U];
-      R rv[U];
+  for (int c = warp; c <= (nwords - 1) / kStatWords; c += warps) {
+    const int w = c * kStatWords + lane;
+    const uint32_t m = lane < kStatWords && w < nwords ? __ldg(mask + w) : 0u;
+    const R* r0 = rho + (size_t)c * (kStatWords * 32) + lane;
+    R r[kStatWords];
+    uint32_t fl = 0;  // bit j: this lane's node of word j is fluid
 #pragma unroll
-      for (int j = 0; j < U; ++j) {
-        nbv[j] = 0u;
-        rv[j] = R(0);
-        if (zb + j < z1) {
-          const long long n = node_index(g, x, y, zb + j);
-          nbv[j] = __ldg(nbw + n);
-          rv[j] = __ldg(rho + n);
+    for (int j = 0; j < kStatWords; ++j) {
+      const uint32_t mj = __shfl_sync(~0u, m, j);
+      const uint32_t b = (mj >> lane) & 1u;
+      fl |= b << j;
+      r[j] = R(0);
+      if (b) r[j] = __ldg(r0 + j * 32);
+    }
+    uint32_t wl = 0, wb = 0;
+#pragma unroll
+    for (int j = 0; j < kStatWords; ++j) {
+      const R v = r[j];
+      const bool fluid = (fl >> j) & 1u, liq = fluid && v > rhol;
+      if (fluid) {
+        const R pr = FULL ? pressure_of<R>(p, v) : R(0);
+        mass += (double)v;
+        if (liq) {
+          ++nl;
+          rl += (double)v;
+          if (FULL) pl += (double)pr;
+        } else if (v < rhog) {
+          ++nv;
+          rv += (double)v;
+          if (FULL) pv += (double)pr;
+        }
+        minr = fmin(minr, v);
+        maxr = fmax(maxr, v);
+        if (FULL) {
+          minp = fmin(minp, pr);
+          maxp = fmax(maxp, pr);
         }
       }
-#pragma unroll
-      for (int j = 0; j < U; ++j)
-        if (nbv[j] & NB_SELF)
-          stat_node<R, FULL>(acc, rho, g, p, x, y, zb + j, nbv[j], rv[j]);
+      if (FULL) {
+        const uint32_t l = __ballot_sync(~0u, liq);
+        const uint32_t b = __ballot_sync(~0u, fluid && v < rhol);
+        if (lane == j) {
+          wl = l;
+          wb = b;
+        }
+      }
+    }
+    nf += __popc(fl);
+    if (FULL && lane < kStatWords && w < nwords) {
+      liquid[w] = wl;
+      low[w] = wb;
     }
   }
-  const long long blk =
-      blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
-  const int tid = threadIdx.y * 32 + threadIdx.x;
-  stat_block_reduce(acc, tid, sc.records + blk * ST_COUNT);
-  stat_last_block(sc, gridDim.x * gridDim.y * gridDim.z, err, tid, FULL);
-}
-
-// Fluid-list form, for a lattice held in the fluid-only layout: the threads
-// walk the compact node table (node word, packed x, y, z), so no lane idles
-// on a solid node.  The grid is one wave of resident blocks (the host sizes
-// it); block b folds slots [b * span, (b + 1) * span) and thread t takes
-// slots t, t + 256, ... of them, ascending -- a fixed assignment, so the
-// sums do not depend on scheduling.
-template <typename R, bool FULL = true>
-__global__ void __launch_bounds__(kStatThreads)
-    k_stats_fluid(const R* __restrict__ rho, const uint2* __restrict__ cinfo,
-                  long long nslots, long long span, Geom g, Phys p,
-                  StatScratch sc, const int* __restrict__ err) {
   double acc[ST_COUNT];
 #pragma unroll
   for (int k = 0; k < ST_COUNT; ++k) acc[k] = stat_identity(k);
-  const long long b0 = (long long)blockIdx.x * span;
-  const long long end = min(b0 + span, nslots);
-  constexpr int U = 8;
-#pragma unroll 1
-  for (long long k0 = b0 + threadIdx.x; k0 < end; k0 += (long long)U * kStatThreads) {
-    uint2 ci[U];
-    R rv[U];
-#pragma unroll
-    for (int j = 0; j < U; ++j) {
-      const long long k = k0 + (long long)j * kStatThreads;
-      ci[j] = k < end ? __ldg(cinfo + k) : make_uint2(0u, 0u);
-    }
-#pragma unroll
-    for (int j = 0; j < U; ++j) {
-      rv[j] = R(0);
-      if (ci[j].x & NB_SELF)
-        rv[j] = __ldg(rho + node_index(g, (int)(ci[j].y & 2047u),
-                                       (int)((ci[j].y >> 11) & 2047u),
-                                       (int)(ci[j].y >> 22)));
-    }
-#pragma unroll
-    for (int j = 0; j < U; ++j)
-      if (ci[j].x & NB_SELF)
-        stat_node<R, FULL>(acc, rho, g, p, (int)(ci[j].y & 2047u),
-                     (int)((ci[j].y >> 11) & 2047u), (int)(ci[j].y >> 22),
-                     ci[j].x, rv[j]);
+  acc[ST_NF] = nf;
+  acc[ST_NL] = nl;
+  acc[ST_NV] = nv;
+  acc[ST_MASS] = mass;
+  acc[ST_PL] = pl;
+  acc[ST_PV] = pv;
+  acc[ST_RL] = rl;
+  acc[ST_RV] = rv;
+  acc[ST_MINR] = fmin(acc[ST_MINR], (double)minr);
+  acc[ST_MAXR] = fmax(acc[ST_MAXR], (double)maxr);
+  if (FULL) {
+    acc[ST_MINP] = fmin(acc[ST_MINP], (double)minp);
+    acc[ST_MAXP] = fmax(acc[ST_MAXP], (double)maxp);
   }
   stat_block_reduce(acc, threadIdx.x, sc.records + (long long)blockIdx.x * ST_COUNT);
-  stat_last_block(sc, gridDim.x, err, threadIdx.x, FULL);
+  if (!FULL) stat_last_block(sc, gridDim.x, gridDim.x, err, threadIdx.x, false);
+}
+
+// 32 neighbours at x + dx of the nodes of word w of a row of bits (periodic).
+__device__ __forceinline__ uint32_t row_shift(const uint32_t* __restrict__ row, int w,
+                                              int dx, const Geom& g) {
+  const uint32_t v = row[w];
+  const int end = (g.lx - 1) & 31, last = g.wpr - 1;
+  if (dx < 0)
+    return (v << 1) | (w > 0 ? row[w - 1] >> 31 : (row[last] >> end) & 1u);
+  if (dx > 0)
+    return w < last ? (v >> 1) | (row[w + 1] << 31)
+                    : (v >> 1) | ((row[0] & 1u) << end);
+  return v;
+}
+
+// Liquid-solid and liquid-vapour boundary nodes, 32 at a time in bits: for a
+// liquid node the first neighbour x - e_i (i = 1..18) that is solid or below
+// rhol decides, as calc_cluster does.  After k_stats_nodes<R, true>, whose
+// records the last block folds.
+static __global__ void __launch_bounds__(kStatThreads)
+    k_stats_boundary(const uint32_t* __restrict__ mask,
+                     const uint32_t* __restrict__ liquid,
+                     const uint32_t* __restrict__ low, int nwords, Geom g,
+                     unsigned nrecords, StatScratch sc,
+                     const int* __restrict__ err) {
+  unsigned ls = 0, lv = 0;
+  for (int i = blockIdx.x * kStatThreads + threadIdx.x; i < nwords;
+       i += gridDim.x * kStatThreads) {
+    uint32_t open = liquid[i];  // liquid nodes no neighbour has decided yet
+    if (!open) continue;
+    const int w = i % g.wpr, r = i / g.wpr;
+    const int y = r % g.ly, z = r / g.ly;
+#pragma unroll
+    for (int k = 1; k < Q; ++k) {
+      const int q = (wrapc(z - ez(k), g.lz) * g.ly + wrapc(y - ey(k), g.ly)) * g.wpr;
+      const uint32_t solid = ~row_shift(mask + q, w, -ex(k), g);
+      const uint32_t below = row_shift(low + q, w, -ex(k), g);
+      ls += __popc(open & solid);
+      lv += __popc(open & ~solid & below);
+      open &= ~(solid | below);
+    }
+  }
+  ls = __reduce_add_sync(~0u, ls);
+  lv = __reduce_add_sync(~0u, lv);
+  __shared__ unsigned sum[2];
+  if (threadIdx.x < 2) sum[threadIdx.x] = 0u;
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) {
+    if (ls) atomicAdd(sum, ls);
+    if (lv) atomicAdd(sum + 1, lv);
+  }
+  __syncthreads();
+  if (threadIdx.x < 2 && sum[threadIdx.x])
+    atomicAdd(sc.boundary + threadIdx.x, (unsigned long long)sum[threadIdx.x]);
+  stat_last_block(sc, gridDim.x, nrecords, err, threadIdx.x, true);
 }
 
 // Per-x-plane fluid / liquid node counts (integers: deterministic).  A thread
@@ -395,7 +414,7 @@ __global__ void __launch_bounds__(kStatThreads)
 // columns up and adds one number per plane (two atomics per fluid node on lx
 // counters took 210 us at 200^3).  blockDim (32, 8), grid x tiles of
 // every row group.
-constexpr int kProfileRows = 64;
+constexpr int kProfileRows = 16;
 template <typename R>
 __global__ void k_plane_profile(const R* __restrict__ rho,
                                 const uint32_t* __restrict__ mask, Geom g,

@@ -13,21 +13,20 @@ namespace {
 
 size_t up256(size_t n) { return (n + 255) / 256 * 256; }
 
-// Pair list and node list of the current mask and slabs, and the
+// Pair list of the current mask and slabs, and the
 // buffers (one allocation).  Waits for the counts.
 mlbm_status build_list(mlbm_lattice* lat) {
   MomentState& s = lat->mom;
   const Geom& g = lat->g;
   const long long grid = TileGrid(g).count();
   size_t temp_bytes = 0;
-  TileCount* counts = nullptr;
-  cudaError_t e = cub::DeviceScan::ExclusiveScan(
-      nullptr, temp_bytes, counts, counts, TileCountSum(), TileCount{0, 0},
-      grid + 1, lat->stream);
+  uint32_t* counts = nullptr;
+  cudaError_t e = cub::DeviceScan::ExclusiveSum(
+      nullptr, temp_bytes, counts, counts, grid + 1, lat->stream);
   if (e != cudaSuccess) return cuda_fail(e, "moment lists");
   // scratch of the scan: the transfer buffer an upload has left (same
   // stream), else an allocation of its own
-  const size_t counts_bytes = up256((size_t)(grid + 1) * sizeof(TileCount));
+  const size_t counts_bytes = up256((size_t)(grid + 1) * sizeof(uint32_t));
   char* own = nullptr;
   char* buf = static_cast<char*>(lat->staging);
   if (lat->staging_bytes < counts_bytes + temp_bytes) {
@@ -35,14 +34,13 @@ mlbm_status build_list(mlbm_lattice* lat) {
     if (e != cudaSuccess) return cuda_fail(e, "moment lists");
     buf = own;
   }
-  counts = reinterpret_cast<TileCount*>(buf);
+  counts = reinterpret_cast<uint32_t*>(buf);
   const unsigned threads = 32 * kPairRows;
   k_mom_tiles<true><<<(unsigned)grid, threads, 0, lat->stream>>>(
-      lat->nbw, counts, nullptr, nullptr, nullptr, nullptr, g);
-  e = cub::DeviceScan::ExclusiveScan(buf + counts_bytes, temp_bytes, counts, counts,
-                                     TileCountSum(), TileCount{0, 0}, grid + 1,
-                                     lat->stream);
-  TileCount total{0, 0};
+      lat->nbw, counts, nullptr, nullptr, nullptr, g);
+  e = cub::DeviceScan::ExclusiveSum(buf + counts_bytes, temp_bytes, counts, counts,
+                                    grid + 1, lat->stream);
+  uint32_t total = 0;
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(&total, counts + grid, sizeof total,
                         cudaMemcpyDeviceToHost, lat->stream);
@@ -50,11 +48,10 @@ mlbm_status build_list(mlbm_lattice* lat) {
   const size_t real = real_bytes(lat->storage);
   const size_t m_bytes = up256((size_t)node_elems(g) * 4 * real);
   const size_t psi_bytes = up256((size_t)node_elems(g) * real);
-  const size_t n_bytes = up256((size_t)total.pairs * 8 * real);
-  const size_t words_bytes = up256((size_t)total.pairs * sizeof(uint2));
-  const size_t xyz_bytes = up256((size_t)total.pairs * sizeof(uint32_t));
-  const size_t need = m_bytes + psi_bytes + n_bytes + words_bytes + xyz_bytes +
-                      (size_t)total.nodes * sizeof(uint2);
+  const size_t n_bytes = up256((size_t)total * 8 * real);
+  const size_t words_bytes = up256((size_t)total * sizeof(uint2));
+  const size_t xyz_bytes = up256((size_t)total * sizeof(uint32_t));
+  const size_t need = m_bytes + psi_bytes + n_bytes + words_bytes + xyz_bytes;
   if (e == cudaSuccess && need > s.buffer_bytes) {
     cudaFree(s.buffer);
     s.buffer = nullptr;
@@ -70,12 +67,10 @@ mlbm_status build_list(mlbm_lattice* lat) {
     s.n = at += psi_bytes;
     s.words = reinterpret_cast<uint2*>(at += n_bytes);
     s.xyz = reinterpret_cast<uint32_t*>(at += words_bytes);
-    s.nodes = reinterpret_cast<uint2*>(at + xyz_bytes);
-    s.npairs = (int)total.pairs;
-    s.nnodes = (int)total.nodes;
-    if (total.pairs)
+    s.npairs = (int)total;
+    if (total)
       k_mom_tiles<false><<<(unsigned)grid, threads, 0, lat->stream>>>(
-          lat->nbw, nullptr, counts, s.words, s.xyz, s.nodes, g);
+          lat->nbw, nullptr, counts, s.words, s.xyz, g);
     e = cudaGetLastError();
   }
   cudaFree(own);

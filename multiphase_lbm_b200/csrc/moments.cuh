@@ -543,26 +543,14 @@ __device__ __forceinline__ uint32_t tile_word(const uint32_t* __restrict__ nbw,
 }
 
 // One block of kPairRows warps per tile (warp = row (y, z / 2), lane = x).
-// COUNT: counts[tile] = its pairs and nodes, for the host's scan.  Otherwise
-// the lists, at the places at[tile] that the scan gave.  nodes: the fluid
-// nodes one by one (neighbour word, packed coordinates), which the statistics
-// walk.
-struct TileCount {
-  uint32_t pairs, nodes;
-};
-struct TileCountSum {
-  __host__ __device__ TileCount operator()(const TileCount& a,
-                                           const TileCount& b) const {
-    return TileCount{a.pairs + b.pairs, a.nodes + b.nodes};
-  }
-};
-
+// COUNT: counts[tile] = its pairs, for the host's scan.  Otherwise the list, at
+// the places at[tile] that the scan gave.
 template <bool COUNT>
 __global__ void __launch_bounds__(32 * kPairRows)
-    k_mom_tiles(const uint32_t* __restrict__ nbw, TileCount* counts,
-                const TileCount* __restrict__ at, uint2* __restrict__ words,
-                uint32_t* __restrict__ xyz, uint2* __restrict__ nodes, Geom g) {
-  __shared__ uint32_t row_pairs[kPairRows], row_nodes[kPairRows];
+    k_mom_tiles(const uint32_t* __restrict__ nbw, uint32_t* counts,
+                const uint32_t* __restrict__ at, uint2* __restrict__ words,
+                uint32_t* __restrict__ xyz, Geom g) {
+  __shared__ uint32_t row_pairs[kPairRows];
   const TileGrid tg(g);
   const long long tile = blockIdx.x;
   const int lane = threadIdx.x & 31, row = threadIdx.x / 32;
@@ -572,36 +560,21 @@ __global__ void __launch_bounds__(32 * kPairRows)
   const uint32_t na = tile_word(nbw, g, x, y, z), nb = tile_word(nbw, g, x, y, z + 1);
   const bool any = (na | nb) != 0u;
   const uint32_t bp = __ballot_sync(~0u, any);
-  const uint32_t ba = __ballot_sync(~0u, na != 0u), bb = __ballot_sync(~0u, nb != 0u);
-  if (lane == 0) {
-    row_pairs[row] = __popc(bp);
-    row_nodes[row] = __popc(ba) + __popc(bb);
-  }
+  if (lane == 0) row_pairs[row] = __popc(bp);
   __syncthreads();
-  uint32_t pairs = 0, count = 0, pairs0 = 0, nodes0 = 0;
+  uint32_t pairs = 0, before = 0;
   for (int r = 0; r < kPairRows; ++r) {
-    if (r == row) {
-      pairs0 = pairs;
-      nodes0 = count;
-    }
+    if (r == row) before = pairs;
     pairs += row_pairs[r];
-    count += row_nodes[r];
   }
   if (COUNT) {
-    if (threadIdx.x == 0) counts[tile] = TileCount{pairs, count};
+    if (threadIdx.x == 0) counts[tile] = pairs;
     return;
   }
-  const TileCount w = at[tile];
-  const uint32_t below = (1u << lane) - 1u;
-  if (any) {
-    const uint32_t k = w.pairs + pairs0 + __popc(bp & below);
-    words[k] = make_uint2(na, nb);
-    xyz[k] = pack_xyz(x, y, z);
-  }
-  const uint32_t k = w.nodes + nodes0;
-  if (na) nodes[k + __popc(ba & below)] = make_uint2(na, pack_xyz(x, y, z));
-  if (nb)
-    nodes[k + __popc(ba) + __popc(bb & below)] = make_uint2(nb, pack_xyz(x, y, z + 1));
+  if (!any) return;
+  const uint32_t k = at[tile] + before + __popc(bp & ((1u << lane) - 1u));
+  words[k] = make_uint2(na, nb);
+  xyz[k] = pack_xyz(x, y, z);
 }
 
 }  // namespace mlbm

@@ -64,7 +64,7 @@ __device__ __forceinline__ double combine(int k, double a, double b) {
 
 // One block per x-plane of the reference layout [x][y][z]: the plane is the
 // contiguous run of ly*lz values starting at x*ly*lz.  Same statistics as
-// k_stats_partial (src/multiphase_lbm.cu:240-316, 1061-1072).
+// k_stats_nodes and k_stats_boundary (src/multiphase_lbm.cu:240-316, 1061-1072).
 __global__ void __launch_bounds__(kThreads)
     k_stats_plane_ref(const float* __restrict__ rho,
                       const uint8_t* __restrict__ fluid, int lx, int ly,
