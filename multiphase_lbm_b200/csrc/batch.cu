@@ -414,10 +414,11 @@ mlbm_status run_steps(mlbm_batch* b, int n, int reverse, unsigned inject) {
       done += kGraphSteps;
     }
   }
-  for (; done < n; ++done) {
-    launch_step_any(b, 0, reverse, inject, done == n - 1);
-    k_advance_step<<<1, 32, 0, b->stream>>>(b->d_step, 1);
-  }
+  // single steps count from the device counter, which moves on once
+  const int first = done;
+  for (; done < n; ++done)
+    launch_step_any(b, done - first, reverse, inject, done == n - 1);
+  if (done > first) k_advance_step<<<1, 32, 0, b->stream>>>(b->d_step, done - first);
   BCUDA(cudaGetLastError(), "batch launch");
   return MLBM_OK;
 }

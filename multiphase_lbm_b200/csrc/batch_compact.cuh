@@ -95,8 +95,8 @@ __global__ void __launch_bounds__(kBCThreads, 3)
                     unsigned inject_type) {
   static_assert(kBCThreads == kC2Threads, "pair_update's parked addresses");
   const long long s = *step + delta;
-  const long long b = blockIdx.x;
-  if (b >= upre[n]) return;
+  const long long b = upre[n] - 1 - blockIdx.x;  // reverse order (k_cupdate)
+  if (b < 0) return;
   const int d = find_domain(upre, n, b);
   const CDomain& D = doms[d];
   const int ph = D.phase_base ^ (int)(s & 1);

@@ -140,14 +140,19 @@ __global__ void __launch_bounds__(kC2Threads, 5)
                                         rho_out, psi, g, p, a, inj);
 }
 
+// The update's blocks run from the end of the lattice to its start: the density
+// pass before it has left the populations it read last in L2, and the next
+// step's density pass starts where the update ends (tau = 0.9, us per step:
+// 128^3 53.5 -> 48.9, 160^3 108 -> 101.6, 200^3 206 -> 198, FP16 176 -> 170).
 template <typename T, int PHASE, bool WRITE_U, bool EQ>
 __global__ void __launch_bounds__(kC2Threads, 3)
     k_cupdate(T* __restrict__ cpop, uint32_t cs, const uint2* __restrict__ cinfo,
               const uint2* __restrict__ wtab, int kbeg, int nfluid,
               const float* __restrict__ psi, float* __restrict__ vel, Geom g,
               Phys p, StepArgs a, bool inj) {
-  const long long k = kbeg + c2_update_nodes_per_thread() *
-                                 ((long long)blockIdx.x * kC2Threads + threadIdx.x);
+  const long long block = gridDim.x - 1 - blockIdx.x;
+  const long long k =
+      kbeg + c2_update_nodes_per_thread() * (block * kC2Threads + threadIdx.x);
   if (k >= nfluid) return;
   pair_update<T, PHASE, WRITE_U, EQ, PsiPlain, true>(cpop, cs, cinfo, wtab, (int)k,
                                                  nfluid, PsiPlain{psi}, vel, g,
