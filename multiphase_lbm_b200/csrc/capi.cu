@@ -487,7 +487,10 @@ mlbm_status mlbm_lattice_create(int32_t lx, int32_t ly, int32_t lz,
     lat->rho_init = reinterpret_cast<float*>(at + psi_bytes);
     lat->mask = reinterpret_cast<uint32_t*>(at + psi_bytes + init_bytes);
     lat->err = reinterpret_cast<int*>(at + psi_bytes + init_bytes + mask_bytes);
+    // waited for: the lattice's own work may go to a stream that the legacy
+    // stream's does not order itself with
     e = cudaMemset(at, 0, zeros);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
   } else {
     lat->buffer = nullptr;
   }
