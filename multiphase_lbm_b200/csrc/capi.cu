@@ -568,7 +568,7 @@ static mlbm_status upload_rho_impl(mlbm_lattice* lat, const float* src,
   CUDA_TRY(cudaMemcpyAsync(lat->staging, src, n * sizeof(float), kind,
                            lat->stream),
            "rho upload copy");
-  k_rho_from_ref<<<tile_grid(g), tile_block(), 0, lat->stream>>>(
+  k_rho_from_ref<<<span_grid(g), tile_block(), 0, lat->stream>>>(
       static_cast<const float*>(lat->staging), lat->rho_init, g);
   CUDA_TRY(cudaGetLastError(), "rho transpose launch");
   CUDA_TRY(cudaStreamSynchronize(lat->stream), "rho upload");

@@ -26,7 +26,18 @@ __device__ __forceinline__ long long ref_index(const Geom& g, int x, int y,
 // across touched a sector per 4 bytes on one side: 56 us for the 64 MB of a
 // 200^3 FP32 field).  blockDim (32, kTileRows), grid (x tiles of every y, z
 // tiles): y has no place among the grid's short dimensions (up to 2^24 rows).
+// The density coming in moves 32 x kSpanZ tiles, runs of 512 bytes read (384^3:
+// 250 -> 177 us a call); on the way out the wider tile gains at 200^3 (23 -> 21
+// us) and loses at 384^3 (181 -> 189) and 64^3.
 constexpr int kTileRows = 8;
+constexpr int kSpanZ = 128;
+#define MLBM_SPAN_COORDS                                             \
+  const int xt = (int)(blockIdx.x % (unsigned)g.wpr), x0 = xt * 32;  \
+  const int y = (int)(blockIdx.x / (unsigned)g.wpr);                 \
+  const int z0 = blockIdx.y * kSpanZ, lane = threadIdx.x;
+inline dim3 span_grid(const Geom& g) {
+  return dim3((unsigned)g.wpr * (unsigned)g.ly, (g.lz + kSpanZ - 1) / kSpanZ, 1);
+}
 #define MLBM_TILE_COORDS                                             \
   const int xt = (int)(blockIdx.x % (unsigned)g.wpr), x0 = xt * 32;  \
   const int y = (int)(blockIdx.x / (unsigned)g.wpr);                 \
@@ -55,15 +66,19 @@ __global__ void k_pack_mask(const uint8_t* __restrict__ fluid_ref,
 
 __global__ void k_rho_from_ref(const float* __restrict__ rho_ref,
                                float* __restrict__ rho_int, Geom g) {
-  __shared__ float t[32][33];
-  MLBM_TILE_COORDS
+  __shared__ float t[32][kSpanZ + 1];
+  MLBM_SPAN_COORDS
+#pragma unroll
   for (int r = threadIdx.y; r < 32; r += kTileRows) {
-    const int x = x0 + r, z = z0 + lane;
-    if (x < g.lx && z < g.lz) t[r][lane] = rho_ref[ref_index(g, x, y, z)];
+#pragma unroll
+    for (int c = 0; c < kSpanZ; c += 32) {
+      const int x = x0 + r, z = z0 + c + lane;
+      if (x < g.lx && z < g.lz) t[r][c + lane] = rho_ref[ref_index(g, x, y, z)];
+    }
   }
   __syncthreads();
   if (x0 + lane >= g.lx) return;
-  for (int r = threadIdx.y; r < 32 && z0 + r < g.lz; r += kTileRows)
+  for (int r = threadIdx.y; r < kSpanZ && z0 + r < g.lz; r += kTileRows)
     rho_int[node_index(g, x0 + lane, y, z0 + r)] = t[lane][r];
 }
 

@@ -189,9 +189,9 @@ __device__ __forceinline__ double expr(double v) { return exp(v); }
 template <typename R>
 __device__ __forceinline__ R pressure_of(const Phys& p, R rho) {
   if (p.carn_star) {
-    const R a = R(1.0), b = R(4.0), Rg = R(1.0), Tc = R(0.0943);
+    const R a = R(1.0), Rg = R(1.0), Tc = R(0.0943);
     const R T = rmul(R(p.T_Tc), Tc);
-    const R eta = rdiv(rmul(b, rho), R(4.0));
+    const R eta = rho;  // b rho / 4 with b = 4: exact
     const R eta2 = rmul(eta, eta), eta3 = rmul(eta2, eta), rho2 = rmul(rho, rho);
     const R ome = rsub(R(1.0), eta);
     const R ome3 = rmul(rmul(ome, ome), ome);
