@@ -49,6 +49,8 @@
 #include "kernels.cuh"
 #include "lattice.cuh"
 
+#include <type_traits>
+
 namespace mlbm {
 
 constexpr int kTileX = 32, kTileY = 8, kTileZ = 4;  // order of the pair list
@@ -171,20 +173,29 @@ struct Source {
   }
 };
 
+// e_i . u, added as collide() adds it (the opposite direction's is its negative).
+template <typename R>
+__device__ __forceinline__ R e_dot_u(int i, const Mom<R>& m) {
+  R eu = R(0);
+  if (ex(i)) eu = ex(i) > 0 ? m.x : -m.x;
+  if (ey(i)) eu = ex(i) ? (ey(i) > 0 ? radd(eu, m.y) : rsub(eu, m.y))
+                        : (ey(i) > 0 ? m.y : -m.y);
+  if (ez(i)) eu = ex(i) || ey(i) ? (ez(i) > 0 ? radd(eu, m.z) : rsub(eu, m.z))
+                                 : (ez(i) > 0 ? m.z : -m.z);
+  return eu;
+}
+__host__ __device__ constexpr bool is_axis(int i) {
+  return ex(i) * ex(i) + ey(i) * ey(i) + ez(i) * ez(i) == 1;
+}
+
 // feq_i of collide(), operation for operation.
 template <typename T>
 __device__ __forceinline__ typename Pop<T>::Real eq_population(int i,
                                                                const Source<T>& s) {
   using R = typename Pop<T>::Real;
   if (i == 0) return rmul(rmul(weight<R>(0), s.m.d), s.base);
-  R eu = R(0);
-  if (ex(i)) eu = ex(i) > 0 ? s.m.x : -s.m.x;
-  if (ey(i)) eu = ex(i) ? (ey(i) > 0 ? radd(eu, s.m.y) : rsub(eu, s.m.y))
-                        : (ey(i) > 0 ? s.m.y : -s.m.y);
-  if (ez(i)) eu = ex(i) || ey(i) ? (ez(i) > 0 ? radd(eu, s.m.z) : rsub(eu, s.m.z))
-                                 : (ez(i) > 0 ? s.m.z : -s.m.z);
-  const bool axis = ex(i) * ex(i) + ey(i) * ey(i) + ez(i) * ez(i) == 1;
-  return rmul(axis ? s.wd1 : s.wd2, Equilibrium<T>::term(s.base, eu));
+  return rmul(is_axis(i) ? s.wd1 : s.wd2,
+              Equilibrium<T>::term(s.base, e_dot_u<R>(i, s.m)));
 }
 
 // Both nodes' population as the storage format T holds it: stored with shift
@@ -298,17 +309,31 @@ struct Gather {
   MomPair<R> own;
   PairSums<T> sum;
 
+  // f_i of one node from source s, or from itself (o, the opposite direction)
+  // where that is solid.  FP32 and FP64 form both and take one; FP16, whose
+  // equilibrium is two operations longer, takes one of the operands first
+  // (200^3: 113 us a step against 117; FP32 116 against 109).
+  static __device__ __forceinline__ R one(int i, bool fluid, const Source<T>& s,
+                                          const Source<T>& o) {
+    if constexpr (std::is_same<T, __half>::value) {
+      const R es = e_dot_u<R>(i, s.m), eo = e_dot_u<R>(i, o.m);
+      const R ws = is_axis(i) ? s.wd1 : s.wd2, wo = is_axis(i) ? o.wd1 : o.wd2;
+      return rmul(fluid ? ws : wo,
+                  Equilibrium<T>::term(fluid ? s.base : o.base, fluid ? es : -eo));
+    } else {
+      const R fs = eq_population<T>(i, s), fo = eq_population<T>(opp(i), o);
+      return fluid ? fs : fo;
+    }
+  }
   // f_i of both nodes from the sources sa, sb
   __device__ __forceinline__ Two<R> population(int i, const Source<T>& sa,
                                                const Source<T>& sb) {
-    Two<R> f{eq_population<T>(i, sa), eq_population<T>(i, sb)};
-    if (i) {
-      const int o = opp(i);
-      const R oa = eq_population<T>(o, Source<T>(own.a)),
-              ob = eq_population<T>(o, Source<T>(own.b));
-      f.a = (na >> i) & 1u ? f.a : oa;
-      f.b = (nb >> i) & 1u ? f.b : ob;
-    }
+    Two<R> f;
+    if (i == 0)
+      f = Two<R>{eq_population<T>(i, sa), eq_population<T>(i, sb)};
+    else
+      f = Two<R>{one(i, (na >> i) & 1u, sa, Source<T>(own.a)),
+                 one(i, (nb >> i) & 1u, sb, Source<T>(own.b))};
     return Stored<T>::pass(f, st * weight<float>(i), ld * weight<float>(i));
   }
   // the three populations from the column (dx, dy): levels z - 1 .. z + 2
@@ -360,9 +385,10 @@ struct Gather {
 
 // Resident blocks the registers are held to.  FP32: 72 registers ran a 200^3
 // step in 109 us and a 96^3 one in 14.9, 64 registers (8 blocks) in 112 and
-// 15.4, 80 (6) in 111 and 15.2, 51 (10) in 121 and 17.9.
+// 15.4, 80 (6) in 111 and 15.2, 51 (10) in 121 and 17.9.  FP16: 64 registers 113
+// at 200^3, 72 115.
 template <typename T>
-constexpr int mom_gather_blocks() { return sizeof(typename Pop<T>::Real) == 8 ? 4 : 7; }
+constexpr int mom_gather_blocks() { return sizeof(typename Pop<T>::Real) == 8 ? 4 : sizeof(T) == 2 ? 8 : 7; }
 
 // Gather pass of pair k of a list.  A thread past its end passes the gate with
 // the others (a branch around the gate cost 4 % of the step).
