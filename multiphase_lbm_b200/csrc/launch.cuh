@@ -29,7 +29,6 @@ void launch_overlapped(bool overlap, void (*kernel)(KArgs...), unsigned grid,
 }
 
 // Launches into a stream that is being captured into a CUDA graph are plain:
-// the batched step's graphs with overlapped launches gave wrong states, so
 // the overlap is used in ordinary stream order only.
 inline bool stream_capturing(cudaStream_t stream) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;

@@ -190,8 +190,20 @@ mlbm_status moments_sync_dense(mlbm_lattice* lat) {
 }
 
 mlbm_status moments_leave(mlbm_lattice* lat) {
+  if (!lat->mom.active) return MLBM_OK;
   if (mlbm_status st = moments_sync_dense(lat)) return st;
   lat->mom.active = false;
+  if (lat->mom.npairs == 0) return MLBM_OK;
+  const Geom& g = lat->g;
+  const dim3 grid((g.lx + 31) / 32, (g.ly + 7) / 8, g.lz), block(32, 8);
+  if (lat->storage == MLBM_STORE_F64)
+    k_mom_psi_back<double><<<grid, block, 0, lat->stream>>>(
+        static_cast<const double*>(lat->mom.psi), static_cast<double*>(lat->psi), g);
+  else
+    k_mom_psi_back<float><<<grid, block, 0, lat->stream>>>(
+        static_cast<const float*>(lat->mom.psi), static_cast<float*>(lat->psi), g);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail(e, "psi of the moments");
   return MLBM_OK;
 }
 

@@ -31,14 +31,19 @@
 // ordered by tiles of 32 x kTileY x kTileZ nodes and by rows within, so that a
 // block's loads share lines in all three directions.
 //
-// What bounds it: the cache lines a warp's loads touch.  A warp of the list
-// spans 2-3 runs of fluid along x, so a 16-byte load of its lanes touches 6
-// lines where a full row would touch 4.  Tried, at 200^3 FP32 (us per step,
-// 110 as it is): the two nodes of a pair side by side with 32-byte loads
-// 117 (19 requests in place of 28, but 9.7 lines each); pairs whose neighbours
-// are all fluid listed first in each tile, to skip their bounce-back selects,
-// 119 (the runs break up: 7.9 lines); tiles staged in shared memory with
-// packed FP32 arithmetic 190 (bank conflicts take the place of the lines).
+// What bounds it: the gather (two thirds of a step) instruction issue and L1
+// together -- about 750 instructions per warp of pairs, and the cache lines its
+// loads touch: a warp of the list spans 2-3 runs of fluid along x, so a 16-byte
+// load of its lanes touches 6 lines where a full row would touch 4 --, the
+// collide the latency of its loads.  At 200^3 FP32 the population kernels take
+// 206 us a step, this step 109.  Tried there: one node per thread 155; the two
+// nodes of a pair side by side with 32-byte loads 117 (19 requests in place of
+// 28, but 9.7 lines each); pairs whose neighbours are all fluid listed first in
+// each tile, to skip their bounce-back selects, 119 (the runs break up: 7.9
+// lines); tiles staged in shared memory with packed FP32 arithmetic 190 (bank
+// conflicts take the place of the lines); packed sums or own populations in
+// registers 112-127; gather and collide blocks side by side in one launch
+// 140-154; other tile shapes and block-to-SM orders, no gain.
 //
 // FP16 storage keeps its meaning: a population read by the gather is rounded
 // to half(f* - t_i rho_shift) exactly as the population kernels store it.
@@ -564,7 +569,7 @@ __global__ void __launch_bounds__(kMomThreads)
   }
 }
 
-// psi of every node into the paired layout, the images in z included (the
+// psi of every node into this step's layout, the images in z included (the
 // solid nodes' psi(rhos), which only initialisation writes).
 template <typename R>
 __global__ void k_mom_psi(const R* __restrict__ psi, R* __restrict__ out, Geom g) {
@@ -573,6 +578,16 @@ __global__ void k_mom_psi(const R* __restrict__ psi, R* __restrict__ out, Geom g
   const int z = (int)blockIdx.z - 1;
   if (x >= g.lx || y >= g.ly) return;
   out[node_element(g, x, y, z)] = psi[psi_index(g, x, y, z)];
+}
+
+// And back, ghost copies included: what the population kernels' passes find.
+template <typename R>
+__global__ void k_mom_psi_back(const R* __restrict__ psi, R* __restrict__ out, Geom g) {
+  const int x = blockIdx.x * 32 + threadIdx.x;
+  const int y = blockIdx.y * blockDim.y + threadIdx.y;
+  const int z = (int)blockIdx.z;
+  if (x >= g.lx || y >= g.ly) return;
+  store_psi<R>(out, g, x, y, z, psi[node_element(g, x, y, z)]);
 }
 
 // ---- tiles and lists -----------------------------------------------------------
