@@ -103,7 +103,7 @@ __device__ __forceinline__ void batch_update_node(const DomainDesc& d,
     const long long sy = g.pxg, sz = (long long)(g.ly + 2) * g.pxg;
     R ux, uy, uz;
     collide<T, R>(
-        d.p, dd, __ldg(ps),
+        d.p.omega == 1.f, d.p, dd, __ldg(ps),
         [&](int i) { return __ldg(ps + ex(i) + ey(i) * sy + ez(i) * sz); }, f,
         ux, uy, uz);
   }

@@ -5,13 +5,12 @@
 // same domain advanced alone.
 //
 // Each domain owns a contiguous range of blocks.  The AA phase of a domain
-// at batch step s is phase_base ^ (s & 1).  The density pass runs one node
-// per thread in the gather step and one pair per thread in the local step,
-// so a domain's block count depends on the parity of s: two block-prefix
-// tables, one per parity, and the launch grid covers the larger total.  The
-// update pass runs one pair per thread in both phases (one table).  The
-// batch step s is read from the device counter (graph replays advance it),
-// so a captured graph stays valid for every start parity.
+// at batch step s is phase_base ^ (s & 1).  Both passes run one node per
+// thread in the gather step and one pair per thread in the local step, so a
+// domain's block count depends on the parity of s: two block-prefix tables,
+// one per parity, and the launch grid covers the larger total.  The batch step
+// s is read from the device counter (graph replays advance it), so a captured
+// graph stays valid for every start parity.
 #pragma once
 
 #include "batch.cuh"
@@ -22,7 +21,7 @@
 
 namespace mlbm {
 
-constexpr int kBCThreads = 256;
+constexpr int kBCThreads = kC2Threads;
 
 struct CDomain {
   Geom g;
@@ -38,15 +37,16 @@ struct CDomain {
   long long step_origin;
 };
 
-// Domain, local block and AA phase of this block at batch step s; false if
-// the block has no work at this parity.
+// Domain and local block of this block at batch step s, in reverse order (as
+// k_cupdate's) or not; false if the block has no work at this parity.
+template <bool REVERSE>
 __device__ __forceinline__ bool bc_locate(const long long* __restrict__ pre,
                                           int n, long long s, int& d,
                                           long long& local) {
   const int par = (int)(s & 1);
   const long long* pp = pre + (size_t)par * (n + 1);
-  const long long b = blockIdx.x;
-  if (b >= pp[n]) return false;
+  const long long b = REVERSE ? pp[n] - 1 - blockIdx.x : blockIdx.x;
+  if (REVERSE ? b < 0 : b >= pp[n]) return false;
   d = find_domain(pp, n, b);
   local = b - pp[d];
   return true;
@@ -57,8 +57,12 @@ __device__ __forceinline__ bool bc_inject(const Phys& p, long long dstep) {
          (unsigned long long)dstep % p.rho_inject_period == 0ull;
 }
 
+// Blocks per SM, (density, update): 24 domains of edges 32-128 at tau 0.9, us per
+// step FP32 / FP16: (10, 8) 302 / 270; (8, 7) 312 / 284, (10, 7) 309 / 274, (6, 8)
+// 304 / 276, (12, 8) 311 / 279, (10, 10) 332 / 294; updates by pairs in both
+// phases, blocks of 256, 321 / 291.
 template <typename T, bool WRITE_RHO>
-__global__ void __launch_bounds__(kBCThreads, 3)
+__global__ void __launch_bounds__(kBCThreads, 10)
     k_batch_cdensity(const CDomain* __restrict__ doms,
                      const long long* __restrict__ pre, int n,
                      const long long* __restrict__ step, int delta, int reverse,
@@ -66,7 +70,7 @@ __global__ void __launch_bounds__(kBCThreads, 3)
   const long long s = *step + delta;
   int d;
   long long local;
-  if (!bc_locate(pre, n, s, d, local)) return;
+  if (!bc_locate<false>(pre, n, s, d, local)) return;
   const CDomain& D = doms[d];
   const int ph = D.phase_base ^ (int)(s & 1);
   StepArgs a{s - D.step_origin, reverse, inject_type};
@@ -78,45 +82,40 @@ __global__ void __launch_bounds__(kBCThreads, 3)
                                 D.wtab, (int)t, D.rho, D.psi, D.g, D.p, a, inj);
   } else {
     if (2 * t >= D.nfluid) return;
-    pair_density<T, 1, WRITE_RHO>(static_cast<const T*>(D.cpop), D.cs, D.cinfo,
-                                  D.wtab, (int)(2 * t), D.nfluid, D.rho, D.psi,
-                                  D.g, D.p, a, inj);
+    pair_density<T, WRITE_RHO>(static_cast<const T*>(D.cpop), D.cs, D.cinfo,
+                               (int)(2 * t), D.nfluid, D.rho, D.psi, D.g, D.p, a,
+                               inj);
   }
 }
 
-// upre: the update pass's block prefixes (n + 1 entries, both parities).
-// Blocks of kBCThreads = kC2Threads threads, as pair_update's phase-0 form
-// requires.
 template <typename T>
-__global__ void __launch_bounds__(kBCThreads, 3)
+__global__ void __launch_bounds__(kBCThreads, 8)
     k_batch_cupdate(const CDomain* __restrict__ doms,
-                    const long long* __restrict__ upre, int n,
+                    const long long* __restrict__ pre, int n,
                     const long long* __restrict__ step, int delta, int reverse,
                     unsigned inject_type) {
-  static_assert(kBCThreads == kC2Threads, "pair_update's parked addresses");
   const long long s = *step + delta;
-  const long long b = upre[n] - 1 - blockIdx.x;  // reverse order (k_cupdate)
-  if (b < 0) return;
-  const int d = find_domain(upre, n, b);
+  int d;
+  long long local;
+  if (!bc_locate<true>(pre, n, s, d, local)) return;
   const CDomain& D = doms[d];
   const int ph = D.phase_base ^ (int)(s & 1);
   StepArgs a{s - D.step_origin, reverse, inject_type};
   const bool inj = bc_inject(D.p, a.step);
-  const long long k = 2 * ((b - upre[d]) * kBCThreads + threadIdx.x);
-  if (k >= D.nfluid) return;
-  auto update = [&](auto phase, auto eq) {
-    pair_update<T, decltype(phase)::value, false, decltype(eq)::value>(
-        static_cast<T*>(D.cpop), D.cs, D.cinfo, D.wtab, (int)k, D.nfluid,
-        PsiPlain{D.psi}, nullptr, D.g, D.p, a, inj);
+  const long long t = local * kBCThreads + threadIdx.x;
+  if ((ph == 0 ? t : 2 * t) >= D.nfluid) return;
+  auto update = [&](auto eq) {
+    if (ph == 0)
+      node_update0<T, false, decltype(eq)::value>(
+          static_cast<T*>(D.cpop), D.cs, D.cinfo, D.wtab, (int)t, D.psi, nullptr,
+          D.g, D.p, a, inj);
+    else
+      pair_update<T, false, decltype(eq)::value>(
+          static_cast<T*>(D.cpop), D.cs, D.cinfo, (int)(2 * t), D.nfluid, D.psi,
+          nullptr, D.g, D.p, a, inj);
   };
-  using std::integral_constant;
-  if (D.p.omega == 1.f) {  // a batch with other taus beside
-    if (ph == 0) update(integral_constant<int, 0>(), std::true_type());
-    else update(integral_constant<int, 1>(), std::true_type());
-  } else {
-    if (ph == 0) update(integral_constant<int, 0>(), std::false_type());
-    else update(integral_constant<int, 1>(), std::false_type());
-  }
+  if (D.p.omega == 1.f) update(std::true_type());  // a batch with other taus beside
+  else update(std::false_type());
 }
 
 }  // namespace mlbm

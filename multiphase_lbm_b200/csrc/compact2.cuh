@@ -25,7 +25,7 @@
 
 namespace mlbm {
 
-constexpr int kC2Threads = 256;
+constexpr int kC2Threads = 128;
 
 __host__ __device__ constexpr uint32_t pack_xyz(int x, int y, int z) {
   return (uint32_t)x | ((uint32_t)y << 11) | ((uint32_t)z << 22);
@@ -106,25 +106,34 @@ static __global__ void k_wtab(const uint32_t* __restrict__ mask,
 
 namespace mlbm {
 
-// The update pass runs one thread per pair of fluid nodes (pair.cuh, k = 2 *
-// thread index) in both AA phases; the gather/push form (phase 0) keeps its
-// addresses in shared memory across the collision.  The density pass runs
-// pairs in the local phase and one node per thread in the gather phase
-// (pairs there measured 1 % slower at 64 and at 80 registers).
-// The density pass is held to 48 registers (5 CTAs per SM); on the 200^3
-// bench that beat 3, 4 and 6 CTAs per SM.  Both kernels advance the compact
-// indices [kbeg, nfluid): the whole lattice, or the own planes of a slab
+// Both passes run one node per thread in the gather/push phase (0) and one
+// thread per pair (k = 2 * thread index) in the local phase (pair.cuh), over the
+// compact indices [kbeg, nfluid): the whole lattice, or the own planes of a slab
 // lattice (kbeg is a plane start, so it is even).
-// EQ: omega is 1 (collide2).
+// EQ: omega is 1 (collide).
+//
+// What bounds them: memory latency at the occupancy their registers allow (the
+// local density pass: DRAM, 6.4 TB/s).  The update in the gather/push phase ran
+// pairs with 2 x 19 parked addresses in blocks of 256, 3 per SM: 24 warps; one
+// node per thread at 48 registers gives 40, the local phase at 72 registers and
+// blocks of 128 gives 28.  us per step at tau 0.9, average of the two phases,
+// pairs in blocks of 256 -> as it is: 128^3 48.9 -> 44.3, 160^3 101.3 -> 94.3,
+// 200^3 198.4 -> 187.1, 256^3 411 -> 389, FP16 200^3 171 -> 157, 128^3 43.6 ->
+// 39.9; 64^3, where launches count, 9.5 either way.  On the way there, at 200^3:
+// pairs (k, k + 32), coalesced, 196.6; with blocks of 128 192.9; one node per
+// thread in blocks of 256 191.4, in blocks of 64 188.5.  Update blocks per SM
+// (phase 0, 1): (8, 6) 190, (10, 6) 188.8, (12, 7) 191, (9, 8) 189.8; density
+// blocks 6, 8, 10, 12: 190, 187.1, 187.4, 192.  Loads that leave L1 alone
+// lost (200^3 198 -> 208), as did a density pass and an update chunk by chunk
+// of planes, for L2's sake (225-284).
 template <int PHASE>
 constexpr int c2_nodes_per_thread() { return PHASE == 0 ? 1 : 2; }
-constexpr int c2_update_nodes_per_thread() { return 2; }
 
 // Both kernels pass pdl_gate() (pair.cuh): launched with programmatic
 // stream serialization, each overlaps its prologue with the end of the
 // kernel before it.
 template <typename T, int PHASE, bool WRITE_RHO>
-__global__ void __launch_bounds__(kC2Threads, 5)
+__global__ void __launch_bounds__(kC2Threads, 8)
     k_cdensity(const T* __restrict__ cpop, uint32_t cs,
                const uint2* __restrict__ cinfo, const uint2* __restrict__ wtab,
                int kbeg, int nfluid, float* __restrict__ rho_out,
@@ -136,27 +145,30 @@ __global__ void __launch_bounds__(kC2Threads, 5)
     node_density0<T, WRITE_RHO, true>(cpop, cs, cinfo, wtab, (int)k, rho_out,
                                       psi, g, p, a, inj);
   else
-    pair_density<T, 1, WRITE_RHO, true>(cpop, cs, cinfo, wtab, (int)k, nfluid,
-                                        rho_out, psi, g, p, a, inj);
+    pair_density<T, WRITE_RHO, true>(cpop, cs, cinfo, (int)k, nfluid, rho_out,
+                                     psi, g, p, a, inj);
 }
 
 // The update's blocks run from the end of the lattice to its start: the density
 // pass before it has left the populations it read last in L2, and the next
-// step's density pass starts where the update ends (tau = 0.9, us per step:
-// 128^3 53.5 -> 48.9, 160^3 108 -> 101.6, 200^3 206 -> 198, FP16 176 -> 170).
+// step's density pass starts where the update ends (200^3 206 -> 198, FP16 176
+// -> 170, when that was done).
 template <typename T, int PHASE, bool WRITE_U, bool EQ>
-__global__ void __launch_bounds__(kC2Threads, 3)
+__global__ void __launch_bounds__(kC2Threads, PHASE == 0 ? 10 : 7)
     k_cupdate(T* __restrict__ cpop, uint32_t cs, const uint2* __restrict__ cinfo,
               const uint2* __restrict__ wtab, int kbeg, int nfluid,
               const float* __restrict__ psi, float* __restrict__ vel, Geom g,
               Phys p, StepArgs a, bool inj) {
   const long long block = gridDim.x - 1 - blockIdx.x;
   const long long k =
-      kbeg + c2_update_nodes_per_thread() * (block * kC2Threads + threadIdx.x);
+      kbeg + c2_nodes_per_thread<PHASE>() * (block * kC2Threads + threadIdx.x);
   if (k >= nfluid) return;
-  pair_update<T, PHASE, WRITE_U, EQ, PsiPlain, true>(cpop, cs, cinfo, wtab, (int)k,
-                                                 nfluid, PsiPlain{psi}, vel, g,
-                                                 p, a, inj);
+  if (PHASE == 0)
+    node_update0<T, WRITE_U, EQ, true>(cpop, cs, cinfo, wtab, (int)k, psi, vel, g,
+                                       p, a, inj);
+  else
+    pair_update<T, WRITE_U, EQ, true>(cpop, cs, cinfo, (int)k, nfluid, psi, vel, g,
+                                      p, a, inj);
 }
 
 }  // namespace mlbm

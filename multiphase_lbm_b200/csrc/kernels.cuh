@@ -150,9 +150,10 @@ struct Equilibrium<__half> {
 };
 
 // Force, velocity shift and BGK relaxation of one interior fluid node
-// (include/iteration_device.cuh:69-206).  psi_nb(i) returns psi at x + e_i.
+// (include/iteration_device.cuh:69-206).  psi_nb(i) returns psi at x + e_i;
+// eq: omega is 1.
 template <typename T, typename R, typename PsiNb>
-__device__ __forceinline__ void collide(const Phys& p, R d, R psi_self,
+__device__ __forceinline__ void collide(bool eq, const Phys& p, R d, R psi_self,
                                         PsiNb psi_nb, R (&f)[Q], R& ux, R& uy,
                                         R& uz) {
   // F = -G psi(x) sum_{i=1..18} w_i psi(x + e_i) e_i, terms in order i
@@ -194,7 +195,7 @@ __device__ __forceinline__ void collide(const Phys& p, R d, R psi_self,
   };
   // omega = 1: f_i + (feq_i - f_i) is feq_i, taken without the two roundings
   // (what the moment step relies on, moments.cuh)
-  if (omega == R(1)) {
+  if (eq) {
     const R base = Equilibrium<T>::base(usq);
     f[0] = rmul(wd0, base);
 #pragma unroll

@@ -1,12 +1,12 @@
-// pair.cuh -- the per-node work of the compact (fluid-only) kernels done for
-// two consecutive fluid nodes per thread with Blackwell's packed FP32
-// instructions.
+// pair.cuh -- the per-node work of the compact (fluid-only) kernels: for two
+// consecutive fluid nodes per thread with Blackwell's packed FP32 instructions
+// in the local AA phase (1), for one in the gather/push phase (0).
 //
-// A thread owns the fluid nodes k and k + 1 (k even).  Their populations of
-// one slot are adjacent in the compact layout, so in the local AA phase a
-// slot of both nodes is one 8-byte load or store (4 bytes in FP16), and all
-// arithmetic runs on float2 pairs with the packed fma.rn.f32x2 instruction,
-// one instruction for both nodes.  Each lane rounds exactly like the scalar
+// A thread of the local phase owns the fluid nodes k and k + 1 (k even).  Their
+// populations of one slot are adjacent in the compact layout, so a slot of both
+// nodes is one 8-byte load or store (4 bytes in FP16), and all arithmetic runs
+// on float2 pairs with the packed fma.rn.f32x2 instruction, one instruction for
+// both nodes.  Each lane rounds exactly like the scalar
 // __fadd_rn / __fsub_rn / __fmul_rn / __fmaf_rn, and the packed code performs
 // the operations of collide() (kernels.cuh) in the same order, so every node
 // gets the same bits as in the scalar kernels.
@@ -15,9 +15,7 @@
 // count is followed by a hole: an unused slot whose node word has no fluid
 // bit), so a pair never straddles two planes.  A pair whose second slot is a
 // hole holds one node: its second lane is made a copy of the first (same
-// node, same loads), so every store of that lane repeats a store of the
-// first; only the pair store of the local phase writes the second lane, into
-// the hole.
+// node, same loads); the pair store writes it into the hole.
 //
 // AA addressing (kernels.cuh conventions): in both phases, direction d
 // (1..18) of a node uses one address A_d for the load of f_opp(d) and for
@@ -133,50 +131,6 @@ __device__ __forceinline__ void aa_addresses0(const uint2* __restrict__ wtab,
   }
 }
 
-// Pre-collision populations of the pair: f[i] = (node a, node b).
-template <typename T, int PHASE>
-__device__ __forceinline__ void pair_gather(const T* cpop, uint32_t cs, int k,
-                                            const uint32_t (&A)[Q],
-                                            const uint32_t (&B)[Q], float shift,
-                                            float2 (&f)[Q]) {
-  if (PHASE == 1) {
-    f[0] = PopPair<T>::ld2(cpop + k, shift * weight<float>(0));
-#pragma unroll
-    for (int d = 1; d < Q; ++d)
-      f[opp(d)] = PopPair<T>::ld2(cpop + (uint32_t)opp(d) * cs + (uint32_t)k,
-                                  shift * weight<float>(d));
-  } else {
-#pragma unroll
-    for (int d = 0; d < Q; ++d) {
-      const float s = shift * weight<float>(d);
-      const int i = opp(d);
-      f[i].x = PopPair<T>::ld1(cpop + A[d], s);
-      f[i].y = PopPair<T>::ld1(cpop + B[d], s);
-    }
-  }
-}
-
-template <typename T, int PHASE>
-__device__ __forceinline__ void pair_scatter(T* cpop, uint32_t cs, int k,
-                                             const uint32_t (&A)[Q],
-                                             const uint32_t (&B)[Q],
-                                             float shift, const float2 (&f)[Q]) {
-  if (PHASE == 1) {
-    PopPair<T>::st2(cpop + k, f[0], shift * weight<float>(0));
-#pragma unroll
-    for (int d = 1; d < Q; ++d)
-      PopPair<T>::st2(cpop + (uint32_t)opp(d) * cs + (uint32_t)k, f[d],
-                      shift * weight<float>(d));
-  } else {
-#pragma unroll
-    for (int d = 0; d < Q; ++d) {
-      const float s = shift * weight<float>(d);
-      PopPair<T>::st1(cpop + A[d], f[d].x, s);
-      PopPair<T>::st1(cpop + B[d], f[d].y, s);
-    }
-  }
-}
-
 // Equilibrium (kernels.cuh) of two nodes: base, and the terms of a direction
 // and of its opposite (term(base, -eu), in the operations that give its bits).
 template <typename T>
@@ -276,16 +230,6 @@ __device__ __forceinline__ void collide2(bool eq, const Phys& p, float2 d,
   }
 }
 
-// psi reader of the update pass, given psi_index() positions: the float psi
-// array through the read-only path (psi complete before the launch).
-// ready() is called once before the first psi read.
-struct PsiPlain {
-  const float* psi;
-  __device__ __forceinline__ void ready() const {}
-  __device__ __forceinline__ float self(uint32_t i) const { return __ldg(psi + i); }
-  __device__ __forceinline__ float nb(uint32_t i, int) const { return __ldg(psi + i); }
-};
-
 // Programmatic dependent launch.  A step kernel launched with the
 // programmatic-serialization attribute may start while the kernel before it
 // in the stream is still running; pdl_gate() waits until that kernel has
@@ -319,24 +263,20 @@ __device__ __forceinline__ Pair load_pair(const uint2* __restrict__ cinfo, int k
   return q;
 }
 
-// Pre-collision populations of pair q (both phases), with the second lane a
-// copy of the first for a single-node pair.
-template <typename T, int PHASE, bool GATE = false>
-__device__ __forceinline__ void pair_load(const T* cpop, uint32_t cs,
-                                          const uint2* __restrict__ wtab,
-                                          const Geom& g, const Pair& q,
-                                          float shift, uint32_t (&A)[Q],
-                                          uint32_t (&B)[Q], float2 (&f)[Q]) {
-  if (PHASE == 0) {
-    aa_addresses0(wtab, g, cs, q.a, A);
-    aa_addresses0(wtab, g, cs, q.b, B);
-  }
-  pdl_gate<GATE>();
+// Pre-collision populations of pair q, f[i] = (node a, node b), with the second
+// lane a copy of the first for a single-node pair.
+template <typename T>
+__device__ __forceinline__ void pair_load(const T* cpop, uint32_t cs, const Pair& q,
+                                          float shift, float2 (&f)[Q]) {
   if (q.a.kind && q.b.kind) {
 #pragma unroll
     for (int i = 0; i < Q; ++i) f[i] = p_dup(0.f);
   } else {
-    pair_gather<T, PHASE>(cpop, cs, q.a.k, A, B, shift, f);
+    f[0] = PopPair<T>::ld2(cpop + q.a.k, shift * weight<float>(0));
+#pragma unroll
+    for (int d = 1; d < Q; ++d)
+      f[opp(d)] = PopPair<T>::ld2(cpop + (uint32_t)opp(d) * cs + (uint32_t)q.a.k,
+                                  shift * weight<float>(d));
   }
   if (!q.two) {
 #pragma unroll
@@ -357,19 +297,18 @@ __device__ __forceinline__ float2 pair_rho(const Phys& p, const Geom& g,
   return d;
 }
 
-// Density pass of one pair (the work of k_cdensity for two nodes).
-template <typename T, int PHASE, bool WRITE_RHO, bool PDL = false>
+// Density pass of one pair, local phase.
+template <typename T, bool WRITE_RHO, bool PDL = false>
 __device__ __forceinline__ void pair_density(const T* cpop, uint32_t cs,
                                              const uint2* __restrict__ cinfo,
-                                             const uint2* __restrict__ wtab,
                                              int k, int nfluid, float* rho_out,
                                              float* psi, const Geom& g,
                                              const Phys& p, const StepArgs& a,
                                              bool inj) {
   const Pair q = load_pair(cinfo, k, nfluid);
-  uint32_t A[Q], B[Q];
   float2 f[Q];
-  pair_load<T, PHASE, PDL>(cpop, cs, wtab, g, q, p.rho_shift, A, B, f);
+  pdl_gate<PDL>();
+  pair_load<T>(cpop, cs, q, p.rho_shift, f);
   const float2 d = pair_rho(p, g, a, inj, q, f);
   if (WRITE_RHO) {
     rho_out[node_index(g, q.a.x, q.a.y, q.a.z)] = d.x;
@@ -379,47 +318,18 @@ __device__ __forceinline__ void pair_density(const T* cpop, uint32_t cs,
   if (q.two) store_psi<float>(psi, g, q.b.x, q.b.y, q.b.z, psi_of<float>(p, d.y));
 }
 
-// Shared memory of the gather/push update: one array for every form of
-// pair_update in a kernel.
-__device__ __forceinline__ uint32_t (*parked_addresses())[kC2Threads] {
-  __shared__ uint32_t parked[2 * Q][kC2Threads];
-  return parked;
-}
-
-// Update pass of one pair (the work of k_cupdate for two nodes).
-template <typename T, int PHASE, bool WRITE_U, bool EQ, class PsiR, bool PDL = false>
+// Update pass of one pair, local phase.
+template <typename T, bool WRITE_U, bool EQ, bool PDL = false>
 __device__ __forceinline__ void pair_update(T* cpop, uint32_t cs,
                                             const uint2* __restrict__ cinfo,
-                                            const uint2* __restrict__ wtab,
-                                            int k, int nfluid, const PsiR& pr,
+                                            int k, int nfluid,
+                                            const float* __restrict__ psi,
                                             float* vel, const Geom& g,
                                             const Phys& p, const StepArgs& a,
                                             bool inj) {
   const Pair q = load_pair(cinfo, k, nfluid);
-  uint32_t A[Q], B[Q];
   float2 f[Q];
-  // The gather/push step (phase 0) parks its 2 x 19 addresses in shared
-  // memory between the gather and the push: held in registers across the
-  // collision they leave too few for 3 CTAs per SM.  Each node's addresses
-  // are parked right after its own gather, so only 19 are live at a time.
-  // (k_cupdate: 1-D blocks of kC2Threads.)
-  if (PHASE == 0) {
-    uint32_t(*parked)[kC2Threads] = parked_addresses();
-    aa_addresses0(wtab, g, cs, q.a, A);
-#pragma unroll
-    for (int e = 0; e < Q; ++e) {
-      f[opp(e)].x = PopPair<T>::ld1(cpop + A[e], p.rho_shift * weight<float>(e));
-      parked[e][threadIdx.x] = A[e];
-    }
-    aa_addresses0(wtab, g, cs, q.b, A);  // q.b is q.a for a one-node pair
-#pragma unroll
-    for (int e = 0; e < Q; ++e) {
-      f[opp(e)].y = PopPair<T>::ld1(cpop + A[e], p.rho_shift * weight<float>(e));
-      parked[Q + e][threadIdx.x] = A[e];
-    }
-  } else {
-    pair_load<T, PHASE>(cpop, cs, wtab, g, q, p.rho_shift, A, B, f);
-  }
+  pair_load<T>(cpop, cs, q, p.rho_shift, f);
   pdl_gate<PDL>();  // psi and the population stores come from / go after it
   const float2 d = pair_rho(p, g, a, inj, q, f);
   float2 ux, uy, uz;
@@ -427,12 +337,11 @@ __device__ __forceinline__ void pair_update(T* cpop, uint32_t cs,
     const uint32_t pa = (uint32_t)psi_index(g, q.a.x, q.a.y, q.a.z);
     const uint32_t pb = (uint32_t)psi_index(g, q.b.x, q.b.y, q.b.z);
     const int sy = g.pxg, sz = (g.ly + 2) * g.pxg;
-    pr.ready();
     collide2<T>(
-        EQ, p, d, make_float2(pr.self(pa), pr.self(pb)),
+        EQ, p, d, make_float2(__ldg(psi + pa), __ldg(psi + pb)),
         [&](int i) {
           const int o = ex(i) + ey(i) * sy + ez(i) * sz;
-          return make_float2(pr.nb(pa + o, i), pr.nb(pb + o, i));
+          return make_float2(__ldg(psi + pa + o), __ldg(psi + pb + o));
         },
         f, ux, uy, uz);
   }
@@ -456,23 +365,17 @@ __device__ __forceinline__ void pair_update(T* cpop, uint32_t cs,
     vel[3 * nb + 1] = uy.y;
     vel[3 * nb + 2] = uz.y;
   }
-  if (PHASE == 0) {
-    const volatile uint32_t(*pk)[kC2Threads] = parked_addresses();
+  PopPair<T>::st2(cpop + k, f[0], p.rho_shift * weight<float>(0));
 #pragma unroll
-    for (int e = 0; e < Q; ++e) {
-      A[e] = pk[e][threadIdx.x];
-      B[e] = pk[Q + e][threadIdx.x];
-    }
-  }
-  pair_scatter<T, PHASE>(cpop, cs, k, A, B, p.rho_shift, f);
+  for (int d = 1; d < Q; ++d)
+    PopPair<T>::st2(cpop + (uint32_t)opp(d) * cs + (uint32_t)k, f[d],
+                    p.rho_shift * weight<float>(d));
 }
 
-
-
 // ---- one node per thread (AA phase 0) -----------------------------------------
-// The density pass of the gather step: one node per thread (on pairs it
-// measured slower at 64 and at 80 registers).  Holes (no fluid bit) are
-// skipped.
+// The gather/push step: a thread's addresses are its node's own, so pairs save
+// no loads, and one node leaves registers for more warps.  Holes (no fluid bit)
+// are skipped.
 template <typename T, bool WRITE_RHO, bool PDL = false>
 __device__ __forceinline__ void node_density0(const T* cpop, uint32_t cs,
                                               const uint2* __restrict__ cinfo,
@@ -501,6 +404,67 @@ __device__ __forceinline__ void node_density0(const T* cpop, uint32_t cs,
   }
   if (WRITE_RHO) rho_out[node_index(g, n.x, n.y, n.z)] = d;
   store_psi<float>(psi, g, n.x, n.y, n.z, psi_of<float>(p, d));
+}
+
+// Shared memory of the gather/push update: one array for every form of
+// node_update0 in a kernel.
+__device__ __forceinline__ uint32_t (*parked_addresses())[kC2Threads] {
+  __shared__ uint32_t parked[Q][kC2Threads];
+  return parked;
+}
+
+// Update pass of one node (1-D blocks of kC2Threads).  The 19 addresses are
+// parked in shared memory between the gather and the push: held in registers
+// across the collision they leave too few for 10 blocks of 128 per SM.
+template <typename T, bool WRITE_U, bool EQ, bool PDL = false>
+__device__ __forceinline__ void node_update0(T* cpop, uint32_t cs,
+                                             const uint2* __restrict__ cinfo,
+                                             const uint2* __restrict__ wtab, int k,
+                                             const float* __restrict__ psi,
+                                             float* vel, const Geom& g,
+                                             const Phys& p, const StepArgs& a,
+                                             bool inj) {
+  const PairNode n = pair_node(cinfo, k);
+  if (!(n.nb & NB_SELF)) return;
+  float f[Q];
+  {
+    uint32_t A[Q];
+    uint32_t(*parked)[kC2Threads] = parked_addresses();
+    aa_addresses0(wtab, g, cs, n, A);
+#pragma unroll
+    for (int e = 0; e < Q; ++e) {
+      f[opp(e)] = PopPair<T>::ld1(cpop + A[e], p.rho_shift * weight<float>(e));
+      parked[e][threadIdx.x] = A[e];
+    }
+  }
+  pdl_gate<PDL>();  // psi and the population stores come from / go after it
+  float d = 0.f;
+#pragma unroll
+  for (int i = 0; i < Q; ++i) d = radd(d, f[i]);
+  d = n.kind ? slab_density(p, n.kind) : inject_on(p, g, a, inj, n.y, d);
+  float ux, uy, uz;
+  const uint32_t at = (uint32_t)psi_index(g, n.x, n.y, n.z);
+  const int sy = g.pxg, sz = (g.ly + 2) * g.pxg;
+  collide<T>(
+      EQ, p, d, __ldg(psi + at),
+      [&](int i) { return __ldg(psi + (at + ex(i) + ey(i) * sy + ez(i) * sz)); },
+      f, ux, uy, uz);
+  if (n.kind) {
+#pragma unroll
+    for (int i = 0; i < Q; ++i) f[i] = rmul(weight<float>(i), d);
+    ux = uy = uz = 0.f;
+  }
+  if (WRITE_U) {
+    float* v = vel + 3 * (long long)node_index(g, n.x, n.y, n.z);
+    v[0] = ux;
+    v[1] = uy;
+    v[2] = uz;
+  }
+  const volatile uint32_t(*parked)[kC2Threads] = parked_addresses();
+#pragma unroll
+  for (int e = 0; e < Q; ++e)
+    PopPair<T>::st1(cpop + parked[e][threadIdx.x], f[e],
+                    p.rho_shift * weight<float>(e));
 }
 
 }  // namespace mlbm

@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(256)
         const R* pp = ring + slot_of(z + 1) * slot_elems;
         const int c = (ly_ + 1) * kBoxX + (tid & 31) + 4;
         collide<T, R>(
-            p, d, p0[c],
+            p.omega == 1.f, p, d, p0[c],
             [&](int i) {
               const R* pl = ez(i) < 0 ? pm : (ez(i) > 0 ? pp : p0);
               return pl[c + ey(i) * kBoxX + ex(i)];
