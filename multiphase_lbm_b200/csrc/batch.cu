@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <climits>
 #include <cstring>
 #include <new>
 #include <type_traits>
@@ -48,17 +49,15 @@ struct mlbm_batch {
   int ccap = 0;
   int grid_c = 0;
   // moment mode (every domain with tau = 1): the domains are held as moments
-  // and every pass is one launch over all of them (batch_moments.cuh)
+  // and every pass is one launch over up to kMomGroup of them (batch_moments.cuh)
   bool moments = false;
-  MomDomain* d_mdesc = nullptr;
-  MomBlock* d_mblocks = nullptr;
-  int mcap = 0, mblocks_cap = 0;
-  int grid_m = 0;
+  std::vector<MomDomain> mdesc;
 };
 
 namespace {
 
 constexpr int kGraphSteps = 8;
+constexpr int kMomGroup = 128, kMomFew = 16;  // domains of a moment launch
 
 __global__ void k_advance_step(long long* step, int n) {
   if (threadIdx.x == 0 && blockIdx.x == 0) *step += n;
@@ -155,8 +154,9 @@ mlbm_status rebuild_compact(mlbm_batch* b) {
 
 // Moment mode: tables of the domains, all held as moments.
 mlbm_status rebuild_moments(mlbm_batch* b) {
-  std::vector<MomDomain> desc;
-  std::vector<MomBlock> blocks;
+  std::vector<MomDomain>& desc = b->mdesc;
+  desc.clear();
+  int n = 0;
   for (size_t s = 0; s < b->dom.size(); ++s) {
     const mlbm_lattice* lat = b->dom[s];
     if (!lat) continue;
@@ -171,38 +171,14 @@ mlbm_status rebuild_moments(mlbm_batch* b) {
     d.rho = lat->rho;
     d.list = PairList{ms.words, ms.xyz, ms.npairs};
     d.step_origin = b->origin[s];
-    for (int k = 0; k < ms.npairs; k += kMomThreads)
-      blocks.push_back(MomBlock{(int)desc.size(), k});
-    desc.push_back(d);
+    if (ms.npairs > 0) desc.push_back(d);
+    ++n;
   }
-  const int n = (int)desc.size(), nb = (int)blocks.size();
   if (n > kMaxBatch) return bfail(MLBM_ERR_ARG, "too many domains in a batch");
-  if (n > b->mcap) {
-    cudaFree(b->d_mdesc);
-    b->d_mdesc = nullptr;
-    b->mcap = 0;
-    const int cap = std::max(n, 64);
-    BCUDA(cudaMalloc(&b->d_mdesc, cap * sizeof(MomDomain)), "batch table");
-    b->mcap = cap;
-  }
-  if (nb > b->mblocks_cap) {
-    cudaFree(b->d_mblocks);
-    b->d_mblocks = nullptr;
-    b->mblocks_cap = 0;
-    BCUDA(cudaMalloc(&b->d_mblocks, (size_t)nb * sizeof(MomBlock)), "batch table");
-    b->mblocks_cap = nb;
-  }
-  if (n)
-    BCUDA(cudaMemcpyAsync(b->d_mdesc, desc.data(), n * sizeof(MomDomain),
-                          cudaMemcpyHostToDevice, b->stream), "batch table");
-  if (nb)
-    BCUDA(cudaMemcpyAsync(b->d_mblocks, blocks.data(), (size_t)nb * sizeof(MomBlock),
-                          cudaMemcpyHostToDevice, b->stream), "batch table");
   BCUDA(cudaMemcpyAsync(b->d_step, &b->bstep, sizeof(long long),
                         cudaMemcpyHostToDevice, b->stream), "batch step");
   BCUDA(cudaStreamSynchronize(b->stream), "batch table");
   b->nactive = n;
-  b->grid_m = nb;
   b->dirty = false;
   return MLBM_OK;
 }
@@ -333,16 +309,34 @@ mlbm_status rebuild(mlbm_batch* b) {
   return MLBM_OK;
 }
 
+// Both passes of the domains first, first + 1, ... (at most N).
+template <typename T, int N>
+void launch_mom_group(mlbm_batch* b, size_t first, int delta, int reverse,
+                      unsigned inject, bool write_rho) {
+  using R = typename Pop<T>::Real;
+  MomDomains<N> t;
+  const int n = (int)std::min<size_t>(b->mdesc.size() - first, N);
+  std::memcpy((void*)t.d, b->mdesc.data() + first, n * sizeof(MomDomain));
+  int grid = 0;
+  for (int i = 0; i < N; ++i) {
+    t.block[i] = i < n ? grid : INT_MAX;
+    if (i < n) grid += (t.d[i].list.count + kMomThreads - 1) / kMomThreads;
+  }
+  auto gather = write_rho ? k_batch_mom_gather<T, true, N> : k_batch_mom_gather<T, false, N>;
+  gather<<<grid, kMomThreads, 0, b->stream>>>(t, b->d_step, delta, reverse, inject);
+  k_batch_mom_collide<R, N><<<grid, kMomThreads, 0, b->stream>>>(t);
+}
+
 template <typename T>
 void launch_step(mlbm_batch* b, int delta, int reverse, unsigned inject,
                  bool write_rho) {
   if (b->moments) {
-    if (b->grid_m == 0) return;
-    auto gather = write_rho ? k_batch_mom_gather<T, true> : k_batch_mom_gather<T, false>;
-    gather<<<b->grid_m, kMomThreads, 0, b->stream>>>(b->d_mdesc, b->d_mblocks,
-                                                     b->d_step, delta, reverse, inject);
-    k_batch_mom_collide<typename Pop<T>::Real>
-        <<<b->grid_m, kMomThreads, 0, b->stream>>>(b->d_mdesc, b->d_mblocks);
+    for (size_t first = 0; first < b->mdesc.size(); first += kMomGroup) {
+      if (b->mdesc.size() - first <= kMomFew)
+        launch_mom_group<T, kMomFew>(b, first, delta, reverse, inject, write_rho);
+      else
+        launch_mom_group<T, kMomGroup>(b, first, delta, reverse, inject, write_rho);
+    }
     return;
   }
   if constexpr (!std::is_same<T, double>::value) {
@@ -474,8 +468,6 @@ mlbm_status mlbm_batch_destroy(mlbm_batch* b) {
   drop_graph(b);
   for (mlbm_lattice* lat : b->dom)
     if (lat) mlbm_lattice_destroy(lat);
-  cudaFree(b->d_mdesc);
-  cudaFree(b->d_mblocks);
   cudaFree(b->d_cdesc);
   cudaFree(b->d_cpre);
   cudaFree(b->d_desc);

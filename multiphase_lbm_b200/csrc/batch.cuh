@@ -56,6 +56,15 @@ __device__ __forceinline__ int find_domain(const long long* pre, int n,
   return lo;
 }
 
+// Whether a domain injects at its step.  (A 64-bit remainder is some 100
+// instructions, a tenth of the gather of a pair of nodes.)
+__device__ __forceinline__ bool batch_inject(const Phys& p, long long step) {
+  const unsigned long long n = p.rho_inject_period, s = (unsigned long long)step;
+  if (n == 0ull) return false;
+  if (((n | s) >> 32) == 0ull) return (uint32_t)s % (uint32_t)n == 0u;
+  return s % n == 0ull;
+}
+
 template <typename T, int PHASE>
 __device__ __forceinline__ void batch_density_node(const DomainDesc& d,
                                                    const StepArgs& s, int x,

@@ -52,11 +52,6 @@ __device__ __forceinline__ bool bc_locate(const long long* __restrict__ pre,
   return true;
 }
 
-__device__ __forceinline__ bool bc_inject(const Phys& p, long long dstep) {
-  return p.rho_inject_period != 0ull &&
-         (unsigned long long)dstep % p.rho_inject_period == 0ull;
-}
-
 // Blocks per SM, (density, update): 24 domains of edges 32-128 at tau 0.9, us per
 // step FP32 / FP16: (10, 8) 302 / 270; (8, 7) 312 / 284, (10, 7) 309 / 274, (6, 8)
 // 304 / 276, (12, 8) 311 / 279, (10, 10) 332 / 294; updates by pairs in both
@@ -74,7 +69,7 @@ __global__ void __launch_bounds__(kBCThreads, 10)
   const CDomain& D = doms[d];
   const int ph = D.phase_base ^ (int)(s & 1);
   StepArgs a{s - D.step_origin, reverse, inject_type};
-  const bool inj = bc_inject(D.p, a.step);
+  const bool inj = batch_inject(D.p, a.step);
   const long long t = local * kBCThreads + threadIdx.x;
   if (ph == 0) {
     if (t >= D.nfluid) return;
@@ -101,7 +96,7 @@ __global__ void __launch_bounds__(kBCThreads, 8)
   const CDomain& D = doms[d];
   const int ph = D.phase_base ^ (int)(s & 1);
   StepArgs a{s - D.step_origin, reverse, inject_type};
-  const bool inj = bc_inject(D.p, a.step);
+  const bool inj = batch_inject(D.p, a.step);
   const long long t = local * kBCThreads + threadIdx.x;
   if ((ph == 0 ? t : 2 * t) >= D.nfluid) return;
   auto update = [&](auto eq) {

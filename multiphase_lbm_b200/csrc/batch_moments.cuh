@@ -4,10 +4,18 @@
 // kernels, so a domain advanced in a batch is bit-identical to the same domain
 // advanced alone.
 //
-// Each domain owns a contiguous range of blocks; a table gives every block its
-// domain and its place in the domain's pair list (one load; a search over the
-// domains' block prefixes would be a chain of dependent ones).  The batch step
-// is read from the device counter, which graph replays advance.
+// Each domain owns a contiguous range of blocks.  The domains' descriptions and
+// first blocks are a kernel parameter: what a block needs before its first load
+// (the search for its domain, pointers, sizes) comes from the constant cache, and
+// the sizes and parameters stay out of L1 and, mostly, of registers.  In device
+// memory, with a table of every block's domain, they cost a chain of two loads at
+// the head of each block and some 40 uniform loads a warp, and the gather spilled.
+// 8 domains of 128^3 / 48 of edges 32-128 / 100 of 32^3, us per step: FP32 293 /
+// 394 / 60 -> 265 / 360 / 56, FP16 281 / 378 / 57 -> 268 / 361 / 56, FP64 637 / 847 /
+// 134 -> 485 / 649 / 106 (the injection test in 32 bits a good part of FP64's).
+// A parameter holds 128 domains (23 KB of 32), more take more launches; up to 16
+// the launch carries less.  The batch step is read from the device counter, which
+// graph replays advance.
 #pragma once
 
 #include "batch.cuh"
@@ -30,31 +38,48 @@ struct MomBlock {
   int domain, first;  // first pair
 };
 
-template <typename T, bool WRITE_RHO>
+// The domains of a launch and the first block of each (the entries past the last
+// domain: INT_MAX).
+template <int N>
+struct MomDomains {
+  MomDomain d[N];
+  int block[N];
+
+  __device__ __forceinline__ MomBlock find(int b) const {
+    int lo = 0;
+#pragma unroll
+    for (int h = N / 2; h; h /= 2)
+      if (block[lo + h] <= b) lo += h;
+    return MomBlock{lo, (b - block[lo]) * kMomThreads};
+  }
+};
+
+template <typename T, bool WRITE_RHO, int N>
 __global__ void __launch_bounds__(kMomThreads, mom_gather_blocks<T>())
-    k_batch_mom_gather(const MomDomain* __restrict__ doms,
-                       const MomBlock* __restrict__ blocks,
+    k_batch_mom_gather(const __grid_constant__ MomDomains<N> doms,
                        const long long* __restrict__ step, int delta, int reverse,
                        unsigned inject_type) {
   using R = typename Pop<T>::Real;
-  const MomBlock b = blocks[blockIdx.x];
-  const MomDomain& D = doms[b.domain];
+  const MomBlock b = doms.find((int)blockIdx.x);
+  const MomDomain& D = doms.d[b.domain];
   const StepArgs a{*step + delta - D.step_origin, reverse, inject_type};
-  const bool inj = D.p.rho_inject_period != 0ull &&
-                   (unsigned long long)a.step % D.p.rho_inject_period == 0ull;
+  const bool inj = batch_inject(D.p, a.step);
   const int k = b.first + (int)threadIdx.x;
-  mom_gather<T, WRITE_RHO, false>(
-      static_cast<const Mom<R>*>(D.m), D.list, k,
-      static_cast<MomPair<R>*>(D.n), static_cast<R*>(D.rho),
-      static_cast<R*>(D.psi), D.g, D.p, a, inj, D.p.rho_shift);
+  if (k >= D.list.count) return;
+  const PairAt q = pair_at(D.g, D.list, k);
+  Gather<T> c{static_cast<const Mom<R>*>(D.m) + q.at, Columns(D.g, q.x, q.y),
+              q.na, q.nb, D.p.rho_shift, D.p.rho_shift};
+  c.run();
+  mom_put<R, WRITE_RHO>(q, c.sum.pair(), static_cast<MomPair<R>*>(D.n), k,
+                        static_cast<R*>(D.rho), static_cast<R*>(D.psi), D.g, D.p, a,
+                        inj);
 }
 
-template <typename R>
-__global__ void __launch_bounds__(kMomThreads, sizeof(R) == 8 ? 6 : 8)
-    k_batch_mom_collide(const MomDomain* __restrict__ doms,
-                        const MomBlock* __restrict__ blocks) {
-  const MomBlock b = blocks[gridDim.x - 1 - blockIdx.x];
-  const MomDomain& D = doms[b.domain];
+template <typename R, int N>
+__global__ void __launch_bounds__(kMomThreads, sizeof(R) == 8 ? 7 : 8)
+    k_batch_mom_collide(const __grid_constant__ MomDomains<N> doms) {
+  const MomBlock b = doms.find((int)(gridDim.x - 1 - blockIdx.x));
+  const MomDomain& D = doms.d[b.domain];
   const int k = b.first + (int)threadIdx.x;
   if (k < D.list.count)
     mom_collide<R, false, false>(static_cast<const MomPair<R>*>(D.n), D.list, k,
