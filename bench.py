@@ -79,7 +79,10 @@ PHYS = phys(200)
 # The end-to-end leg runs a job of at least this many steps (its one-time
 # upload and layout change are part of it), whatever --steps is.
 E2E_MIN_STEPS = 500
+# Bytes of state a step reads and writes per fluid node: 19 populations, or
+# the 4 moments of the tau = 1 step (32-bit in FP16 storage too).
 BYTES_PER_FLUID = {"f32": 152, "f16": 76, "f64": 304}
+MOMENT_BYTES_PER_FLUID = {"f32": 32, "f16": 32, "f64": 64}
 
 
 def workload(shape=SHAPE, seed=2024):
@@ -189,6 +192,16 @@ def load_traffic(kernel, storage):
 KERNEL_INFO = {6: ("band", "k_band (one-pass step, compact layout, two buffers)", 1),
                3: ("compact", "time step (k_cdensity + k_cupdate, compact layout)", 2),
                2: ("two-pass", "time step (k_density + k_update_zm)", 2)}
+MOMENT_INFO = ("moments", "time step (k_mom_gather + k_mom_collide)", 2)
+
+
+def step_info(kernel, kernel_id):
+    """(name, label, launches per step, bytes per fluid node by storage) of
+    the step that runs: at tau = 1 the compact kernel, and the two-pass one
+    where none was asked for, advance the lattice as moments."""
+    if PHYS["tau"] == 1.0 and (kernel == 3 or (kernel == 2 and kernel_id is None)):
+        return MOMENT_INFO + (MOMENT_BYTES_PER_FLUID,)
+    return KERNEL_INFO[kernel] + (BYTES_PER_FLUID,)
 
 
 class ClockSampler:
@@ -445,7 +458,7 @@ def measure_64(capi, torch, args, local):
     torch.cuda.synchronize()
     ms, blocks, _ = timed_blocks(lat, torch, args.warmup, steps, None,
                                  min(args.min_time, 0.5))
-    kernel = KERNEL_INFO.get(lat.step_kernel, ("", str(lat.step_kernel)))[1]
+    kernel = step_info(lat.step_kernel, None)[1]
     lat.close()
     per = ms / steps
     return {"ms_per_step": round(per, 5),
@@ -504,12 +517,12 @@ def main():
     # ---- device-timed region (inputs resident) --------------------------
     s_per_step, blocks, clocks, kernel = measure(
         capi, torch, fluid, rho, args.storage, args, local, dist, kernel_id)
-    kname, klabel, klaunches = KERNEL_INFO[kernel]
+    kname, klabel, klaunches, node_bytes = step_info(kernel, kernel_id)
     mlups = n_nodes * world / s_per_step / 1e6
 
     # ---- roofline of the time step ----------------------------------------
     peak, peak_kind = load_peaks()
-    alg_bytes = n_fluid * BYTES_PER_FLUID[args.storage] + n_nodes / 8
+    alg_bytes = n_fluid * node_bytes[args.storage] + n_nodes / 8
     achieved = alg_bytes / s_per_step / 1e9
     traffic = load_traffic(kname, args.storage) if args.size == 200 else None
 
@@ -517,7 +530,7 @@ def main():
     if args.storage == "f32" and not args.no_fp16:
         s16, b16, c16, _ = measure(capi, torch, fluid, rho, "f16", args, local,
                                    dist, kernel_id)
-        alg16 = n_fluid * BYTES_PER_FLUID["f16"] + n_nodes / 8
+        alg16 = n_fluid * node_bytes["f16"] + n_nodes / 8
         fp16 = {"ms_per_step": round(s16 * 1e3, 4),
                 "value": round(n_nodes * world / s16 / 1e6, 2), "unit": "MLUPS",
                 "speedup_vs_fp32": round(s_per_step / s16, 3),
