@@ -164,8 +164,8 @@ def bench_config(fluid_nodes: int, spheres: int, n: int = 200) -> dict:
                         f"x={n - 1} rho 1.95, G -6, tau 1, rhos 0.182322",
             "lattice": [n, n, n], "fluid_nodes": int(fluid_nodes),
             "porosity": round(fluid_nodes / n ** 3, 5), "spheres": int(spheres),
-            "l2": "inputs larger than L2 (FP32 populations 0.61 GB, FP16 "
-                  "0.30 GB per step), no flush"}
+            "l2": "inputs larger than L2 (moments and psi 0.25 GB; populations "
+                  "0.61 GB in FP32, 0.30 GB in FP16), no flush"}
 
 
 def load_peaks():
