@@ -20,8 +20,8 @@ struct CompactState {
   bool active = false;     // the compact buffer holds the current state
   long long nfluid = 0, cs = 0;
   void* cpop = nullptr;        // [Q][cs] populations (T)
-  uint2* cinfo = nullptr;      // [cs] (neighbour word, packed x, y, z)
-  uint2* wtab = nullptr;       // [rows * wpr + 1] (mask word, wbase)
+  uint2* cinfo = nullptr;      // [cs] (neighbour word, packed x, y, z); with cpop
+  uint2* wtab = nullptr;       // [rows * wpr + 1] (mask word, wbase); with wbase
   bool two_pass_ok = false;    // the compact kernels fit the lattice
   uint32_t* wbase = nullptr;   // [rows * wpr + 1]
   long long cap = 0;           // cs the buffers were allocated for
