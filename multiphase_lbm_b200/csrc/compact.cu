@@ -76,11 +76,16 @@ mlbm_status build_tables(mlbm_lattice* lat) {
   c.row_start.assign((size_t)g.lz * g.ly + 1, 0);
   for (long long r = 0; r <= (long long)g.lz * g.ly; ++r)
     c.row_start[r] = h[r * g.wpr];
-  e = cudaMemcpy(c.wbase, h.data(), (nwords + 1) * sizeof(uint32_t),
-                 cudaMemcpyHostToDevice);
+  // on the lattice's stream, where k_wtab follows it: a copy through the
+  // default stream may return before it is done (pageable memory), and a
+  // non-blocking stream's kernels do not wait for it
+  e = cudaMemcpyAsync(c.wbase, h.data(), (nwords + 1) * sizeof(uint32_t),
+                      cudaMemcpyHostToDevice, lat->stream);
   if (e != cudaSuccess) return cuda_fail(e, "compact tables");
   k_wtab<<<(unsigned)((nwords + 256) / 256), 256, 0, lat->stream>>>(
       lat->mask, c.wbase, c.wtab, nwords);
+  e = cudaStreamSynchronize(lat->stream);  // h is read until then
+  if (e != cudaSuccess) return cuda_fail(e, "compact tables");
   c.nfluid = (long long)run;  // compact slots: fluid nodes and holes
   c.cs = std::max(64LL, (c.nfluid + 63) / 64 * 64);
   if (c.cs > c.cap) {

@@ -1,0 +1,48 @@
+"""Tables that a lattice builds on first use, against its own stream: a
+non-blocking stream is not ordered with the default stream, so what its
+kernels read has to come in on it, whatever the default stream does meanwhile."""
+import numpy as np
+import pytest
+
+from conftest import sphere_case
+
+pytestmark = pytest.mark.gpu
+
+BUSY = 600_000_000  # cycles: some 0.3 s of the default stream
+
+
+def _lattice(capi, shape, fluid, rho, storage, kernel, **kw):
+    lat = capi.Lattice(shape, storage=storage)
+    lat.set_step_kernel(kernel)
+    lat.set_params(capi.default_params(G=-5.0, rhos=0.2, rho_shift=1.0, **kw))
+    lat.upload(fluid, rho)
+    lat.initialize()
+    return lat
+
+
+@pytest.mark.parametrize("storage", [0, 1])
+def test_fluid_only_tables_come_in_on_the_lattices_stream(storage):
+    import torch
+
+    from multiphase_lbm_b200 import capi
+    shape = (70, 36, 28)
+    fluid, rho = sphere_case(shape, seed=3, rmin=2.0, rmax=4.0, porosity=0.6,
+                             rho0=1.2, amp=0.4)
+    want = _lattice(capi, shape, fluid, rho, storage, capi.KERNEL_TWO_PASS, tau=0.8)
+    want.iterate(0, 6)
+    stream = torch.cuda.Stream()  # non-blocking
+    for rep in range(2):  # the first one loads the kernels
+        lat = _lattice(capi, shape, fluid, rho, storage, capi.KERNEL_COMPACT, tau=0.8)
+        torch.cuda.synchronize()  # set-up ran on the default stream
+        lat.set_stream(stream.cuda_stream)
+        busy = torch.cuda.Event()
+        if rep:
+            torch.cuda._sleep(BUSY)
+        busy.record()
+        lat.iterate(0, 6)
+        if rep:  # built and launched without the default stream
+            assert not busy.query()
+        torch.cuda.synchronize()
+        assert np.array_equal(lat.field("f"), want.field("f"))
+        lat.close()
+    want.close()
