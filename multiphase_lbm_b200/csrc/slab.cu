@@ -305,9 +305,12 @@ mlbm_status mlbm_slab_ring_create(mlbm_lattice* const* slabs, int32_t n,
     r->njobs[w] = (int)jobs.size();
     if (jobs.empty()) continue;
     e = cudaMalloc((void**)&r->jobs[w], jobs.size() * sizeof(HaloJob));
+    // on the stream of the exchanges: a copy through the default stream may
+    // return before it is done, and a non-blocking stream does not wait for it
     if (e == cudaSuccess)
-      e = cudaMemcpy(r->jobs[w], jobs.data(), jobs.size() * sizeof(HaloJob),
-                     cudaMemcpyHostToDevice);
+      e = cudaMemcpyAsync(r->jobs[w], jobs.data(), jobs.size() * sizeof(HaloJob),
+                          cudaMemcpyHostToDevice, slabs[0]->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(slabs[0]->stream);
   }
   r->ready.assign(n, nullptr);
   for (int i = 0; i < n && e == cudaSuccess; ++i) {

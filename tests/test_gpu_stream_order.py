@@ -46,3 +46,33 @@ def test_fluid_only_tables_come_in_on_the_lattices_stream(storage):
         assert np.array_equal(lat.field("f"), want.field("f"))
         lat.close()
     want.close()
+
+
+def test_ring_jobs_come_in_on_the_slabs_stream():
+    import torch
+
+    from multiphase_lbm_b200 import capi, slab
+    shape = (40, 24, 20)
+    fluid, rho = sphere_case(shape, seed=5, rmin=2.0, rmax=4.0, porosity=0.6,
+                             rho0=1.2, amp=0.4)
+    want = _lattice(capi, shape, fluid, rho, 0, capi.KERNEL_TWO_PASS, tau=0.8)
+    want.iterate(0, 7)
+    m = fluid.astype(bool)
+    params = capi.default_params(G=-5.0, rhos=0.2, rho_shift=1.0, tau=0.8)
+    stream = torch.cuda.Stream()
+    for rep in range(2):  # the first one loads the kernels
+        with torch.cuda.stream(stream):
+            slabs = [slab.Slab(fluid, rho, params, 10 * i, 10) for i in range(2)]
+        torch.cuda.synchronize()
+        busy = torch.cuda.Event()
+        if rep:
+            torch.cuda._sleep(BUSY)
+        busy.record()
+        run = slab.SlabRun(slabs, slab.RingExchange(slabs))
+        run.run(0, 7)
+        if rep:
+            assert not busy.query()
+        torch.cuda.synchronize()
+        assert np.array_equal(slab.gather(slabs, "f")[m], want.field("f")[m])
+        run.close()
+    want.close()
