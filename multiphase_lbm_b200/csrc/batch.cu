@@ -25,6 +25,7 @@ struct mlbm_batch {
   std::vector<mlbm_lattice*> dom;     // slots (nullptr = free)
   std::vector<long long> origin;      // batch step at which step 0 would be
   std::vector<int> phase_base;        // AA phase offset (see DomainDesc)
+  std::vector<unsigned long long> seen;  // lattice's `changes` at the rebuild
   long long bstep = 0;                // steps executed by the batch
   // device tables, rebuilt when the set of domains or the tuning changes
   DomainDesc* d_desc = nullptr;
@@ -233,6 +234,12 @@ bool compact_mode(const mlbm_batch* b) {
 
 mlbm_status rebuild(mlbm_batch* b) {
   drop_graph(b);
+  // a domain advanced on its own may be in the other AA phase
+  for (size_t s = 0; s < b->dom.size(); ++s)
+    if (const mlbm_lattice* lat = b->dom[s]) {
+      b->phase_base[s] = (lat->phase + (int)(b->bstep & 1)) & 1;
+      b->seen[s] = lat->changes;
+    }
   if (b->moments) return rebuild_moments(b);
   b->compact = compact_mode(b);
   if (b->compact) return rebuild_compact(b);
@@ -424,10 +431,10 @@ int32_t insert_domain(mlbm_batch* b, mlbm_lattice* lat, int64_t step0) {
     b->dom.push_back(nullptr);
     b->origin.push_back(0);
     b->phase_base.push_back(0);
+    b->seen.push_back(0);
   }
   b->dom[slot] = lat;
   b->origin[slot] = b->bstep - step0;
-  b->phase_base[slot] = (lat->phase + (int)(b->bstep & 1)) & 1;
   b->dirty = true;
   return slot;
 }
@@ -570,17 +577,18 @@ mlbm_status mlbm_batch_iterate(mlbm_batch* b, int32_t nsteps, int32_t reverse,
   mlbm::DeviceGuard restore_device;
   BCUDA(cudaSetDevice(b->device), "cudaSetDevice");
   // the domains' form: it follows a domain added or removed since, one whose
-  // parameters changed, one advanced on its own
+  // tau came to or left 1, one advanced on its own
   bool moments = false;
   if (mlbm_status st = moments_mode(b, &moments)) return st;
   if (moments != b->moments) b->dirty = true;
   b->moments = moments;
   bool alone = false;
-  for (const mlbm_lattice* l : b->dom) {
+  for (size_t s = 0; s < b->dom.size(); ++s) {
+    const mlbm_lattice* l = b->dom[s];
     if (!l) continue;
+    if (l->changes != b->seen[s]) b->dirty = true;
     if (moments && (!l->mom.active || l->mom.shift != l->phys.rho_shift))
       alone = b->dirty = true;
-    if (!moments && b->compact && !l->compact.active) b->dirty = true;
   }
   if (alone) {
     if (mlbm_status st = step_alone(b, reverse, inject_type, nsteps == 1)) return st;

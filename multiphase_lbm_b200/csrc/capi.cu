@@ -555,6 +555,7 @@ static mlbm_status upload_mask_impl(mlbm_lattice* lat, const uint8_t* src,
   CUDA_TRY(cudaGetLastError(), "mask pack launch");
   CUDA_TRY(cudaStreamSynchronize(lat->stream), "mask upload");
   compact_invalidate(lat);
+  ++lat->changes;
   lat->has_mask = true;
   lat->initialized = false;
   return MLBM_OK;
@@ -622,6 +623,7 @@ mlbm_status mlbm_initialize(mlbm_lattice* lat) {
   if (st) return st;
   lat->compact.active = false;  // the initial state is written densely
   moments_reset(lat);
+  ++lat->changes;
   lat->phase = 0;
   lat->initialized = true;
   lat->vel_valid = false;
@@ -642,6 +644,7 @@ mlbm_status mlbm_iterate(mlbm_lattice* lat, int64_t step0, int32_t nsteps,
   if (nsteps == 0) return MLBM_OK;
   DeviceGuard restore_device;
   if (mlbm_status st = activate(lat)) return st;
+  ++lat->changes;
   switch (lat->storage) {
     case MLBM_STORE_F32:
       return launch_steps<float>(lat, step0, nsteps, reverse, inject_type, flags);

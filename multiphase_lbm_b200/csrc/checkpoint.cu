@@ -239,6 +239,7 @@ mlbm_status mlbm_checkpoint_load(mlbm_lattice* lat, const void* image,
   if (e == cudaSuccess) e = cudaStreamSynchronize(lat->stream);
   if (e != cudaSuccess) return cuda_err(e, "checkpoint load");
   compact_invalidate(lat);  // the fluid-only tables follow the new mask
+  ++lat->changes;
   lat->phase = h.phase;
   lat->has_mask = true;
   lat->has_rho = true;
