@@ -577,7 +577,7 @@ mlbm_status mlbm_batch_iterate(mlbm_batch* b, int32_t nsteps, int32_t reverse,
   mlbm::DeviceGuard restore_device;
   BCUDA(cudaSetDevice(b->device), "cudaSetDevice");
   // the domains' form: it follows a domain added or removed since, one whose
-  // tau came to or left 1, one advanced on its own
+  // parameters changed, one advanced on its own
   bool moments = false;
   if (mlbm_status st = moments_mode(b, &moments)) return st;
   if (moments != b->moments) b->dirty = true;

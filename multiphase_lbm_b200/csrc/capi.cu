@@ -539,6 +539,7 @@ mlbm_status mlbm_set_params(mlbm_lattice* lat, const mlbm_params* p) {
     return fail(MLBM_ERR_ARG, "Carnahan-Starling psi needs G != 0");
   lat->params = *p;
   lat->phys = to_phys(*p);
+  ++lat->changes;
   lat->has_params = true;
   return MLBM_OK;
 }

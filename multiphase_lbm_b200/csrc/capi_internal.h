@@ -91,7 +91,7 @@ struct mlbm_lattice {
   bool stall_test = false;  // the next step launch makes a wait run out
   int phase = 0;  // 0: post-collision at opp slots of own node; 1: pushed
   // counts the calls on this lattice after which a table made of its phase,
-  // layout and buffers (batch.cu) is out of date
+  // layout, buffers and parameters (batch.cu) is out of date
   unsigned long long changes = 0;
   bool slab = false;  // planes 0 and lz - 1 are halo planes (slab.cu)
   bool has_params = false, has_mask = false, has_rho = false;

@@ -1,7 +1,6 @@
 """Domains of a batch that change between its iterate calls: advanced on
 their own by any step kernel, given other parameters.  Every domain has the
 bits of the same domain advanced alone by the dense two-pass kernels."""
-import numpy as np
 import pytest
 
 from conftest import random_case
@@ -56,7 +55,9 @@ class Pair:
             for field in ("rho", "f"):
                 got = self.lattice(i).field(field, f64=self.storage == 2)
                 want = lat.field(field, f64=self.storage == 2)
-                assert np.array_equal(got, want), (i, field)
+                # bits: a change of rho_shift in FP16 storage moves every
+                # density, and may drive a domain to infinities and NaN
+                assert got.tobytes() == want.tobytes(), (i, field)
 
     def close(self):
         self.b.close()
@@ -84,4 +85,26 @@ def test_an_odd_number_of_steps_alone(storage, kernel, taus):
         t.own(0, 1)
         t.set(1, tau=1.0)
     t.run(2)
+    t.close()
+
+
+@pytest.mark.parametrize("storage", [0, 1, 2])
+@pytest.mark.parametrize("taus", [(1.0, 1.0), (1.0, 0.8)])
+def test_changed_parameters(storage, taus):
+    """What mlbm_set_params on a domain's lattice changes holds from the next
+    batch step on, as it does for a lattice alone."""
+    t = Pair(storage, taus)
+    t.run(10)
+    t.set(0, G=-4.5)
+    t.run(10)
+    t.set(1, rho_inlet=0.3)
+    t.set(0, rho_outlet=1.7)
+    t.run(3)
+    t.set(0, rho_increment=0.01, rho_inject_period=2, inject_position=0.6)
+    t.run(11)
+    t.set(1, rho_shift=0.5)
+    t.run(2)
+    if taus[1] != 1.0:
+        t.set(1, tau=1.1)
+        t.run(9)
     t.close()
