@@ -197,9 +197,9 @@ MOMENT_INFO = ("moments", "time step (k_mom_gather + k_mom_collide)", 2)
 
 def step_info(kernel, kernel_id):
     """(name, label, launches per step, bytes per fluid node by storage) of
-    the step that runs: at tau = 1 the compact kernel, and the two-pass one
-    where none was asked for, advance the lattice as moments."""
-    if PHYS["tau"] == 1.0 and (kernel == 3 or (kernel == 2 and kernel_id is None)):
+    the step that runs: at tau = 1 and with no kernel asked for, the lattice
+    advances as moments."""
+    if PHYS["tau"] == 1.0 and kernel_id is None:
         return MOMENT_INFO + (MOMENT_BYTES_PER_FLUID,)
     return KERNEL_INFO[kernel] + (BYTES_PER_FLUID,)
 

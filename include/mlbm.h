@@ -195,7 +195,14 @@ mlbm_status mlbm_iterate(mlbm_lattice* lat, int64_t step0, int32_t nsteps,
  *                allocated on first use.  Where even a band of one row does
  *                not fit shared memory (very long rows), the steps run as
  *                COMPACT;
- *   AUTO         (default) COMPACT where supported, else TWO_PASS.
+ *   AUTO         (default) COMPACT where supported, else TWO_PASS; at tau = 1
+ *                the moment step: with omega = 1 the collision leaves
+ *                f* = feq(rho, u), so the lattice is held as the 4 moments
+ *                of every fluid node and advanced by a gather and a collide
+ *                launch per step.  Any storage, whole lattices (not slabs),
+ *                at most 2048 x 2048 x 1024 nodes; bit-identical to the
+ *                kernels above.  Its buffers are allocated on first use;
+ *                where they are refused, the population kernels run.
  * (Values 1, 4 and 5 belonged to step kernels this library no longer has;
  * they are refused.)  The state moves between the layouts on demand (the
  * dense buffers stay allocated; the fluid-only layout adds 19 populations
@@ -205,7 +212,8 @@ mlbm_status mlbm_iterate(mlbm_lattice* lat, int64_t step0, int32_t nsteps,
 #define MLBM_KERNEL_COMPACT 3
 #define MLBM_KERNEL_BAND 6
 mlbm_status mlbm_set_step_kernel(mlbm_lattice* lat, int32_t kind);
-/* The kernel the next mlbm_iterate runs (AUTO resolved); -1 for NULL. */
+/* The kernel the next mlbm_iterate runs (AUTO resolved to the population
+ * kernel, which at tau = 1 stands back for the moment step); -1 for NULL. */
 int32_t mlbm_get_step_kernel(const mlbm_lattice* lat);
 /* Tiling of the BAND step: bands of at most `rows` rows (y, 1..64; fewer
  * where the staged rows would not fit shared memory) and chunks of about

@@ -496,13 +496,9 @@ mlbm_status mlbm_batch_add(mlbm_batch* b, int32_t nx, int32_t ny, int32_t nz,
   mlbm_lattice* lat = nullptr;
   if (mlbm_status st = mlbm_lattice_create(nx, ny, nz, b->storage, b->device, &lat))
     return st;
-  // a domain advanced on its own (mlbm_iterate on its lattice) uses the
-  // kernels bit-identical to the batch's: the compact two-pass step where the
-  // compact kernels fit, else the dense two-pass step
+  // a domain advanced on its own (mlbm_iterate on its lattice) stays with AUTO,
+  // whose kernels are bit-identical to the batch's
   mlbm_status st = mlbm_set_stream(lat, b->stream);
-  if (!st)
-    st = mlbm_set_step_kernel(lat, lat->compact.two_pass_ok ? MLBM_KERNEL_COMPACT
-                                                           : MLBM_KERNEL_TWO_PASS);
   if (!st) st = mlbm_set_params(lat, params);
   if (!st) st = mlbm_upload_fluid_mask(lat, is_fluid);
   if (!st) st = mlbm_upload_rho(lat, rho);
@@ -531,9 +527,6 @@ mlbm_status mlbm_batch_add_checkpoint(mlbm_batch* b, const void* image,
                                            b->device, &lat))
     return st;
   mlbm_status st = mlbm_set_stream(lat, b->stream);
-  if (!st)
-    st = mlbm_set_step_kernel(lat, lat->compact.two_pass_ok ? MLBM_KERNEL_COMPACT
-                                                           : MLBM_KERNEL_TWO_PASS);
   if (!st) st = mlbm_checkpoint_load(lat, image, bytes, &step0);
   if (st) {
     mlbm_lattice_destroy(lat);

@@ -217,11 +217,12 @@ mlbm_status launch_two_pass(mlbm_lattice* lat, const StepArgs& a, bool wu,
   return MLBM_OK;
 }
 
-// One lattice step per launch (two launches for the two-pass kernels, which
-// AUTO selects).  rho is written on the last step of each mlbm_iterate call
-// (the field the caller can read afterwards).
-// The step kernel a lattice runs: AUTO is the compact two-pass step where it
-// supports the lattice (FP32 / FP16 storage), else the dense two-pass step.
+// One lattice step per launch (two launches for the two-pass kernels).  rho is
+// written on the last step of each mlbm_iterate call (the field the caller can
+// read afterwards).
+// The population kernel a lattice runs: AUTO is the compact two-pass step where
+// it supports the lattice (FP32 / FP16 storage), else the dense two-pass step;
+// at tau = 1 AUTO takes the moment step before either (launch_steps).
 int effective_kernel(const mlbm_lattice* lat) {
   if (lat->step_kernel != MLBM_KERNEL_AUTO) return lat->step_kernel;
   return lat->compact.two_pass_ok ? MLBM_KERNEL_COMPACT : MLBM_KERNEL_TWO_PASS;
@@ -246,16 +247,13 @@ mlbm_status launch_steps(mlbm_lattice* lat, int64_t step0, int32_t nsteps,
                              lat->stream),
              "velocity clear");
   }
-  // tau = 1 and no kernel asked for that holds populations: the moment step.
-  // Where its buffers do not fit the device, the population kernels run.
+  // tau = 1 and no kernel asked for: the moment step.  Where its buffers do not
+  // fit the device, the population kernels run.
   bool moments = false;
-  if ((compact && !band) ||
-      (lat->step_kernel == MLBM_KERNEL_AUTO && kind == MLBM_KERNEL_TWO_PASS)) {
-    if (moments_apply(lat)) {
-      const mlbm_status st = moments_prepare(lat);
-      if (st && st != MLBM_ERR_NOMEM) return st;
-      moments = st == MLBM_OK;
-    }
+  if (lat->step_kernel == MLBM_KERNEL_AUTO && moments_apply(lat)) {
+    const mlbm_status st = moments_prepare(lat);
+    if (st && st != MLBM_ERR_NOMEM) return st;
+    moments = st == MLBM_OK;
   }
   if (moments) {
     if (lat->compact.active)

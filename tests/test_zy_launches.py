@@ -1,0 +1,44 @@
+"""Which step kernels run: a kernel that the caller asks for is the one that
+advances the lattice, at tau = 1 too; AUTO takes the moment step there.
+
+The launches are read from torch's profiler, which may leave later launches of
+the process slower: this file is named to be collected after the others."""
+import pytest
+
+from conftest import random_case
+
+pytestmark = pytest.mark.gpu
+
+
+def _launched(run):
+    """Names of the library's kernels that `run` launches, with repeats."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        run()
+        torch.cuda.synchronize()
+    return [e.name for e in p.events() if "mlbm" in e.name]
+
+
+@pytest.mark.parametrize("storage,kernel,tau,want", [
+    (0, "AUTO", 1.0, "k_mom_collide"), (1, "AUTO", 1.0, "k_mom_collide"),
+    (2, "AUTO", 1.0, "k_mom_collide"), (0, "AUTO", 0.8, "k_cupdate"),
+    (2, "AUTO", 0.8, "k_update_zm"), (0, "COMPACT", 1.0, "k_cupdate"),
+    (1, "COMPACT", 1.0, "k_cupdate"), (0, "TWO_PASS", 1.0, "k_update_zm"),
+    (2, "TWO_PASS", 1.0, "k_update_zm"), (0, "BAND", 1.0, "k_band")])
+def test_the_kernel_asked_for_runs(storage, kernel, tau, want):
+    from multiphase_lbm_b200 import capi
+    shape = (40, 18, 11)
+    fluid, rho = random_case(shape, seed=1, rho0=1.2, amp=0.3)
+    lat = capi.Lattice(shape, storage=storage)
+    lat.set_step_kernel(getattr(capi, "KERNEL_" + kernel))
+    lat.set_params(capi.default_params(G=-5.0, rhos=0.2, tau=tau))
+    lat.upload(fluid, rho)
+    lat.initialize()
+    lat.iterate(0, 1)
+    names = _launched(lambda: lat.iterate(1, 3))
+    updates = [n for n in names for k in ("k_mom_collide", "k_cupdate", "k_update_zm",
+                                          "k_band") if k in n]
+    assert len(updates) == 3 and all(want in n for n in updates), names
+    lat.close()
