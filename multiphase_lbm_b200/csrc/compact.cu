@@ -442,8 +442,9 @@ mlbm_status launch_compact_band(mlbm_lattice* lat, const StepArgs& a,
   if (lat->phase != 1)
     return set_error(MLBM_ERR_STATE, "one-pass step needs the AA phase-1 state");
   if (!c.cpop_alt) {
+    // as large as cpop, which later masks of up to cap slots reuse
     const cudaError_t e =
-        cudaMalloc(&c.cpop_alt, (size_t)c.cs * Q * pop_elem_bytes(lat->storage));
+        cudaMalloc(&c.cpop_alt, (size_t)c.cap * Q * pop_elem_bytes(lat->storage));
     if (e != cudaSuccess) {
       c.cpop_alt = nullptr;
       cudaGetLastError();
