@@ -202,7 +202,9 @@ mlbm_status mlbm_iterate(mlbm_lattice* lat, int64_t step0, int32_t nsteps,
  *                launch per step.  Any storage, whole lattices (not slabs),
  *                at most 2048 x 2048 x 1024 nodes; bit-identical to the
  *                kernels above.  Its buffers are allocated on first use;
- *                where they are refused, the population kernels run.
+ *                where they are refused, or have to make room for another
+ *                buffer of the lattice, the population kernels run until
+ *                the next mlbm_initialize.
  * (Values 1, 4 and 5 belonged to step kernels this library no longer has;
  * they are refused.)  The state moves between the layouts on demand (the
  * dense buffers stay allocated; the fluid-only layout adds 19 populations
@@ -242,6 +244,10 @@ mlbm_status mlbm_set_wait_limit(mlbm_lattice* lat, uint64_t ns);
  * a barrier that nothing completes, so the limit runs out (MLBM_ERR_STATE
  * for other step kernels).  The lattice must be initialised again after. */
 mlbm_status mlbm_test_stall_wait(mlbm_lattice* lat);
+/* Testing refused allocations: from now on an allocation that would bring
+ * the lattice above `bytes` of device memory is refused as the device refuses
+ * one (0: no limit).  Returns the device bytes that the lattice holds. */
+uint64_t mlbm_test_memory_limit(mlbm_lattice* lat, uint64_t bytes);
 /* Wait for the lattice's stream and report a device-side failure (a bounded
  * wait of a step kernel that ran out: MLBM_ERR_TIMEOUT; the
  * lattice must then be initialised again). */

@@ -117,6 +117,7 @@ SIGNATURES = [
     ("mlbm_set_band_shape", C.c_int, [_VP, C.c_int32, C.c_int32]),
     ("mlbm_set_wait_limit", C.c_int, [_VP, C.c_uint64]),
     ("mlbm_test_stall_wait", C.c_int, [_VP]),
+    ("mlbm_test_memory_limit", C.c_uint64, [_VP, C.c_uint64]),
     ("mlbm_get_step_kernel", C.c_int32, [_VP]),
     ("mlbm_autotune", C.c_int, [_VP, C.c_int64, C.c_int32, _VP, _VP]),
     ("mlbm_set_slab", C.c_int, [_VP, C.c_int32]),
@@ -257,6 +258,11 @@ class Lattice:
     def test_stall_wait(self) -> None:
         """Make one wait of the next BAND launch run out (testing)."""
         check(lib().mlbm_test_stall_wait(self.h))
+
+    def test_memory_limit(self, nbytes: int = 0) -> int:
+        """Refuse allocations that would bring the lattice above `nbytes` of
+        device memory (0: none); returns the bytes it holds."""
+        return int(lib().mlbm_test_memory_limit(self.h, nbytes))
 
     def set_band_shape(self, rows: int = 4, planes: int = 24) -> None:
         """Tiling of KERNEL_BAND: rows per band (y) and planes per chunk (z)."""

@@ -52,6 +52,34 @@ mlbm_status cuda_fail(cudaError_t e, const char* where) {
   return fail(MLBM_ERR_CUDA, "%s: %s", where, cudaGetErrorString(e));
 }
 
+size_t held_bytes(const mlbm_lattice* lat) {
+  const CompactState& c = lat->compact;
+  return lat->buffer_bytes +
+         (lat->vel ? (size_t)lat->g.plane * 3 * sizeof(float) : 0) +
+         lat->staging_bytes + lat->stats_scratch_bytes + c.table_bytes +
+         c.pop_bytes + c.alt_bytes + lat->mom.buffer_bytes;
+}
+
+cudaError_t lattice_try_malloc(const mlbm_lattice* lat, void** p, size_t bytes) {
+  *p = nullptr;
+  if (lat->memory_limit && held_bytes(lat) + bytes > lat->memory_limit)
+    return cudaErrorMemoryAllocation;
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) {
+    *p = nullptr;
+    cudaGetLastError();
+  }
+  return e;
+}
+
+cudaError_t lattice_malloc(mlbm_lattice* lat, void** p, size_t bytes) {
+  const cudaError_t e = lattice_try_malloc(lat, p, bytes);
+  if (e != cudaErrorMemoryAllocation || !lat->mom.buffer) return e;
+  if (moments_release(lat) != MLBM_OK) return e;
+  lat->mom.no_room = true;
+  return lattice_try_malloc(lat, p, bytes);
+}
+
 void prefault(void* p, size_t bytes) {
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
@@ -240,7 +268,8 @@ mlbm_status launch_steps(mlbm_lattice* lat, int64_t step0, int32_t nsteps,
   }
   if ((flags & MLBM_ITER_WRITE_VELOCITY) && !lat->vel) {
     // the velocity field is allocated on first request
-    CUDA_TRY(cudaMalloc((void**)&lat->vel, (size_t)lat->g.plane * 3 * sizeof(float)),
+    CUDA_TRY(lattice_malloc(lat, (void**)&lat->vel,
+                            (size_t)lat->g.plane * 3 * sizeof(float)),
              "velocity allocation");
     // solid nodes are never written: they read zero velocity
     CUDA_TRY(cudaMemsetAsync(lat->vel, 0, (size_t)lat->g.plane * 3 * sizeof(float),
@@ -381,7 +410,7 @@ mlbm_status ensure_staging(mlbm_lattice* lat, size_t bytes) {
   if (lat->staging) cudaFree(lat->staging);
   lat->staging = nullptr;
   lat->staging_bytes = 0;
-  CUDA_TRY(cudaMalloc(&lat->staging, bytes), "staging allocation");
+  CUDA_TRY(lattice_malloc(lat, &lat->staging, bytes), "staging allocation");
   lat->staging_bytes = bytes;
   return MLBM_OK;
 }
@@ -473,9 +502,10 @@ mlbm_status mlbm_lattice_create(int32_t lx, int32_t ly, int32_t lz,
   const size_t mask_bytes = up(mask_words * sizeof(uint32_t));
   const size_t words_bytes = up(2 * mask_words * sizeof(uint32_t));
   const size_t zeros = psi_bytes + init_bytes + mask_bytes + up(sizeof(int));
-  cudaError_t e =
-      cudaMalloc(&lat->buffer, pop_bytes + rho_bytes + nbw_bytes + words_bytes + zeros);
+  const size_t bytes = pop_bytes + rho_bytes + nbw_bytes + words_bytes + zeros;
+  cudaError_t e = cudaMalloc(&lat->buffer, bytes);
   if (e == cudaSuccess) {
+    lat->buffer_bytes = bytes;
     char* at = static_cast<char*>(lat->buffer);
     lat->pop = at;
     lat->rho = at += pop_bytes;
@@ -729,7 +759,7 @@ mlbm_status stats_enqueue(mlbm_lattice* lat, double* h, bool full) {
     cudaFree(lat->stats_scratch);
     lat->stats_scratch = nullptr;
     lat->stats_scratch_bytes = 0;
-    CUDA_TRY(cudaMalloc((void**)&lat->stats_scratch, need), "stats scratch");
+    CUDA_TRY(lattice_malloc(lat, (void**)&lat->stats_scratch, need), "stats scratch");
     CUDA_TRY(cudaMemsetAsync(lat->stats_scratch, 0, kStatCounters * sizeof(double),
                              lat->stream),
              "stats counter");
@@ -906,6 +936,12 @@ mlbm_status mlbm_test_stall_wait(mlbm_lattice* lat) {
                 "(select MLBM_KERNEL_BAND)");
   lat->stall_test = true;
   return MLBM_OK;
+}
+
+uint64_t mlbm_test_memory_limit(mlbm_lattice* lat, uint64_t bytes) {
+  if (!lat) return 0;
+  lat->memory_limit = (size_t)bytes;
+  return held_bytes(lat);
 }
 
 mlbm_status mlbm_set_band_shape(mlbm_lattice* lat, int32_t rows,

@@ -25,6 +25,7 @@ struct CompactState {
   bool two_pass_ok = false;    // the compact kernels fit the lattice
   uint32_t* wbase = nullptr;   // [rows * wpr + 1]
   long long cap = 0;           // cs the buffers were allocated for
+  size_t table_bytes = 0, pop_bytes = 0, alt_bytes = 0;  // of wbase, cpop, cpop_alt
   std::vector<long long> plane_start;  // [lz + 1] first compact index of each plane
   std::vector<uint32_t> row_start;     // [lz * ly + 1] first compact index of each row
   // one-pass step (band.cuh): the second population buffer and the tiling
@@ -65,6 +66,8 @@ struct mlbm_lattice {
   bool stream_owned_sync = true;
 
   void* buffer = nullptr;       // one allocation for pop .. nbw and err
+  size_t buffer_bytes = 0;
+  size_t memory_limit = 0;      // mlbm_test_memory_limit; 0: none
   void* pop = nullptr;          // 19 planes of g.plane elements (T)
   void* rho = nullptr;          // density, R per node
   void* psi = nullptr;          // pseudopotential, R per node
@@ -101,6 +104,14 @@ struct mlbm_lattice {
 
 namespace mlbm {
 mlbm_status cuda_fail(cudaError_t e, const char* where);
+// Device bytes a lattice holds.
+size_t held_bytes(const mlbm_lattice* lat);
+// Device memory for a lattice.  Where it is refused while the lattice holds
+// the moment step's buffers, lattice_malloc gives those back (the lattice then
+// runs on populations) and asks again: they are there for speed, and what ran
+// without them must run beside them.
+cudaError_t lattice_try_malloc(const mlbm_lattice* lat, void** p, size_t bytes);
+cudaError_t lattice_malloc(mlbm_lattice* lat, void** p, size_t bytes);
 size_t pop_elem_bytes(int storage);
 size_t real_bytes(int storage);
 Geom make_geom(int lx, int ly, int lz);
@@ -140,6 +151,7 @@ mlbm_status launch_moment_step(mlbm_lattice* lat, const StepArgs& a,
                                bool write_u, bool write_rho);
 mlbm_status moments_sync_dense(mlbm_lattice* lat);   // dense copy, stay
 mlbm_status moments_leave(mlbm_lattice* lat);        // moments -> dense state
+mlbm_status moments_release(mlbm_lattice* lat);      // leave; buffers freed
 void moments_reset(mlbm_lattice* lat);  // a new mask or initial state
 void moments_free(mlbm_lattice* lat);
 mlbm_status compact_set_band_shape(mlbm_lattice* lat, int rows, int planes);

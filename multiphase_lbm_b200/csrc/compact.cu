@@ -41,12 +41,15 @@ mlbm_status build_tables(mlbm_lattice* lat) {
   cudaFree(c.wbase);
   c.wbase = nullptr;
   c.wtab = nullptr;
+  c.table_bytes = 0;
   // wbase and wtab are one allocation, and so are cpop and cinfo below: apart
   // they cost the first pass on a new lattice 0.4-0.7 ms more (200 x 150 x 170
   // FP16 2.8 -> 2.1 ms, 160 x 144 x 128 FP32 2.4 -> 2.0)
   const size_t wbase_bytes = ((nwords + 1) * sizeof(uint32_t) + 255) / 256 * 256;
-  e = cudaMalloc((void**)&c.wbase, wbase_bytes + (nwords + 1) * sizeof(uint2));
+  const size_t table_bytes = wbase_bytes + (nwords + 1) * sizeof(uint2);
+  e = lattice_malloc(lat, (void**)&c.wbase, table_bytes);
   if (e != cudaSuccess) return cuda_fail(e, "compact tables");
+  c.table_bytes = table_bytes;
   c.wtab = reinterpret_cast<uint2*>(reinterpret_cast<char*>(c.wbase) + wbase_bytes);
   k_word_counts<<<(unsigned)((nwords + 255) / 256), 256, 0, lat->stream>>>(
       lat->mask, c.wbase, nwords);
@@ -95,14 +98,13 @@ mlbm_status build_tables(mlbm_lattice* lat) {
     c.cpop_alt = nullptr;
     c.cinfo = nullptr;
     c.cap = 0;
+    c.pop_bytes = c.alt_bytes = 0;
     const size_t pop_bytes =
         ((size_t)c.cs * Q * pop_elem_bytes(lat->storage) + 255) / 256 * 256;
-    e = cudaMalloc(&c.cpop, pop_bytes + (size_t)c.cs * sizeof(uint2));
-    if (e != cudaSuccess) {
-      c.cpop = nullptr;
-      cudaGetLastError();
-      return cuda_fail(e, "compact buffers");
-    }
+    const size_t bytes = pop_bytes + (size_t)c.cs * sizeof(uint2);
+    e = lattice_malloc(lat, &c.cpop, bytes);
+    if (e != cudaSuccess) return cuda_fail(e, "compact buffers");
+    c.pop_bytes = bytes;
     c.cinfo = reinterpret_cast<uint2*>(static_cast<char*>(c.cpop) + pop_bytes);
     c.cap = c.cs;
   }
@@ -443,13 +445,10 @@ mlbm_status launch_compact_band(mlbm_lattice* lat, const StepArgs& a,
     return set_error(MLBM_ERR_STATE, "one-pass step needs the AA phase-1 state");
   if (!c.cpop_alt) {
     // as large as cpop, which later masks of up to cap slots reuse
-    const cudaError_t e =
-        cudaMalloc(&c.cpop_alt, (size_t)c.cap * Q * pop_elem_bytes(lat->storage));
-    if (e != cudaSuccess) {
-      c.cpop_alt = nullptr;
-      cudaGetLastError();
-      return cuda_fail(e, "one-pass step buffer");
-    }
+    const size_t bytes = (size_t)c.cap * Q * pop_elem_bytes(lat->storage);
+    const cudaError_t e = lattice_malloc(lat, &c.cpop_alt, bytes);
+    if (e != cudaSuccess) return cuda_fail(e, "one-pass step buffer");
+    c.alt_bytes = bytes;
   }
   const BandShape s = fit_band_shape<T>(lat, c.band_rows, c.band_planes);
   if (s.nb == 0)

@@ -30,7 +30,7 @@ mlbm_status build_list(mlbm_lattice* lat) {
   char* own = nullptr;
   char* buf = static_cast<char*>(lat->staging);
   if (lat->staging_bytes < counts_bytes + temp_bytes) {
-    e = cudaMalloc((void**)&own, counts_bytes + temp_bytes);
+    e = lattice_try_malloc(lat, (void**)&own, counts_bytes + temp_bytes);
     if (e != cudaSuccess) return cuda_fail(e, "moment lists");
     buf = own;
   }
@@ -56,9 +56,8 @@ mlbm_status build_list(mlbm_lattice* lat) {
     cudaFree(s.buffer);
     s.buffer = nullptr;
     s.buffer_bytes = 0;
-    e = cudaMalloc(&s.buffer, need);
+    e = lattice_try_malloc(lat, &s.buffer, need);
     if (e == cudaSuccess) s.buffer_bytes = need;
-    else s.buffer = nullptr;
   }
   if (e == cudaSuccess) {
     char* at = static_cast<char*>(s.buffer);
@@ -204,6 +203,16 @@ mlbm_status moments_leave(mlbm_lattice* lat) {
         static_cast<const float*>(lat->mom.psi), static_cast<float*>(lat->psi), g);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "psi of the moments");
+  return MLBM_OK;
+}
+
+mlbm_status moments_release(mlbm_lattice* lat) {
+  MomentState& s = lat->mom;
+  if (!s.buffer) return MLBM_OK;
+  if (mlbm_status st = moments_leave(lat)) return st;
+  const cudaError_t e = cudaStreamSynchronize(lat->stream);
+  if (e != cudaSuccess) return cuda_fail(e, "moment buffers");
+  moments_free(lat);
   return MLBM_OK;
 }
 

@@ -222,7 +222,7 @@ mlbm_status mlbm_step_pass(mlbm_lattice* lat, int64_t step, int32_t pass,
   if (wu && !lat->vel) {
     // the velocity field is allocated on first request; solid nodes read 0
     const size_t bytes = (size_t)lat->g.plane * 3 * sizeof(float);
-    cudaError_t e = cudaMalloc((void**)&lat->vel, bytes);
+    cudaError_t e = lattice_malloc(lat, (void**)&lat->vel, bytes);
     if (e == cudaSuccess) e = cudaMemsetAsync(lat->vel, 0, bytes, lat->stream);
     if (e != cudaSuccess) return slab_cuda(e, "velocity allocation");
   }
