@@ -93,17 +93,44 @@ const void* pick_update(int storage) {
                                      : update_fn<double>();
 }
 
+// Give back the moment buffers of every domain; whether any held some.
+mlbm_status release_moments(mlbm_batch* b, bool* some) {
+  *some = false;
+  for (mlbm_lattice* lat : b->dom) {
+    if (!lat || !lat->mom.buffer) continue;
+    *some = true;
+    if (mlbm_status st = moments_release(lat)) return st;
+  }
+  return MLBM_OK;
+}
+
+// Every domain into the fluid-only layout; where that is refused beside moment
+// buffers, they make room.
+mlbm_status enter_compact(mlbm_batch* b) {
+  for (;;) {
+    mlbm_status st = MLBM_OK;
+    for (mlbm_lattice* lat : b->dom) {
+      if (lat) st = compact_enter(lat);
+      if (st) break;
+    }
+    bool some = false;
+    if (st != MLBM_ERR_NOMEM) return st;
+    if (mlbm_status rs = release_moments(b, &some)) return rs;
+    if (!some) return st;
+  }
+}
+
 // Compact mode: every domain enters the fluid-only layout; block prefixes for
 // both step parities (one node per thread in the gather step, one pair per
 // thread in the local step).
 mlbm_status rebuild_compact(mlbm_batch* b) {
+  if (mlbm_status st = enter_compact(b)) return st;
   std::vector<CDomain> desc;
   std::vector<long long> pre[2] = {std::vector<long long>(1, 0),
                                    std::vector<long long>(1, 0)};
   for (size_t s = 0; s < b->dom.size(); ++s) {
     mlbm_lattice* lat = b->dom[s];
     if (!lat) continue;
-    if (mlbm_status st = compact_enter(lat)) return st;
     const CompactState& c = lat->compact;
     CDomain d;
     std::memset(&d, 0, sizeof d);
@@ -185,7 +212,8 @@ mlbm_status rebuild_moments(mlbm_batch* b) {
 }
 
 // Whether every domain can be held as moments; builds their lists and
-// buffers.  Where one's do not fit the device, none is.
+// buffers.  Where one's do not fit the device, none is, and the others' are
+// given back: the populations' buffers need the room.
 mlbm_status moments_mode(mlbm_batch* b, bool* on) {
   *on = false;
   for (const mlbm_lattice* lat : b->dom)
@@ -193,7 +221,8 @@ mlbm_status moments_mode(mlbm_batch* b, bool* on) {
   for (mlbm_lattice* lat : b->dom)
     if (lat) {
       const mlbm_status st = moments_prepare(lat);
-      if (st == MLBM_ERR_NOMEM) return MLBM_OK;
+      bool some;
+      if (st == MLBM_ERR_NOMEM) return release_moments(b, &some);
       if (st) return st;
     }
   *on = true;
@@ -438,6 +467,30 @@ int32_t insert_domain(mlbm_batch* b, mlbm_lattice* lat, int64_t step0) {
   b->dirty = true;
   return slot;
 }
+
+// Create a lattice and set it up on the batch's stream.  Where the device
+// refuses its memory beside the moment buffers of the batch, they make room.
+template <typename SetUp>
+mlbm_status make_domain(mlbm_batch* b, int nx, int ny, int nz, SetUp set_up,
+                        mlbm_lattice** out) {
+  for (;;) {
+    mlbm_lattice* lat = nullptr;
+    mlbm_status st = mlbm_lattice_create(nx, ny, nz, b->storage, b->device, &lat);
+    // (a domain advanced on its own -- mlbm_iterate on its lattice -- stays with
+    // AUTO, whose kernels are bit-identical to the batch's)
+    if (!st) st = mlbm_set_stream(lat, b->stream);
+    if (!st) st = set_up(lat);
+    if (!st) {
+      *out = lat;
+      return MLBM_OK;
+    }
+    mlbm_lattice_destroy(lat);
+    bool some = false;
+    if (st == MLBM_ERR_NOMEM)
+      if (mlbm_status rs = release_moments(b, &some)) return rs;
+    if (!some) return st;
+  }
+}
 }  // namespace
 
 extern "C" {
@@ -494,19 +547,14 @@ mlbm_status mlbm_batch_add(mlbm_batch* b, int32_t nx, int32_t ny, int32_t nz,
   mlbm::DeviceGuard restore_device;
   BCUDA(cudaSetDevice(b->device), "cudaSetDevice");
   mlbm_lattice* lat = nullptr;
-  if (mlbm_status st = mlbm_lattice_create(nx, ny, nz, b->storage, b->device, &lat))
+  auto set_up = [&](mlbm_lattice* l) {
+    mlbm_status st = mlbm_set_params(l, params);
+    if (!st) st = mlbm_upload_fluid_mask(l, is_fluid);
+    if (!st) st = mlbm_upload_rho(l, rho);
+    if (!st) st = mlbm_initialize(l);
     return st;
-  // a domain advanced on its own (mlbm_iterate on its lattice) stays with AUTO,
-  // whose kernels are bit-identical to the batch's
-  mlbm_status st = mlbm_set_stream(lat, b->stream);
-  if (!st) st = mlbm_set_params(lat, params);
-  if (!st) st = mlbm_upload_fluid_mask(lat, is_fluid);
-  if (!st) st = mlbm_upload_rho(lat, rho);
-  if (!st) st = mlbm_initialize(lat);
-  if (st) {
-    mlbm_lattice_destroy(lat);
-    return st;
-  }
+  };
+  if (mlbm_status st = make_domain(b, nx, ny, nz, set_up, &lat)) return st;
   *id = insert_domain(b, lat, step0);
   return MLBM_OK;
 }
@@ -523,15 +571,11 @@ mlbm_status mlbm_batch_add_checkpoint(mlbm_batch* b, const void* image,
   mlbm::DeviceGuard restore_device;
   BCUDA(cudaSetDevice(b->device), "cudaSetDevice");
   mlbm_lattice* lat = nullptr;
-  if (mlbm_status st = mlbm_lattice_create(dims[0], dims[1], dims[2], b->storage,
-                                           b->device, &lat))
+  auto set_up = [&](mlbm_lattice* l) {
+    return mlbm_checkpoint_load(l, image, bytes, &step0);
+  };
+  if (mlbm_status st = make_domain(b, dims[0], dims[1], dims[2], set_up, &lat))
     return st;
-  mlbm_status st = mlbm_set_stream(lat, b->stream);
-  if (!st) st = mlbm_checkpoint_load(lat, image, bytes, &step0);
-  if (st) {
-    mlbm_lattice_destroy(lat);
-    return st;
-  }
   *id = insert_domain(b, lat, step0);
   return MLBM_OK;
 }

@@ -111,3 +111,96 @@ def test_refused_moments_leave_the_population_kernels(storage):
     _same(a, b)
     a.close()
     b.close()
+
+
+def _batch(capi, storage, tau1=1.0):
+    from multiphase_lbm_b200 import batch
+    b = batch.Batch(storage=storage)
+    ids, alone = [], []
+    for i in range(2):
+        fluid, rho = sphere_case(SHAPE, seed=9 + i, rmin=2.0, rmax=5.0, porosity=0.5,
+                                 rho0=1.2, amp=0.4)
+        p = capi.default_params(tau=tau1 if i else 1.0, **KW)
+        ids.append(b.add(fluid, rho, p))
+        lat = capi.Lattice(SHAPE, storage=storage)
+        lat.set_step_kernel(capi.KERNEL_TWO_PASS)
+        lat.set_params(p)
+        lat.upload(fluid, rho)
+        lat.initialize()
+        alone.append(lat)
+    return b, ids, alone
+
+
+def _run(b, ids, alone, step, n):
+    b.iterate(n)
+    for did, lat in zip(ids, alone):
+        lat.iterate(step, n)
+        _same(b.lattice(did), lat, ("rho",))
+    return step + n
+
+
+@pytest.mark.parametrize("storage", [1, 2])
+def test_a_batch_whose_moments_are_refused_keeps_none(storage):
+    from multiphase_lbm_b200 import capi
+    mom = _grown(capi, storage, 0)
+    layout = _grown(capi, storage, capi.KERNEL_COMPACT) if storage == 1 else 0
+    b, ids, alone = _batch(capi, storage)
+    first, second = (b.lattice(i) for i in ids)
+    held = first.test_memory_limit()
+    # the second domain's packing differs by less than its moments' half
+    second.test_memory_limit(second.test_memory_limit() + layout + (mom - layout) // 2)
+    step = _run(b, ids, alone, 0, 5)
+    step = _run(b, ids, alone, step, 9)
+    assert first.test_memory_limit() == held + layout
+    b.remove(ids.pop())
+    alone.pop().close()
+    _run(b, ids, alone, step, 3)  # alone again, it is held as moments
+    assert first.test_memory_limit() == held + layout + mom
+    b.close()
+
+
+@pytest.mark.parametrize("storage", [0, 1])
+def test_a_batch_that_leaves_tau_1_makes_room(storage):
+    """The second domain is refused its populations' layout: the first one's
+    moments go, and the call fails; it goes on once there is room."""
+    from multiphase_lbm_b200 import capi
+    layout = _grown(capi, storage, capi.KERNEL_COMPACT)
+    b, ids, alone = _batch(capi, storage)
+    first, second = (b.lattice(i) for i in ids)
+    held = first.test_memory_limit()
+    step = _run(b, ids, alone, 0, 4)
+    for lat in (second, alone[1]):
+        lat.set_params(capi.default_params(tau=0.8, **KW))
+    second.test_memory_limit(held)
+    with pytest.raises(capi.MlbmError, match="NOMEM"):
+        b.iterate(3)
+    assert first.test_memory_limit() == held + layout
+    second.test_memory_limit()
+    step = _run(b, ids, alone, step, 3)
+    assert b.domain_step(ids[0]) == step
+    b.close()
+
+
+def test_a_domain_that_does_not_fit_takes_the_batchs_moments_first():
+    import ctypes as C
+
+    import numpy as np
+
+    from multiphase_lbm_b200 import batch, capi
+    b, ids, alone = _batch(capi, 2)
+    first = b.lattice(ids[0])
+    held = first.test_memory_limit()
+    step = _run(b, ids, alone, 0, 4)
+    grown = first.test_memory_limit()
+    assert grown > held
+    # 1280^3 FP64 nodes take 369 GB: refused before an array is read
+    one = np.ones(1, np.float32)
+    did = C.c_int32()
+    p = capi.default_params(**KW)
+    st = batch.blib().mlbm_batch_add(b.h, 1280, 1280, 1280, C.byref(p),
+                                     one.ctypes.data, one.ctypes.data, 0, C.byref(did))
+    assert st == 3  # MLBM_ERR_NOMEM
+    assert first.test_memory_limit() == held
+    _run(b, ids, alone, step, 4)
+    assert first.test_memory_limit() == grown
+    b.close()
