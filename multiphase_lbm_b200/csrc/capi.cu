@@ -404,13 +404,18 @@ mlbm_status check_device_error(mlbm_lattice* lat) {
 
 mlbm_status ensure_staging(mlbm_lattice* lat, size_t bytes) {
   if (lat->staging_bytes >= bytes) return MLBM_OK;
-  // room for a scalar field at once: mask, density and result follow
+  // room for a scalar field at once where there is any (mask, density and
+  // result follow), else for what is asked
   const Geom& g = lat->g;
-  bytes = std::max(bytes, (size_t)g.lx * g.ly * g.lz * real_bytes(lat->storage));
+  const size_t field =
+      std::max(bytes, (size_t)g.lx * g.ly * g.lz * real_bytes(lat->storage));
   if (lat->staging) cudaFree(lat->staging);
   lat->staging = nullptr;
   lat->staging_bytes = 0;
-  CUDA_TRY(lattice_malloc(lat, &lat->staging, bytes), "staging allocation");
+  cudaError_t e = lattice_try_malloc(lat, &lat->staging, field);
+  if (e == cudaSuccess) bytes = field;
+  else if (e == cudaErrorMemoryAllocation) e = lattice_malloc(lat, &lat->staging, bytes);
+  CUDA_TRY(e, "staging allocation");
   lat->staging_bytes = bytes;
   return MLBM_OK;
 }

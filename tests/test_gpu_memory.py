@@ -204,3 +204,24 @@ def test_a_domain_that_does_not_fit_takes_the_batchs_moments_first():
     _run(b, ids, alone, step, 4)
     assert first.test_memory_limit() == grown
     b.close()
+
+
+@pytest.mark.parametrize("storage", [0, 1, 2])
+def test_a_small_transfer_needs_no_room_for_a_field(storage):
+    """A restored lattice has no transfer buffer yet: the profile's few bytes
+    per plane, and the fluid mask, fit where a field does not."""
+    import numpy as np
+
+    from multiphase_lbm_b200 import capi
+    ref = _lattice(capi, storage)
+    ref.iterate(0, 2)
+    lat = capi.Lattice(SHAPE, storage=storage)
+    lat.restore(ref.checkpoint(2))
+    nodes = SHAPE[0] * SHAPE[1] * SHAPE[2]
+    lat.test_memory_limit(lat.test_memory_limit() + 16 * SHAPE[0])
+    for got, want in zip(lat.plane_profile(), ref.plane_profile()):
+        assert np.array_equal(got, want)
+    lat.test_memory_limit(lat.test_memory_limit() + nodes - 16 * SHAPE[0])
+    assert np.array_equal(lat.field("fluid"), ref.field("fluid"))
+    lat.close()
+    ref.close()
