@@ -136,12 +136,17 @@ const char* mlbm_last_error(void);
 void mlbm_d3q19(int32_t* e, float* w);
 
 /* Create a lattice of nx*ny*nz nodes on `device` with the given storage.
- * Allocates all device memory up front (MLBM_ERR_NOMEM if refused). */
+ * Allocates its fields (MLBM_ERR_NOMEM if refused); the buffers of the step
+ * kernels, of transfers and of the velocity field come on first use. */
 mlbm_status mlbm_lattice_create(int32_t nx, int32_t ny, int32_t nz,
                                 int32_t storage, int32_t device,
                                 mlbm_lattice** out);
 mlbm_status mlbm_lattice_destroy(mlbm_lattice* lat);
-/* Device bytes held by a lattice of this size and storage (no allocation). */
+/* Device bytes that a lattice of this size and storage holds at most once it
+ * is uploaded and steps at tau = 1 with AUTO: what its creation allocates, the
+ * transfer buffer of a scalar field, the statistics' scratch and the moment
+ * step's buffers.  Other step kernels, the velocity field (12 bytes per node)
+ * and larger transfers add to it, each on first use.  (No allocation.) */
 uint64_t mlbm_lattice_bytes(int32_t nx, int32_t ny, int32_t nz,
                             int32_t storage);
 

@@ -602,7 +602,7 @@ uint64_t mlbm_batch_bytes(const mlbm_batch* b) {
   if (!b) return 0;
   uint64_t s = 0;
   for (mlbm_lattice* l : b->dom)
-    if (l) s += mlbm_lattice_bytes(l->g.lx, l->g.ly, l->g.lz, b->storage);
+    if (l) s += held_bytes(l);
   return s;
 }
 

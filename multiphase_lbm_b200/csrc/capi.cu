@@ -194,6 +194,33 @@ Phys to_phys(const mlbm_params& p) {
   return q;
 }
 
+// Sizes of the parts of a lattice's first allocation.
+struct DenseParts {
+  size_t pop, rho, nbw, words, psi, init, mask, err;
+  DenseParts(const Geom& g, int storage) {
+    auto up = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+    const size_t np = (size_t)g.plane, mask_words = (size_t)g.lz * g.ly * g.wpr;
+    pop = up(np * Q * pop_elem_bytes(storage));
+    rho = up(np * real_bytes(storage));
+    nbw = up(np * sizeof(uint32_t));
+    words = up(2 * mask_words * sizeof(uint32_t));
+    psi = up((size_t)psi_elems(g) * real_bytes(storage));
+    init = up(np * sizeof(float));
+    mask = up(mask_words * sizeof(uint32_t));
+    err = up(sizeof(int));
+  }
+  size_t zeros() const { return psi + init + mask + err; }  // what starts as zeros
+  size_t total() const { return pop + rho + nbw + words + zeros(); }
+};
+
+// Blocks of a statistics pass: up to four per SM, as every record is folded
+// again by one block.
+constexpr int kStatBlocks = 592;
+size_t stats_scratch_bytes(unsigned blocks) {
+  return (kStatCounters + (size_t)blocks * ST_COUNT + ST_COUNT + 1) * sizeof(double);
+}
+size_t stats_scratch_max() { return stats_scratch_bytes(kStatBlocks); }
+
 mlbm_status check_lat(const mlbm_lattice* lat) {
   if (!lat) return fail(MLBM_ERR_ARG, "null lattice handle");
   return MLBM_OK;
@@ -458,14 +485,10 @@ uint64_t mlbm_lattice_bytes(int32_t lx, int32_t ly, int32_t lz,
                             int32_t storage) {
   if (lx <= 0 || ly <= 0 || lz <= 0) return 0;
   const Geom g = make_geom(lx, ly, lz);
-  const uint64_t np = (uint64_t)g.plane;
-  return np * Q * pop_elem_bytes(storage)     // populations
-         + np * real_bytes(storage)           // rho
-         + (uint64_t)psi_elems(g) * real_bytes(storage)  // psi with ghosts
-         + np * 4                             // initial density
-         + (uint64_t)g.lz * g.ly * g.wpr * 4  // mask
-         + np * 4;                            // neighbour words
-  // (the velocity field, 12 bytes per node, is allocated on first request)
+  return DenseParts(g, storage).total()             // allocated at creation
+         + (uint64_t)lx * ly * lz * real_bytes(storage)  // transfer buffer
+         + stats_scratch_max()
+         + moments_max_bytes(g, storage);           // the step at tau = 1
 }
 
 mlbm_status mlbm_lattice_create(int32_t lx, int32_t ly, int32_t lz,
@@ -493,36 +516,25 @@ mlbm_status mlbm_lattice_create(int32_t lx, int32_t ly, int32_t lz,
   lat->storage = storage;
   lat->g = make_geom(lx, ly, lz);
   lat->compact.two_pass_ok = compact_two_pass_supported(lx, ly, lz, storage);
-  const size_t np = (size_t)lat->g.plane;
-  const size_t mask_words = (size_t)lz * ly * lat->g.wpr;
   // one allocation for all buffers (an allocation and its release cost about
   // half a millisecond of host time, whatever its size); what starts as zeros
   // lies together
-  auto up = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
-  const size_t pop_bytes = up(np * Q * pop_elem_bytes(storage));
-  const size_t rho_bytes = up(np * real_bytes(storage));
-  const size_t nbw_bytes = up(np * sizeof(uint32_t));
-  const size_t psi_bytes = up((size_t)psi_elems(lat->g) * real_bytes(storage));
-  const size_t init_bytes = up(np * sizeof(float));
-  const size_t mask_bytes = up(mask_words * sizeof(uint32_t));
-  const size_t words_bytes = up(2 * mask_words * sizeof(uint32_t));
-  const size_t zeros = psi_bytes + init_bytes + mask_bytes + up(sizeof(int));
-  const size_t bytes = pop_bytes + rho_bytes + nbw_bytes + words_bytes + zeros;
-  cudaError_t e = cudaMalloc(&lat->buffer, bytes);
+  const DenseParts part(lat->g, storage);
+  cudaError_t e = cudaMalloc(&lat->buffer, part.total());
   if (e == cudaSuccess) {
-    lat->buffer_bytes = bytes;
+    lat->buffer_bytes = part.total();
     char* at = static_cast<char*>(lat->buffer);
     lat->pop = at;
-    lat->rho = at += pop_bytes;
-    lat->nbw = reinterpret_cast<uint32_t*>(at += rho_bytes);
-    lat->stat_words = reinterpret_cast<uint32_t*>(at += nbw_bytes);
-    lat->psi = at += words_bytes;
-    lat->rho_init = reinterpret_cast<float*>(at + psi_bytes);
-    lat->mask = reinterpret_cast<uint32_t*>(at + psi_bytes + init_bytes);
-    lat->err = reinterpret_cast<int*>(at + psi_bytes + init_bytes + mask_bytes);
+    lat->rho = at += part.pop;
+    lat->nbw = reinterpret_cast<uint32_t*>(at += part.rho);
+    lat->stat_words = reinterpret_cast<uint32_t*>(at += part.nbw);
+    lat->psi = at += part.words;
+    lat->rho_init = reinterpret_cast<float*>(at + part.psi);
+    lat->mask = reinterpret_cast<uint32_t*>(at + part.psi + part.init);
+    lat->err = reinterpret_cast<int*>(at + part.psi + part.init + part.mask);
     // waited for: the lattice's own work may go to a stream that the legacy
     // stream's does not order itself with
-    e = cudaMemset(at, 0, zeros);
+    e = cudaMemset(at, 0, part.zeros());
     if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
   } else {
     lat->buffer = nullptr;
@@ -750,14 +762,13 @@ mlbm_status stats_enqueue(mlbm_lattice* lat, double* h, bool full) {
                 "gather the slabs' own planes first");
   DeviceGuard restore_device;
   if (mlbm_status st = activate(lat)) return st;
-  // up to four blocks per SM: every record is folded again by one block
   const int nwords = (int)((long long)lat->g.lz * lat->g.ly * lat->g.wpr);
   constexpr int kPer = kStatThreads / 32 * kStatWords;
-  const unsigned nodes = (unsigned)std::min(592, (nwords + kPer - 1) / kPer);
+  const unsigned nodes = (unsigned)std::min(kStatBlocks, (nwords + kPer - 1) / kPer);
   const unsigned bound = (unsigned)((nwords + kStatThreads - 1) / kStatThreads);
   // the counters; the block records; the results
   const size_t records = (size_t)nodes * ST_COUNT;
-  const size_t need = (kStatCounters + records + ST_COUNT + 1) * sizeof(double);
+  const size_t need = stats_scratch_bytes(nodes);
   if (lat->stats_scratch_bytes < need) {
     // a larger area: earlier calls may still be reading the old one
     CUDA_TRY(cudaStreamSynchronize(lat->stream), "stats");

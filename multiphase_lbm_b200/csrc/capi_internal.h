@@ -144,6 +144,7 @@ bool compact_band_fits(mlbm_lattice* lat);
 // The moment step (moments.cu): tau = 1, any storage, whole lattices.
 bool moments_supported(const Geom& g);
 bool moments_apply(const mlbm_lattice* lat);
+size_t moments_max_bytes(const Geom& g, int storage);  // every node fluid; 0: unsupported
 mlbm_status moments_prepare(mlbm_lattice* lat);      // lists and buffers
 // One step; starts from moments, or from populations in the dense layout.
 template <typename T>

@@ -13,6 +13,20 @@ namespace {
 
 size_t up256(size_t n) { return (n + 255) / 256 * 256; }
 
+// Sizes of the parts of the buffer for a list of `pairs`.
+struct Parts {
+  size_t m, psi, n, words, xyz;
+  Parts(const Geom& g, int storage, size_t pairs) {
+    const size_t real = real_bytes(storage);
+    m = up256((size_t)node_elems(g) * 4 * real);
+    psi = up256((size_t)node_elems(g) * real);
+    n = up256(pairs * 8 * real);
+    words = up256(pairs * sizeof(uint2));
+    xyz = up256(pairs * sizeof(uint32_t));
+  }
+  size_t total() const { return m + psi + n + words + xyz; }
+};
+
 // Pair list of the current mask and slabs, and the
 // buffers (one allocation).  Waits for the counts.
 mlbm_status build_list(mlbm_lattice* lat) {
@@ -45,13 +59,8 @@ mlbm_status build_list(mlbm_lattice* lat) {
     e = cudaMemcpyAsync(&total, counts + grid, sizeof total,
                         cudaMemcpyDeviceToHost, lat->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(lat->stream);
-  const size_t real = real_bytes(lat->storage);
-  const size_t m_bytes = up256((size_t)node_elems(g) * 4 * real);
-  const size_t psi_bytes = up256((size_t)node_elems(g) * real);
-  const size_t n_bytes = up256((size_t)total * 8 * real);
-  const size_t words_bytes = up256((size_t)total * sizeof(uint2));
-  const size_t xyz_bytes = up256((size_t)total * sizeof(uint32_t));
-  const size_t need = m_bytes + psi_bytes + n_bytes + words_bytes + xyz_bytes;
+  const Parts part(g, lat->storage, total);
+  const size_t need = part.total();
   if (e == cudaSuccess && need > s.buffer_bytes) {
     cudaFree(s.buffer);
     s.buffer = nullptr;
@@ -62,10 +71,10 @@ mlbm_status build_list(mlbm_lattice* lat) {
   if (e == cudaSuccess) {
     char* at = static_cast<char*>(s.buffer);
     s.m = at;
-    s.psi = at += m_bytes;
-    s.n = at += psi_bytes;
-    s.words = reinterpret_cast<uint2*>(at += n_bytes);
-    s.xyz = reinterpret_cast<uint32_t*>(at += words_bytes);
+    s.psi = at += part.m;
+    s.n = at += part.psi;
+    s.words = reinterpret_cast<uint2*>(at += part.n);
+    s.xyz = reinterpret_cast<uint32_t*>(at += part.words);
     s.npairs = (int)total;
     if (total)
       k_mom_tiles<false><<<(unsigned)grid, threads, 0, lat->stream>>>(
@@ -134,6 +143,11 @@ mlbm_status to_populations(mlbm_lattice* lat) {
 bool moments_supported(const Geom& g) {
   return g.lx <= kC2MaxX && g.ly <= kC2MaxY && g.lz <= kC2MaxZ &&
          node_elems(g) < (1LL << 31);
+}
+
+size_t moments_max_bytes(const Geom& g, int storage) {
+  if (!moments_supported(g)) return 0;
+  return Parts(g, storage, (size_t)g.lx * g.ly * ((g.lz + 1) / 2)).total();
 }
 
 bool moments_apply(const mlbm_lattice* lat) {

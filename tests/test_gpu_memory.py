@@ -225,3 +225,28 @@ def test_a_small_transfer_needs_no_room_for_a_field(storage):
     assert np.array_equal(lat.field("fluid"), ref.field("fluid"))
     lat.close()
     ref.close()
+
+
+@pytest.mark.parametrize("storage", [0, 1, 2])
+@pytest.mark.parametrize("shape,solid", [((40, 24, 17), 0.0), ((33, 20, 16), 0.4),
+                                         ((5, 3, 1), 0.0)])
+def test_stated_bytes_cover_what_is_held(shape, solid, storage):
+    """A server that admits by mlbm_lattice_bytes: at most that is held by a
+    domain that is uploaded, stepped at tau = 1 and read, and a batch says what
+    its domains hold."""
+    from conftest import random_case
+
+    from multiphase_lbm_b200 import batch, capi
+    fluid, rho = random_case(shape, seed=4, solid_frac=solid, rho0=1.2, amp=0.3)
+    b = batch.Batch(storage=storage)
+    ids = [b.add(fluid, rho, capi.default_params(G=-5.0)) for _ in range(2)]
+    b.iterate(3)
+    for did in ids:
+        b.lattice(did).stats()
+        b.lattice(did).field("rho", f64=storage == 2)
+    held = [b.lattice(did).test_memory_limit() for did in ids]
+    assert max(held) <= capi.lattice_bytes(shape, storage)
+    if solid == 0.0 and shape[2] > 1:  # not by much above it, either
+        assert max(held) >= 0.9 * (capi.lattice_bytes(shape, storage) - 70_000)
+    assert b.nbytes() == sum(held)
+    b.close()
