@@ -38,6 +38,7 @@ struct CompactState {
 // The moment step (moments.cuh): lists and buffers, built on first use.
 struct MomentState {
   bool list_built = false;  // the lists match the mask and the slabs
+  int inlet = -1, outlet = -1;  // widths of the slabs of the initial state
   bool no_room = false;     // a buffer was refused: population kernels run
   bool active = false;      // m holds the current state
   void* buffer = nullptr;   // one allocation for all of the following
@@ -153,7 +154,7 @@ mlbm_status launch_moment_step(mlbm_lattice* lat, const StepArgs& a,
 mlbm_status moments_sync_dense(mlbm_lattice* lat);   // dense copy, stay
 mlbm_status moments_leave(mlbm_lattice* lat);        // moments -> dense state
 mlbm_status moments_release(mlbm_lattice* lat);      // leave; buffers freed
-void moments_reset(mlbm_lattice* lat);  // a new mask or initial state
+void moments_reset(mlbm_lattice* lat);  // a new initial state
 void moments_free(mlbm_lattice* lat);
 mlbm_status compact_set_band_shape(mlbm_lattice* lat, int rows, int planes);
 }  // namespace mlbm

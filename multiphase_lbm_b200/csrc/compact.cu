@@ -192,6 +192,7 @@ mlbm_status compact_leave(mlbm_lattice* lat) {
 void compact_invalidate(mlbm_lattice* lat) {
   lat->compact.built = false;
   lat->compact.active = false;
+  lat->mom.list_built = false;
   moments_reset(lat);
 }
 

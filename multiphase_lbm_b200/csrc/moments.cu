@@ -230,10 +230,16 @@ mlbm_status moments_release(mlbm_lattice* lat) {
   return MLBM_OK;
 }
 
+// The lists stay where mask and slabs do: a step after a new initial state then
+// allocates nothing and waits for nothing, so it can be captured into a graph.
 void moments_reset(mlbm_lattice* lat) {
-  lat->mom.list_built = false;
-  lat->mom.no_room = false;
-  lat->mom.active = false;
+  MomentState& s = lat->mom;
+  if (s.inlet != lat->phys.inlet_width || s.outlet != lat->phys.outlet_width)
+    s.list_built = false;
+  s.inlet = lat->phys.inlet_width;
+  s.outlet = lat->phys.outlet_width;
+  s.no_room = false;
+  s.active = false;
 }
 
 void moments_free(mlbm_lattice* lat) {

@@ -76,3 +76,47 @@ def test_ring_jobs_come_in_on_the_slabs_stream():
         assert np.array_equal(slab.gather(slabs, "f")[m], want.field("f")[m])
         run.close()
     want.close()
+
+
+@pytest.mark.parametrize("storage", [0, 1, 2])
+@pytest.mark.parametrize("tau", [1.0, 0.8])
+def test_a_step_after_a_new_initial_state_can_be_captured(storage, tau):
+    """The buffers and tables of the first run serve the next: nothing is
+    allocated or waited for, which a capture would refuse."""
+    import torch
+
+    from multiphase_lbm_b200 import capi
+    shape = (40, 24, 17)
+    fluid, rho = sphere_case(shape, seed=8, rmin=2.0, rmax=4.0, porosity=0.6,
+                             rho0=1.2, amp=0.4)
+    want = _lattice(capi, shape, fluid, rho, storage, capi.KERNEL_TWO_PASS, tau=tau,
+                    inlet_width=2, rho_inlet=0.3)
+    want.iterate(0, 5)
+    stream = torch.cuda.Stream()
+    lat = _lattice(capi, shape, fluid, rho, storage, capi.KERNEL_AUTO, tau=tau,
+                   inlet_width=2, rho_inlet=0.3)
+    torch.cuda.synchronize()
+    lat.set_stream(stream.cuda_stream)
+    lat.iterate(0, 3)
+    lat.initialize()
+    lat.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        lat.iterate(0, 4)
+    graph.replay()
+    torch.cuda.synchronize()
+    lat.iterate(4, 1)
+    torch.cuda.synchronize()
+    assert lat.field("f", f64=storage == 2).tobytes() == \
+        want.field("f", f64=storage == 2).tobytes()
+    del graph
+    # slabs of another width: the lists follow them
+    for l in (lat, want):
+        l.set_params(capi.default_params(G=-5.0, rhos=0.2, rho_shift=1.0, tau=tau,
+                                         inlet_width=5, rho_inlet=0.3))
+        l.initialize()
+        l.iterate(0, 5)
+    torch.cuda.synchronize()
+    assert lat.field("f").tobytes() == want.field("f").tobytes()
+    lat.close()
+    want.close()
