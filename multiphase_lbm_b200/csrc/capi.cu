@@ -52,6 +52,25 @@ mlbm_status cuda_fail(cudaError_t e, const char* where) {
   return fail(MLBM_ERR_CUDA, "%s: %s", where, cudaGetErrorString(e));
 }
 
+// Sizes of the parts of a lattice's first allocation.
+struct DenseParts {
+  size_t pop, rho, nbw, words, psi, init, mask, err;
+  DenseParts(const Geom& g, int storage) {
+    auto up = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+    const size_t np = (size_t)g.plane, mask_words = (size_t)g.lz * g.ly * g.wpr;
+    pop = up(np * Q * pop_elem_bytes(storage));
+    rho = up(np * real_bytes(storage));
+    nbw = up(np * sizeof(uint32_t));
+    words = up(2 * mask_words * sizeof(uint32_t));
+    psi = up((size_t)psi_elems(g) * real_bytes(storage));
+    init = up(np * sizeof(float));
+    mask = up(mask_words * sizeof(uint32_t));
+    err = up(sizeof(int));
+  }
+  size_t zeros() const { return psi + init + mask + err; }  // what starts as zeros
+  size_t total() const { return pop + rho + nbw + words + zeros(); }
+};
+
 size_t held_bytes(const mlbm_lattice* lat) {
   const CompactState& c = lat->compact;
   return lat->buffer_bytes +
@@ -78,6 +97,15 @@ cudaError_t lattice_malloc(mlbm_lattice* lat, void** p, size_t bytes) {
   if (moments_release(lat) != MLBM_OK) return e;
   lat->mom.no_room = true;
   return lattice_try_malloc(lat, p, bytes);
+}
+
+mlbm_status lattice_clear(mlbm_lattice* lat) {
+  if (lat->cleared) return MLBM_OK;
+  const cudaError_t e = cudaMemsetAsync(
+      lat->psi, 0, DenseParts(lat->g, lat->storage).zeros(), lat->stream);
+  if (e != cudaSuccess) return cuda_fail(e, "lattice clear");
+  lat->cleared = true;
+  return MLBM_OK;
 }
 
 void prefault(void* p, size_t bytes) {
@@ -194,25 +222,6 @@ Phys to_phys(const mlbm_params& p) {
   return q;
 }
 
-// Sizes of the parts of a lattice's first allocation.
-struct DenseParts {
-  size_t pop, rho, nbw, words, psi, init, mask, err;
-  DenseParts(const Geom& g, int storage) {
-    auto up = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
-    const size_t np = (size_t)g.plane, mask_words = (size_t)g.lz * g.ly * g.wpr;
-    pop = up(np * Q * pop_elem_bytes(storage));
-    rho = up(np * real_bytes(storage));
-    nbw = up(np * sizeof(uint32_t));
-    words = up(2 * mask_words * sizeof(uint32_t));
-    psi = up((size_t)psi_elems(g) * real_bytes(storage));
-    init = up(np * sizeof(float));
-    mask = up(mask_words * sizeof(uint32_t));
-    err = up(sizeof(int));
-  }
-  size_t zeros() const { return psi + init + mask + err; }  // what starts as zeros
-  size_t total() const { return pop + rho + nbw + words + zeros(); }
-};
-
 // Blocks of a statistics pass: up to four per SM, as every record is folded
 // again by one block.
 constexpr int kStatBlocks = 592;
@@ -226,9 +235,9 @@ mlbm_status check_lat(const mlbm_lattice* lat) {
   return MLBM_OK;
 }
 
-mlbm_status activate(const mlbm_lattice* lat) {
+mlbm_status activate(mlbm_lattice* lat) {
   CUDA_TRY(cudaSetDevice(lat->device), "cudaSetDevice");
-  return MLBM_OK;
+  return lattice_clear(lat);
 }
 
 template <typename T, int PHASE>
@@ -532,10 +541,9 @@ mlbm_status mlbm_lattice_create(int32_t lx, int32_t ly, int32_t lz,
     lat->rho_init = reinterpret_cast<float*>(at + part.psi);
     lat->mask = reinterpret_cast<uint32_t*>(at + part.psi + part.init);
     lat->err = reinterpret_cast<int*>(at + part.psi + part.init + part.mask);
-    // waited for: the lattice's own work may go to a stream that the legacy
-    // stream's does not order itself with
-    e = cudaMemset(at, 0, part.zeros());
-    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+    // (psi and what follows are cleared by the first call that uses them, on
+    // the lattice's stream: here no stream is ordered with the work to come,
+    // and a wait would be one for whatever else the default stream does)
   } else {
     lat->buffer = nullptr;
   }

@@ -68,6 +68,7 @@ struct mlbm_lattice {
 
   void* buffer = nullptr;       // one allocation for pop .. nbw and err
   size_t buffer_bytes = 0;
+  bool cleared = false;         // what starts as zeros is (lattice_clear)
   size_t memory_limit = 0;      // mlbm_test_memory_limit; 0: none
   void* pop = nullptr;          // 19 planes of g.plane elements (T)
   void* rho = nullptr;          // density, R per node
@@ -105,6 +106,9 @@ struct mlbm_lattice {
 
 namespace mlbm {
 mlbm_status cuda_fail(cudaError_t e, const char* where);
+// Before a lattice's first work: its psi, initial density, mask and error flag
+// start as zeros (on its stream).
+mlbm_status lattice_clear(mlbm_lattice* lat);
 // Device bytes a lattice holds.
 size_t held_bytes(const mlbm_lattice* lat);
 // Device memory for a lattice.  Where it is refused while the lattice holds

@@ -215,6 +215,7 @@ mlbm_status mlbm_checkpoint_load(mlbm_lattice* lat, const void* image,
   DeviceGuard restore_device;
   cudaError_t e = cudaSetDevice(lat->device);
   if (e != cudaSuccess) return cuda_err(e, "checkpoint");
+  if (mlbm_status st = lattice_clear(lat)) return st;
   if (mlbm_status st = mlbm_set_params(lat, &h.params)) return st;
   e = cudaMemcpyAsync(lat->mask, payload, s.mask, cudaMemcpyDefault, lat->stream);
   if (e == cudaSuccess)

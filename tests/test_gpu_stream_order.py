@@ -120,3 +120,18 @@ def test_a_step_after_a_new_initial_state_can_be_captured(storage, tau):
     assert lat.field("f").tobytes() == want.field("f").tobytes()
     lat.close()
     want.close()
+
+
+def test_creating_a_lattice_does_not_wait_for_the_default_stream():
+    import torch
+
+    from multiphase_lbm_b200 import capi
+    capi.Lattice((40, 24, 17)).close()  # the first one loads the library
+    torch.cuda.synchronize()
+    busy = torch.cuda.Event()
+    torch.cuda._sleep(BUSY)
+    busy.record()
+    lat = capi.Lattice((40, 24, 17))
+    assert not busy.query()
+    torch.cuda.synchronize()
+    lat.close()
