@@ -234,7 +234,8 @@ mlbm_status mlbm_set_update_shape(mlbm_lattice* lat, int32_t rows,
                                   int32_t planes);
 /* Time candidate shapes of the lattice's step kernel (update shape for
  * TWO_PASS, rows x planes for BAND; COMPACT has none: out = {0, 0}, no
- * steps) and keep the fastest.  The trial steps are
+ * steps; nor has the moment step: out = the present update shape, no steps)
+ * and keep the fastest.  The trial steps are
  * real steps (step0, step0+1, ...): the lattice advances by *steps_done of
  * them.  out (optional, 2 ints) receives rows, planes. */
 mlbm_status mlbm_autotune(mlbm_lattice* lat, int64_t step0,

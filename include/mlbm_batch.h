@@ -67,7 +67,8 @@ mlbm_status mlbm_batch_set_tuning(mlbm_batch* b, int32_t rows_density,
                                   int32_t rows_update, int32_t planes,
                                   int32_t blocks_per_sm, int32_t use_graphs);
 /* Time candidate shapes on the current domains and keep the fastest (dense
- * mode; the compact mode has no shape to tune and runs no trial steps).  The
+ * mode; domains held as moments and the compact mode have no shape to tune and
+ * run no trial steps).  The
  * trial steps are real steps: every domain advances by them.  out (optional,
  * 4 ints) receives rows_density, rows_update, planes, blocks_per_sm. */
 mlbm_status mlbm_batch_autotune(mlbm_batch* b, int32_t trial_steps,

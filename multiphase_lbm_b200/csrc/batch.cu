@@ -681,7 +681,11 @@ mlbm_status mlbm_batch_autotune(mlbm_batch* b, int32_t trial_steps,
                                 int32_t* out) {
   if (!b) return bfail(MLBM_ERR_ARG, "null batch");
   if (trial_steps < 1) trial_steps = 2;
-  if (compact_mode(b)) {
+  mlbm::DeviceGuard restore_device;
+  BCUDA(cudaSetDevice(b->device), "cudaSetDevice");
+  bool moments = false;
+  if (mlbm_status st = moments_mode(b, &moments)) return st;
+  if (moments || compact_mode(b)) {
     // one thread per node (pair) per pass: no work-item shape to tune
     if (out) {
       out[0] = b->By_d;

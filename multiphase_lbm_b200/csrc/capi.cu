@@ -292,6 +292,17 @@ int effective_kernel(const mlbm_lattice* lat) {
   return lat->compact.two_pass_ok ? MLBM_KERNEL_COMPACT : MLBM_KERNEL_TWO_PASS;
 }
 
+// Whether the next step is the moment step (its lists and buffers are then in
+// place): tau = 1 and no kernel asked for.  Where its buffers do not fit the
+// device, the population kernels run.
+mlbm_status takes_moments(mlbm_lattice* lat, bool* yes) {
+  *yes = false;
+  if (lat->step_kernel != MLBM_KERNEL_AUTO || !moments_apply(lat)) return MLBM_OK;
+  const mlbm_status st = moments_prepare(lat);
+  *yes = st == MLBM_OK;
+  return st == MLBM_ERR_NOMEM ? MLBM_OK : st;
+}
+
 template <typename T>
 mlbm_status launch_steps(mlbm_lattice* lat, int64_t step0, int32_t nsteps,
                          int32_t reverse, uint32_t inject_type,
@@ -312,14 +323,8 @@ mlbm_status launch_steps(mlbm_lattice* lat, int64_t step0, int32_t nsteps,
                              lat->stream),
              "velocity clear");
   }
-  // tau = 1 and no kernel asked for: the moment step.  Where its buffers do not
-  // fit the device, the population kernels run.
   bool moments = false;
-  if (lat->step_kernel == MLBM_KERNEL_AUTO && moments_apply(lat)) {
-    const mlbm_status st = moments_prepare(lat);
-    if (st && st != MLBM_ERR_NOMEM) return st;
-    moments = st == MLBM_OK;
-  }
+  if (mlbm_status st = takes_moments(lat, &moments)) return st;
   if (moments) {
     if (lat->compact.active)
       if (mlbm_status st = compact_leave(lat)) return st;
@@ -988,6 +993,16 @@ mlbm_status mlbm_autotune(mlbm_lattice* lat, int64_t step0,
   if (effective_kernel(lat) == MLBM_KERNEL_COMPACT) {
     // one thread per fluid node: nothing to tune
     if (out) out[0] = out[1] = 0;
+    if (steps_done) *steps_done = 0;
+    return MLBM_OK;
+  }
+  bool moments = false;
+  if (mlbm_status st = takes_moments(lat, &moments)) return st;
+  if (moments) {  // trial steps would not run the kernels of these shapes
+    if (out) {
+      out[0] = lat->zm.By;
+      out[1] = lat->zm.Dz;
+    }
     if (steps_done) *steps_done = 0;
     return MLBM_OK;
   }
