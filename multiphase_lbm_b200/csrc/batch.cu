@@ -180,14 +180,20 @@ mlbm_status rebuild_compact(mlbm_batch* b) {
   return MLBM_OK;
 }
 
-// Moment mode: tables of the domains, all held as moments.
+// Whether the state of a domain is moments that the batched kernels can take up
+// (theirs are stored under the rho_shift they are read back with).
+bool held_as_moments(const mlbm_lattice* lat) {
+  return lat->mom.active && lat->mom.shift == lat->phys.rho_shift;
+}
+
+// Moment mode: tables of the domains held as moments.
 mlbm_status rebuild_moments(mlbm_batch* b) {
   std::vector<MomDomain>& desc = b->mdesc;
   desc.clear();
   int n = 0;
   for (size_t s = 0; s < b->dom.size(); ++s) {
     const mlbm_lattice* lat = b->dom[s];
-    if (!lat) continue;
+    if (!lat || !held_as_moments(lat)) continue;
     const MomentState& ms = lat->mom;
     MomDomain d;
     std::memset(&d, 0, sizeof d);
@@ -227,31 +233,6 @@ mlbm_status moments_mode(mlbm_batch* b, bool* on) {
     }
   *on = true;
   return MLBM_OK;
-}
-
-template <typename T>
-mlbm_status step_alone_t(mlbm_batch* b, int reverse, unsigned inject, bool write_rho) {
-  for (size_t s = 0; s < b->dom.size(); ++s) {
-    mlbm_lattice* lat = b->dom[s];
-    if (!lat) continue;
-    if (!lat->mom.active)
-      if (mlbm_status st = compact_leave(lat)) return st;
-    const StepArgs a{b->bstep - b->origin[s], reverse, inject};
-    if (mlbm_status st = launch_moment_step<T>(lat, a, false, write_rho)) return st;
-    lat->phase ^= 1;
-  }
-  b->bstep += 1;
-  return MLBM_OK;
-}
-
-// One step of every domain by its own launches: the step that takes new
-// domains from populations to moments.
-mlbm_status step_alone(mlbm_batch* b, int reverse, unsigned inject, bool write_rho) {
-  switch (b->storage) {
-    case MLBM_STORE_F32: return step_alone_t<float>(b, reverse, inject, write_rho);
-    case MLBM_STORE_F16: return step_alone_t<__half>(b, reverse, inject, write_rho);
-    default: return step_alone_t<double>(b, reverse, inject, write_rho);
-  }
 }
 
 bool compact_mode(const mlbm_batch* b) {
@@ -410,6 +391,38 @@ void launch_step_any(mlbm_batch* b, int delta, int reverse, unsigned inject,
     launch_step<__half>(b, delta, reverse, inject, write_rho);
   else
     launch_step<double>(b, delta, reverse, inject, write_rho);
+}
+
+// One step of one domain by its own launches, from whatever form it is in.
+mlbm_status step_alone(mlbm_batch* b, size_t s, int reverse, unsigned inject,
+                       bool write_rho) {
+  mlbm_lattice* lat = b->dom[s];
+  if (!lat->mom.active)
+    if (mlbm_status st = compact_leave(lat)) return st;
+  const StepArgs a{b->bstep - b->origin[s], reverse, inject};
+  switch (b->storage) {
+    case MLBM_STORE_F32: return launch_moment_step<float>(lat, a, false, write_rho);
+    case MLBM_STORE_F16: return launch_moment_step<__half>(lat, a, false, write_rho);
+    default: return launch_moment_step<double>(lat, a, false, write_rho);
+  }
+}
+
+// The step that takes domains from populations to moments: those by their own
+// launches, the domains held as moments already by the batched ones.
+mlbm_status step_joining(mlbm_batch* b, int reverse, unsigned inject, bool write_rho) {
+  std::vector<size_t> joining;
+  for (size_t s = 0; s < b->dom.size(); ++s)
+    if (b->dom[s] && !held_as_moments(b->dom[s])) joining.push_back(s);
+  if (mlbm_status st = rebuild_moments(b)) return st;
+  launch_step_any(b, 0, reverse, inject, write_rho);
+  BCUDA(cudaGetLastError(), "batch launch");
+  for (size_t s : joining)
+    if (mlbm_status st = step_alone(b, s, reverse, inject, write_rho)) return st;
+  for (mlbm_lattice* lat : b->dom)
+    if (lat) lat->phase ^= 1;
+  b->bstep += 1;
+  b->dirty = true;
+  return MLBM_OK;
 }
 
 // Run n steps: the first n-1 without rho output (graph replays of
@@ -619,16 +632,15 @@ mlbm_status mlbm_batch_iterate(mlbm_batch* b, int32_t nsteps, int32_t reverse,
   if (mlbm_status st = moments_mode(b, &moments)) return st;
   if (moments != b->moments) b->dirty = true;
   b->moments = moments;
-  bool alone = false;
+  bool joining = false;
   for (size_t s = 0; s < b->dom.size(); ++s) {
     const mlbm_lattice* l = b->dom[s];
     if (!l) continue;
     if (l->changes != b->seen[s]) b->dirty = true;
-    if (moments && (!l->mom.active || l->mom.shift != l->phys.rho_shift))
-      alone = b->dirty = true;
+    if (moments && !held_as_moments(l)) joining = true;
   }
-  if (alone) {
-    if (mlbm_status st = step_alone(b, reverse, inject_type, nsteps == 1)) return st;
+  if (joining) {
+    if (mlbm_status st = step_joining(b, reverse, inject_type, nsteps == 1)) return st;
     if (--nsteps == 0) return MLBM_OK;
   }
   if (b->dirty)

@@ -42,3 +42,25 @@ def test_the_kernel_asked_for_runs(storage, kernel, tau, want):
                                           "k_band") if k in n]
     assert len(updates) == 3 and all(want in n for n in updates), names
     lat.close()
+
+
+@pytest.mark.parametrize("storage", [0, 1, 2])
+def test_only_a_joining_domain_steps_by_itself(storage):
+    """A batch held as moments takes in a domain: one step of that domain by its
+    own launches, beside the batched launches of the others."""
+    from multiphase_lbm_b200 import batch, capi
+    b = batch.Batch(storage=storage)
+
+    def add(i):
+        fluid, rho = random_case((20 + i, 9, 6), seed=i, rho0=1.2, amp=0.3)
+        return b.add(fluid, rho, capi.default_params(G=-5.0, rhos=0.2))
+
+    for i in range(5):
+        add(i)
+    b.iterate(2)
+    add(5)
+    names = _launched(lambda: b.iterate(3))
+    alone = [n for n in names if "k_mom_collide" in n]
+    batched = [n for n in names if "k_batch_mom_collide" in n]
+    assert len(alone) == 1 and len(batched) == 3, names
+    b.close()
