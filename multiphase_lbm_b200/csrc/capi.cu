@@ -108,6 +108,12 @@ mlbm_status lattice_clear(mlbm_lattice* lat) {
   return MLBM_OK;
 }
 
+cudaError_t velocity_clear(mlbm_lattice* lat) {
+  if (!lat->vel) return cudaSuccess;
+  return cudaMemsetAsync(lat->vel, 0, (size_t)lat->g.plane * 3 * sizeof(float),
+                         lat->stream);
+}
+
 void prefault(void* p, size_t bytes) {
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
@@ -318,10 +324,7 @@ mlbm_status launch_steps(mlbm_lattice* lat, int64_t step0, int32_t nsteps,
     CUDA_TRY(lattice_malloc(lat, (void**)&lat->vel,
                             (size_t)lat->g.plane * 3 * sizeof(float)),
              "velocity allocation");
-    // solid nodes are never written: they read zero velocity
-    CUDA_TRY(cudaMemsetAsync(lat->vel, 0, (size_t)lat->g.plane * 3 * sizeof(float),
-                             lat->stream),
-             "velocity clear");
+    CUDA_TRY(velocity_clear(lat), "velocity clear");
   }
   bool moments = false;
   if (mlbm_status st = takes_moments(lat, &moments)) return st;
@@ -612,6 +615,7 @@ static mlbm_status upload_mask_impl(mlbm_lattice* lat, const uint8_t* src,
   k_pack_mask<<<tile_grid(g), tile_block(), 0, lat->stream>>>(
       static_cast<const uint8_t*>(lat->staging), lat->mask, g);
   CUDA_TRY(cudaGetLastError(), "mask pack launch");
+  CUDA_TRY(velocity_clear(lat), "velocity clear");
   CUDA_TRY(cudaStreamSynchronize(lat->stream), "mask upload");
   compact_invalidate(lat);
   ++lat->changes;

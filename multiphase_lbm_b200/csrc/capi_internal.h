@@ -109,6 +109,9 @@ mlbm_status cuda_fail(cudaError_t e, const char* where);
 // Before a lattice's first work: its psi, initial density, mask and error flag
 // start as zeros (on its stream).
 mlbm_status lattice_clear(mlbm_lattice* lat);
+// Zero velocity everywhere (where the field is allocated): solid nodes are never
+// written and read zero, so a new mask needs it too.
+cudaError_t velocity_clear(mlbm_lattice* lat);
 // Device bytes a lattice holds.
 size_t held_bytes(const mlbm_lattice* lat);
 // Device memory for a lattice.  Where it is refused while the lattice holds

@@ -237,6 +237,7 @@ mlbm_status mlbm_checkpoint_load(mlbm_lattice* lat, const void* image,
         static_cast<const float*>(lat->rho), static_cast<float*>(lat->psi), g,
         lat->phys);
   e = cudaGetLastError();
+  if (e == cudaSuccess) e = velocity_clear(lat);
   if (e == cudaSuccess) e = cudaStreamSynchronize(lat->stream);
   if (e != cudaSuccess) return cuda_err(e, "checkpoint load");
   compact_invalidate(lat);  // the fluid-only tables follow the new mask

@@ -220,10 +220,10 @@ mlbm_status mlbm_step_pass(mlbm_lattice* lat, int64_t step, int32_t pass,
   if (mlbm_status st = ready_for_passes(lat, "step_pass")) return st;
   const bool wu = pass == 1 && (flags & MLBM_ITER_WRITE_VELOCITY);
   if (wu && !lat->vel) {
-    // the velocity field is allocated on first request; solid nodes read 0
+    // the velocity field is allocated on first request
     const size_t bytes = (size_t)lat->g.plane * 3 * sizeof(float);
     cudaError_t e = lattice_malloc(lat, (void**)&lat->vel, bytes);
-    if (e == cudaSuccess) e = cudaMemsetAsync(lat->vel, 0, bytes, lat->stream);
+    if (e == cudaSuccess) e = velocity_clear(lat);
     if (e != cudaSuccess) return slab_cuda(e, "velocity allocation");
   }
   const StepArgs a{(long long)step, reverse, inject_type};
