@@ -179,11 +179,12 @@ mlbm_status mlbm_iterate(mlbm_lattice* lat, int64_t step0, int32_t nsteps,
 
 /* Which kernels advance the lattice:
  *   TWO_PASS     a density launch and an update launch per step over the
- *                dense layout; bit-identical to the reference's kernels;
+ *                dense layout; FP32 within 1e-5 of the reference's kernels
+ *                over the first 100 steps;
  *   COMPACT      the two passes over a fluid-only population layout (solid
  *                nodes own no population storage), one thread per fluid
- *                node pair (one per node in the gather step's density
- *                pass), each launch overlapping the end of the one before
+ *                node pair (one per node in the gather step), each launch
+ *                overlapping the end of the one before
  *                (programmatic dependent launch); bit-identical to
  *                TWO_PASS.  FP32 / FP16 storage, at most 2048 x 2048 x 1024
  *                nodes;
@@ -211,9 +212,11 @@ mlbm_status mlbm_iterate(mlbm_lattice* lat, int64_t step0, int32_t nsteps,
  *                buffer of the lattice, the population kernels run until
  *                the next mlbm_initialize.
  * (Values 1, 4 and 5 belonged to step kernels this library no longer has;
- * they are refused.)  The state moves between the layouts on demand (the
- * dense buffers stay allocated; the fluid-only layout adds 19 populations
- * and 8 bytes of node table per fluid node, allocated on first use). */
+ * they are refused.)  The state moves between the layouts on demand.  The
+ * dense buffers stay allocated; what a step kernel adds is allocated on its
+ * first use: the fluid-only layout 19 populations and 8 bytes of node table
+ * per fluid node, the moment step 20 bytes (FP64: 40) per node, rows padded to
+ * 32 nodes, and 44 (FP64: 76) per pair of nodes in z that holds fluid. */
 #define MLBM_KERNEL_AUTO 0
 #define MLBM_KERNEL_TWO_PASS 2
 #define MLBM_KERNEL_COMPACT 3

@@ -5,15 +5,18 @@
  *
  * A batch owns one mlbm_lattice per domain (same storage format, each with
  * its own size, parameters, AA phase and step origin).  mlbm_batch_iterate
- * advances every domain with one density launch and one update launch per
- * step over all domains, replayed through a CUDA graph: with FP32 / FP16
- * storage the domains live in the fluid-only (compact) layout and the
- * launches run one thread per fluid node or node pair of every domain; with
- * FP64 storage (or a domain beyond the compact kernels' limits) persistent
- * launches walk a work list of tiles of the dense layout.  Results are
- * bit-identical to the same domain advanced alone with mlbm_iterate.
- * Domains can be added and removed between iterate calls (continuous
- * batching).
+ * advances every domain with two launches per step over all domains, replayed
+ * through a CUDA graph.  Where every domain has tau = 1 they are held as
+ * moments (mlbm.h, AUTO), a gather and a collide launch per 128 domains.  Else,
+ * or where the device has no room for those buffers, every domain holds
+ * populations: with FP32 / FP16 storage in the fluid-only (compact) layout, a
+ * density and an update launch with one thread per fluid node or node pair of
+ * every domain; with FP64 storage (or a domain beyond the compact kernels'
+ * limits) persistent launches walk a work list of tiles of the dense layout.
+ * Results are bit-identical to the same domain advanced alone with
+ * mlbm_iterate.  Domains can be added and removed between iterate calls
+ * (continuous batching); what is changed or advanced through a domain's own
+ * lattice holds from the next iterate call on.
  */
 #ifndef MLBM_BATCH_H_
 #define MLBM_BATCH_H_
@@ -46,7 +49,7 @@ mlbm_status mlbm_batch_add_checkpoint(mlbm_batch* b, const void* image,
                                       uint64_t bytes, int32_t* id);
 /* Remove a domain and free its memory. */
 mlbm_status mlbm_batch_remove(mlbm_batch* b, int32_t id);
-/* Number of domains, and device bytes they hold. */
+/* Number of domains, and device bytes that they hold now. */
 int32_t mlbm_batch_count(const mlbm_batch* b);
 uint64_t mlbm_batch_bytes(const mlbm_batch* b);
 
@@ -54,7 +57,8 @@ uint64_t mlbm_batch_bytes(const mlbm_batch* b);
 mlbm_status mlbm_batch_iterate(mlbm_batch* b, int32_t nsteps, int32_t reverse,
                                uint32_t inject_type);
 /* The lattice of a domain: use mlbm_download_field / mlbm_phase_stats on it
- * (they run on the batch's stream and synchronise). */
+ * (they run on the batch's stream and synchronise), mlbm_set_params, or
+ * mlbm_iterate to advance it alone (its step counter in the batch stays). */
 mlbm_lattice* mlbm_batch_lattice(mlbm_batch* b, int32_t id);
 /* Steps a domain has been advanced (its step counter). */
 int64_t mlbm_batch_domain_step(const mlbm_batch* b, int32_t id);

@@ -8,16 +8,15 @@ U[-2, 0] (rhos = -ln(1 - G_ads/G), G = -6); the drainage boundaries of the
 outlet plane x = lx - 1 at rho 1.95, pores start at rho 2.0); FP16 storage.
 
 Two executions of the same steps, bit-identical results:
-  * batched -- mlbm_batch_iterate: one persistent density launch and one
-    persistent update launch per step for all domains, CUDA graphs, work-item
-    shape from the autotuner;
+  * batched -- mlbm_batch_iterate: the domains held as moments (tau = 1), two
+    launches per step and up to 128 domains, CUDA graphs;
   * plain   -- each domain advanced by its own mlbm_iterate calls, one domain
-    after the other (sequential per-domain launches), with the same two-pass
-    kernels as the batch.
-Two more executions advance the domains one after the other with the
-fluid-only kernels: plain_compact (the compact two-pass step, two launches
-per step and domain) and plain_band (the one-pass step, one launch per step
-and domain); both bit-identical to the batch.
+    after the other (sequential per-domain launches), with the dense two-pass
+    kernels.
+Three more executions advance the domains one after the other: plain_default
+(no kernel asked for: the moment step), plain_compact (the compact two-pass
+step, two launches per step and domain) and plain_band (the one-pass step, one
+launch per step and domain); all bit-identical to the batch.
 All are timed with CUDA events over `--steps` steps (default 5,000, the
 configured run); solves/s = domains / (time for 5,000 steps).
 
@@ -128,6 +127,7 @@ def run(ndomains=512, steps=100, storage=capi.STORE_F16, solve_steps=5000,
         return ms, wall
 
     ms_p, wall_p = plain(capi.KERNEL_TWO_PASS)
+    ms_d, wall_d = plain(capi.KERNEL_AUTO)
     ms_c, wall_c = plain(capi.KERNEL_COMPACT) if compact else (None, None)
     ms_band, wall_band = plain(capi.KERNEL_BAND) if compact else (None, None)
 
@@ -145,8 +145,11 @@ def run(ndomains=512, steps=100, storage=capi.STORE_F16, solve_steps=5000,
         "speedup": round(ms_p / ms_b, 3),
         "form": "batching",
         "wall_s": {"batched": round(wall_b, 2), "plain": round(wall_p, 2),
+                   "plain_default": round(wall_d, 2),
                    "plain_compact": None if wall_c is None else round(wall_c, 2),
                    "plain_band": None if wall_band is None else round(wall_band, 2)},
+        "plain_default_ms_per_step": round(ms_d, 4),
+        "speedup_vs_plain_default": round(ms_d / ms_b, 3),
         "plain_compact_ms_per_step": None if ms_c is None else round(ms_c, 4),
         "speedup_vs_plain_compact": None if ms_c is None else round(ms_c / ms_b, 3),
         "plain_band_ms_per_step": None if ms_band is None else round(ms_band, 4),

@@ -219,7 +219,8 @@ class Lattice:
     @property
     def step_kernel(self) -> int:
         """The kernel the next iterate runs (KERNEL_COMPACT, ... ; AUTO
-        resolved)."""
+        resolved to the population kernel, which at tau = 1 stands back for
+        the moment step)."""
         return int(lib().mlbm_get_step_kernel(self.h))
 
     def checkpoint(self, step: int, out: "np.ndarray | None" = None) -> np.ndarray:

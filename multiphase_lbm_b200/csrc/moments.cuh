@@ -35,8 +35,9 @@
 // together -- about 750 instructions per warp of pairs, and the cache lines its
 // loads touch: a warp of the list spans 2-3 runs of fluid along x, so a 16-byte
 // load of its lanes touches 6 lines where a full row would touch 4 --, the
-// collide the latency of its loads.  At 200^3 FP32 the population kernels take
-// 206 us a step, this step 109.  Tried there: one node per thread 155; the two
+// collide the latency of its loads.  At 200^3, tau = 1, the population kernels
+// (compact2.cuh) take 183 us a step in FP32 and 152 in FP16 storage, this step
+// 109 and 112.  Tried there (FP32): one node per thread 155; the two
 // nodes of a pair side by side with 32-byte loads 117 (19 requests in place of
 // 28, but 9.7 lines each); pairs whose neighbours are all fluid listed first in
 // each tile, to skip their bounce-back selects, 119 (the runs break up: 7.9

@@ -49,7 +49,7 @@ SERVE_G = -5.0
 CONVERGENCE_DS = 1e-5
 CONVERGENCE_STEPS = 1000
 # Active lattice nodes beyond which arrivals wait (about twice what fills
-# every SM of a B200 with the compact kernels).
+# every SM of a B200).
 DEFAULT_NODE_CAP = 16_000_000
 
 
@@ -234,9 +234,8 @@ def serve_batched(reqs, hbm_cap=150e9, chunk=CONVERGENCE_STEPS, log=None,
 def serve_fifo(reqs, chunk=CONVERGENCE_STEPS, log=None,
                kernel=capi.KERNEL_AUTO):
     """Requests one at a time in arrival order, each alone on the GPU, with
-    the fastest plain kernels (AUTO: the compact two-pass step, bit-identical
-    to the batch's kernels, so every result equals the batched one bit for
-    bit)."""
+    the fastest plain kernels (AUTO: the moment step, bit-identical to the
+    batch's kernels, so every result equals the batched one bit for bit)."""
     t0 = time.perf_counter()
     idle = 0.0
     for r in sorted(reqs, key=lambda q: q.arrival):
