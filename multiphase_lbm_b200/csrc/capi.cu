@@ -598,9 +598,9 @@ mlbm_status mlbm_set_params(mlbm_lattice* lat, const mlbm_params* p) {
                 p->inlet_width, p->outlet_width);
   if (p->carn_star && p->G == 0.f)
     return fail(MLBM_ERR_ARG, "Carnahan-Starling psi needs G != 0");
+  if (!lat->has_params || std::memcmp(&lat->params, p, sizeof *p) != 0) ++lat->changes;
   lat->params = *p;
   lat->phys = to_phys(*p);
-  ++lat->changes;
   lat->has_params = true;
   return MLBM_OK;
 }
