@@ -25,7 +25,10 @@ struct mlbm_batch {
   std::vector<mlbm_lattice*> dom;     // slots (nullptr = free)
   std::vector<long long> origin;      // batch step at which step 0 would be
   std::vector<int> phase_base;        // AA phase offset (see DomainDesc)
-  std::vector<unsigned long long> seen;  // lattice's `changes` at the rebuild
+  struct Counts {
+    unsigned long long changes, moves;
+  };
+  std::vector<Counts> seen;           // of the lattices at the rebuild
   long long bstep = 0;                // steps executed by the batch
   // device tables, rebuilt when the set of domains or the tuning changes
   DomainDesc* d_desc = nullptr;
@@ -248,7 +251,7 @@ mlbm_status rebuild(mlbm_batch* b) {
   for (size_t s = 0; s < b->dom.size(); ++s)
     if (const mlbm_lattice* lat = b->dom[s]) {
       b->phase_base[s] = (lat->phase + (int)(b->bstep & 1)) & 1;
-      b->seen[s] = lat->changes;
+      b->seen[s] = {lat->changes, lat->moves};
     }
   if (b->moments) return rebuild_moments(b);
   b->compact = compact_mode(b);
@@ -473,7 +476,7 @@ int32_t insert_domain(mlbm_batch* b, mlbm_lattice* lat, int64_t step0) {
     b->dom.push_back(nullptr);
     b->origin.push_back(0);
     b->phase_base.push_back(0);
-    b->seen.push_back(0);
+    b->seen.push_back({0, 0});
   }
   b->dom[slot] = lat;
   b->origin[slot] = b->bstep - step0;
@@ -636,7 +639,9 @@ mlbm_status mlbm_batch_iterate(mlbm_batch* b, int32_t nsteps, int32_t reverse,
   for (size_t s = 0; s < b->dom.size(); ++s) {
     const mlbm_lattice* l = b->dom[s];
     if (!l) continue;
-    if (l->changes != b->seen[s]) b->dirty = true;
+    // (moments have no phase, and stay where they are while they are held)
+    if (l->changes != b->seen[s].changes || (!moments && l->moves != b->seen[s].moves))
+      b->dirty = true;
     if (moments && !held_as_moments(l)) joining = true;
   }
   if (joining) {

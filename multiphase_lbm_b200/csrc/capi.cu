@@ -707,7 +707,7 @@ mlbm_status mlbm_iterate(mlbm_lattice* lat, int64_t step0, int32_t nsteps,
   if (nsteps == 0) return MLBM_OK;
   DeviceGuard restore_device;
   if (mlbm_status st = activate(lat)) return st;
-  ++lat->changes;
+  ++lat->moves;
   switch (lat->storage) {
     case MLBM_STORE_F32:
       return launch_steps<float>(lat, step0, nsteps, reverse, inject_type, flags);

@@ -95,9 +95,9 @@ struct mlbm_lattice {
   unsigned long long wait_ns = mlbm::kDefaultWaitNs;  // bounded waits
   bool stall_test = false;  // the next step launch makes a wait run out
   int phase = 0;  // 0: post-collision at opp slots of own node; 1: pushed
-  // counts the calls on this lattice after which a table made of its phase,
-  // layout, buffers and parameters (batch.cu) is out of date
-  unsigned long long changes = 0;
+  // count the calls on this lattice after which tables made of it (batch.cu)
+  // are out of date: of its parameters and lists, of its phase and layout
+  unsigned long long changes = 0, moves = 0;
   bool slab = false;  // planes 0 and lz - 1 are halo planes (slab.cu)
   bool has_params = false, has_mask = false, has_rho = false;
   bool initialized = false;

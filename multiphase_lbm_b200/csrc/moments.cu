@@ -84,6 +84,7 @@ mlbm_status build_list(mlbm_lattice* lat) {
   cudaFree(own);
   if (e != cudaSuccess) return cuda_fail(e, "moment lists");
   s.list_built = true;
+  ++lat->changes;
   return MLBM_OK;
 }
 

@@ -59,7 +59,7 @@ mlbm_status ready_for_passes(mlbm_lattice* lat, const char* who) {
   }
   cudaError_t e = cudaSetDevice(lat->device);
   if (e != cudaSuccess) return slab_cuda(e, "cudaSetDevice");
-  ++lat->changes;
+  ++lat->moves;
   return compact_enter(lat);
 }
 

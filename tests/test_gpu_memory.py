@@ -193,7 +193,7 @@ def test_a_domain_that_does_not_fit_takes_the_batchs_moments_first():
     step = _run(b, ids, alone, 0, 4)
     grown = first.test_memory_limit()
     assert grown > held
-    # 1280^3 FP64 nodes take 369 GB: refused before an array is read
+    # 1280^3 FP64 nodes take 370 GB: refused before an array is read
     one = np.ones(1, np.float32)
     did = C.c_int32()
     p = capi.default_params(**KW)
@@ -249,4 +249,30 @@ def test_stated_bytes_cover_what_is_held(shape, solid, storage):
     if solid == 0.0 and shape[2] > 1:  # not by much above it, either
         assert max(held) >= 0.9 * (capi.lattice_bytes(shape, storage) - 70_000)
     assert b.nbytes() == sum(held)
+    b.close()
+
+
+@pytest.mark.parametrize("storage", [0, 2])
+def test_buffers_given_back_and_taken_again_between_batch_calls(storage):
+    """The only domain's moments make room for one that does not fit after all;
+    its own steps then take new buffers, which the batch goes on with."""
+    import ctypes as C
+
+    import numpy as np
+
+    from multiphase_lbm_b200 import batch, capi
+    b, ids, alone = _batch(capi, storage)
+    b.remove(ids.pop())
+    alone.pop().close()
+    step = _run(b, ids, alone, 0, 12)  # a graph of 8 steps is kept
+    one = np.ones(1, np.float32)
+    did = C.c_int32()
+    p = capi.default_params(**KW)
+    n = 1280 if storage == 2 else 1287  # 370 GB, 196 GB
+    assert batch.blib().mlbm_batch_add(b.h, n - n % 32, n, n, C.byref(p), one.ctypes.data,
+                                       one.ctypes.data, 0, C.byref(did)) == 3
+    for lat in (b.lattice(ids[0]), alone[0]):
+        lat.iterate(step, 3)
+    step += 3
+    _run(b, ids, alone, step, 12)
     b.close()

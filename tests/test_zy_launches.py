@@ -86,6 +86,9 @@ def test_the_same_parameters_again_change_nothing(tau):
         b.iterate(12)
 
     assert not [n for n in _launched(lambda: again(p), True) if "HtoD" in n]
+    if tau == 1.0:  # nor after steps of its own, which leave it held as moments
+        b.lattice(did).iterate(24, 3)
+        assert not [n for n in _launched(lambda: again(p), True) if "HtoD" in n]
     q = capi.default_params(G=-4.9, rhos=0.2, tau=tau)
     assert [n for n in _launched(lambda: again(q), True) if "HtoD" in n]
     b.close()
